@@ -35,7 +35,8 @@ void gemm_entry(Context& c, char ta, char tb, int m, int n, int k, CT alpha, con
     if ((k > 0 && (!a || !b)) || !cc) throw q3b::Status(Q3B_ERR_INVALID, "gemm: null matrix");
     if (lda < (conj ? k : m) || ldb < k || ldc < m || lda < 1 || ldb < 1)
         throw q3b::Status(Q3B_ERR_INVALID, "gemm: leading dimension too small");
-    q3b::GemmWorkspace ws = c.gemm_ws(conj ? q3b::cgemm_workspace_bytes<R>(m, n, k) : 0);
+    q3b::GemmWorkspace ws = c.gemm_ws(conj ? q3b::cgemm_workspace_bytes<R>(m, n, k) : 0,
+                                      q3b::cgemm_wanted_bytes<R>(conj, m, n, k));
     if constexpr (std::is_same<R, float>::value) {
         // the single-precision entry point always runs on the tensor cores
         // (the library's own products route small ones to the CUDA cores)
@@ -352,7 +353,8 @@ int q3b_hegv_lowest(q3b_context* ctx, int n, const q3b_cplx128* h, const q3b_cpl
         if (n == 0) return;
         c.ws_dense.reserve(&c, q3b::dense::hegv_scratch_bytes(n));
         q3b::dense::Scratch ws{c.ws_dense.as<char>(), c.ws_dense.bytes, 0};
-        q3b::GemmWorkspace g = c.gemm_ws(q3b::cgemm_workspace_bytes<double>(n, n, n));
+        q3b::GemmWorkspace g = c.gemm_ws(q3b::cgemm_workspace_bytes<double>(n, n, n),
+                                         q3b::cgemm_wanted_bytes<double>(true, n, n, n));
         const int info = q3b::dense::hegv(c.stream, n, reinterpret_cast<const double2*>(h),
                                           reinterpret_cast<const double2*>(s), ld, w,
                                           reinterpret_cast<double2*>(evec), nvec, ws, g, &c.hegv_graphs);
@@ -415,7 +417,8 @@ int q3b_hegv(q3b_context* ctx, int n, const q3b_cplx128* h, const q3b_cplx128* s
         if (n == 0) return;
         c.ws_dense.reserve(&c, q3b::dense::hegv_scratch_bytes(n));
         q3b::dense::Scratch ws{c.ws_dense.as<char>(), c.ws_dense.bytes, 0};
-        q3b::GemmWorkspace g = c.gemm_ws(q3b::cgemm_workspace_bytes<double>(n, n, n));
+        q3b::GemmWorkspace g = c.gemm_ws(q3b::cgemm_workspace_bytes<double>(n, n, n),
+                                         q3b::cgemm_wanted_bytes<double>(true, n, n, n));
         const int info = q3b::dense::hegv(c.stream, n, reinterpret_cast<const double2*>(h),
                                           reinterpret_cast<const double2*>(s), ld, w,
                                           reinterpret_cast<double2*>(evec), n, ws, g, &c.hegv_graphs);

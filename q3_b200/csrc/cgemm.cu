@@ -4,6 +4,7 @@
 #include <type_traits>
 
 #include "cgemm.cuh"
+#include "zgemm_mod.cuh"
 
 namespace q3b {
 namespace {
@@ -451,6 +452,13 @@ template <typename R> size_t cgemm_workspace_bytes(int M, int N, int K) {
     return simt;
 }
 
+template <typename R> size_t cgemm_wanted_bytes(bool conj_a, int M, int N, int K) {
+    if constexpr (std::is_same<R, double>::value) {
+        if (zmod::worth(conj_a, M, N, K, false)) return zmod::workspace_bytes(conj_a, M, N, K, false);
+    }
+    return 0;
+}
+
 template <typename R>
 void cgemm(cudaStream_t st, bool conj_a, int M, int N, int K, cplx_t<R> alpha, const cplx_t<R>* A,
            long lda, const cplx_t<R>* B, long ldb, cplx_t<R> beta, cplx_t<R>* C, long ldc,
@@ -475,6 +483,12 @@ void cgemm(cudaStream_t st, bool conj_a, int M, int N, int K, cplx_t<R> alpha, c
         return;
     }
     if constexpr (std::is_same<R, double>::value) {
+        if (zmod::worth(conj_a, M, N, K, false) && ws.ptr &&
+            ws.bytes >= zmod::workspace_bytes(conj_a, M, N, K, false) && reinterpret_cast<uintptr_t>(A) % 16 == 0 &&
+            reinterpret_cast<uintptr_t>(B) % 16 == 0) {
+            zmod::zgemm(st, conj_a, M, N, K, alpha, A, lda, nullptr, B, ldb, beta, C, ldc, ws);
+            return;
+        }
         if (big_tiles(M, N) && reinterpret_cast<uintptr_t>(A) % 16 == 0 &&
             reinterpret_cast<uintptr_t>(B) % 16 == 0) {
             zgemm_big_launch(st, conj_a, M, N, K, alpha, A, lda, B, ldb, beta, C, ldc, ws);
@@ -553,5 +567,7 @@ template void cgemm<float>(cudaStream_t, bool, int, int, int, float2, const floa
                            const float2*, long, float2, float2*, long, const GemmWorkspace&);
 template size_t cgemm_workspace_bytes<double>(int, int, int);
 template size_t cgemm_workspace_bytes<float>(int, int, int);
+template size_t cgemm_wanted_bytes<double>(bool, int, int, int);
+template size_t cgemm_wanted_bytes<float>(bool, int, int, int);
 
 }  // namespace q3b

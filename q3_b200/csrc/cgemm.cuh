@@ -31,6 +31,9 @@ double measure_dfma_tflops(cudaStream_t st);
 
 // bytes of workspace cgemm may use for a C,N product of this shape
 template <typename R> size_t cgemm_workspace_bytes(int M, int N, int K);
+// bytes with which a large FP64 product runs on the integer tensor cores
+// (zgemm_mod.cuh); with less it runs on the FP64 units
+template <typename R> size_t cgemm_wanted_bytes(bool conj_a, int M, int N, int K);
 
 // FP32 products of at least this many complex multiply-adds (M N K) run on
 // the tensor cores, smaller ones on the CUDA cores

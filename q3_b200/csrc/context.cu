@@ -95,12 +95,18 @@ void DevBuf::reserve(Context* c, size_t need) {
     release();
     ctx = c;
     if (need == 0) return;
-    if (c->budget && c->held + need > c->budget) {
+    auto over = [&] { return c->budget && c->held + need > c->budget; };
+    if (over()) c->release_optional();
+    if (over()) {
         throw Status(Q3B_ERR_MEMORY, "HBM budget exceeded: need " + std::to_string(need) +
                                          " bytes, hold " + std::to_string(c->held) + " of " +
                                          std::to_string(c->budget));
     }
     cudaError_t e = cudaMalloc(&ptr, need);
+    if (e == cudaErrorMemoryAllocation && c->release_optional()) {
+        cudaGetLastError();
+        e = cudaMalloc(&ptr, need);
+    }
     if (e != cudaSuccess) {
         ptr = nullptr;
         cudaGetLastError();
@@ -108,6 +114,22 @@ void DevBuf::reserve(Context* c, size_t need) {
     }
     bytes = need;
     c->held += need;
+}
+
+bool DevBuf::try_reserve(Context* c, size_t need) {
+    if (need <= bytes && ptr) return true;
+    if (c->budget && c->held - bytes + need > c->budget) return false;
+    release();
+    ctx = c;
+    if (need == 0) return true;
+    if (cudaMalloc(&ptr, need) != cudaSuccess) {
+        ptr = nullptr;
+        cudaGetLastError();
+        return false;
+    }
+    bytes = need;
+    c->held += need;
+    return true;
 }
 
 template <typename T>
@@ -153,9 +175,29 @@ void Context::ensure_io_streams() {
     }
 }
 
-GemmWorkspace Context::gemm_ws(size_t need) {
+GemmWorkspace Context::gemm_ws(size_t need, size_t want) {
+    if (need > ws_gemm_need_) ws_gemm_need_ = need;
+    if (want > need && want > ws_gemm.bytes && !(ws_gemm_refused_ && want >= ws_gemm_refused_)) {
+        const bool in_budget = !budget || held - ws_gemm.bytes + want <= budget;
+        if (!ws_gemm.try_reserve(this, want) && in_budget) ws_gemm_refused_ = want;
+    }
     ws_gemm.reserve(this, need);
     return GemmWorkspace{ws_gemm.ptr, ws_gemm.bytes};
+}
+
+bool Context::release_optional() {
+    // callers ask for the GEMM workspace after all their other buffers, so no
+    // product that still has to be issued holds its address here
+    bool any = false;
+    for (DevBuf* b : {&kp.beta_zm_overlap, &kp.beta_zm_accum}) {
+        any = any || b->ptr;
+        b->release();
+    }
+    if (ws_gemm.bytes > ws_gemm_need_) {
+        any = true;
+        ws_gemm.release();
+    }
+    return any;
 }
 
 void Context::require_ready() const {
@@ -568,15 +610,41 @@ void Context::prepare_kpoint(int npw, const int32_t* g2g, const double* ke, cons
         kp.dpk_len = d64.size();
     }
     build_plan();
+    pack_beta64();
     kp.valid = true;
+}
+
+// Residue tiles of the projectors for <beta|psi> and beta B', where a block of
+// bands of usual size (half the projectors, as four bands an atom make) runs
+// its products on them.
+void Context::pack_beta64() {
+    kp.beta_zm_overlap.release();
+    kp.beta_zm_accum.release();
+    const int P = kp.nproj, npw = kp.npw;
+    if (P <= 0 || !zmod::worth(true, P, P / 2, npw, true)) return;
+    const size_t to = zmod::packed_a_bytes(P, npw), ta = zmod::packed_a_bytes(npw, P);
+    if (!kp.beta_zm_overlap.try_reserve(this, to + zmod::packed_a_exps(P) * sizeof(int))) return;
+    if (!kp.beta_zm_accum.try_reserve(this, ta + zmod::packed_a_exps(npw) * sizeof(int))) return;
+    unsigned char* o = kp.beta_zm_overlap.as<unsigned char>();
+    unsigned char* a = kp.beta_zm_accum.as<unsigned char>();
+    zmod::pack_a(stream, P, npw, kp.beta64.as<double2>(), npw, true, o, reinterpret_cast<int*>(o + to));
+    zmod::pack_a(stream, npw, P, kp.beta64.as<double2>(), npw, false, a, reinterpret_cast<int*>(a + ta));
 }
 
 template <> const LocalPlan<double>& Context::local_plan<double>() const { return kp.lp64; }
 template <> const LocalPlan<float>& Context::local_plan<float>() const { return kp.lp32; }
 
 template <> NonlocalData<double> Context::nonlocal<double>() const {
-    return NonlocalData<double>{kp.nproj, kp.beta64.as<double2>(), kp.pstart.as<int>(),
-                                kp.psize.as<int>(), kp.poff.as<int>(), kp.dpk64.as<double>()};
+    NonlocalData<double> d{kp.nproj, kp.beta64.as<double2>(), kp.pstart.as<int>(),
+                           kp.psize.as<int>(), kp.poff.as<int>(), kp.dpk64.as<double>()};
+    auto packed = [](const DevBuf& b, int M, int K) {
+        if (!b.ptr) return zmod::PackedA{};
+        const unsigned char* t = b.as<unsigned char>();
+        return zmod::PackedA{t, reinterpret_cast<const int*>(t + zmod::packed_a_bytes(M, K)), M, K};
+    };
+    d.zm_overlap = packed(kp.beta_zm_overlap, kp.nproj, kp.npw);
+    d.zm_accum = packed(kp.beta_zm_accum, kp.npw, kp.nproj);
+    return d;
 }
 template <> NonlocalData<float> Context::nonlocal<float>() const {
     NonlocalData<float> d{kp.nproj, kp.beta32.as<float2>(), kp.pstart.as<int>(),
@@ -758,7 +826,8 @@ void Context::apply_h(const cplx_t<R>* psi, long ldpsi, cplx_t<R>* hpsi, long ld
         const size_t pb = (size_t)kp.nproj * nvec * sizeof(T);
         ws_bm.reserve(this, pb);
         ws_bp.reserve(this, pb);
-        GemmWorkspace ws = gemm_ws(cgemm_workspace_bytes<R>(kp.nproj, nvec, kp.npw));
+        GemmWorkspace ws = gemm_ws(cgemm_workspace_bytes<R>(kp.nproj, nvec, kp.npw),
+                                   nonlocal_wanted_bytes<R>(nonlocal<R>(), kp.npw, nvec));
         apply_nonlocal<R>(stream, nonlocal<R>(), kp.npw, nvec, psi, ldpsi, hpsi, ldh,
                           ws_bm.as<T>(), ws_bp.as<T>(), ws, tm);
     }

@@ -36,6 +36,9 @@ struct DevBuf {
     void release();
     // grow to at least `need` bytes (contents are not kept)
     void reserve(Context* c, size_t need);
+    // the same, but false (and the buffer as it was, or empty) where the budget
+    // or the device does not have the bytes
+    bool try_reserve(Context* c, size_t need);
     template <typename T> T* as() const { return static_cast<T*>(ptr); }
 };
 
@@ -49,6 +52,9 @@ struct KPoint {
     DevBuf ke64, ke32;
     DevBuf beta64, beta32;
     DevBuf beta_pk_overlap, beta_pk_accum;  // beta32 as packed tensor-core A tiles
+    // beta64 as residue tiles for the FP64 products, each followed by its rows'
+    // exponents; empty for small sets and where memory is short
+    DevBuf beta_zm_overlap, beta_zm_accum;
     DevBuf pstart, psize, poff, dpk64, dpk32;
     size_t dpk_len = 0;             // packed block entries (D, and Q when set)
     bool has_q = false;             // ultrasoft overlap blocks set for this k-point
@@ -132,7 +138,11 @@ class Context {
     void apply_h(const cplx_t<R>* psi, long ldpsi, cplx_t<R>* hpsi, long ldh, int nvec,
                  PhaseTimer* timer = nullptr);
 
-    GemmWorkspace gemm_ws(size_t need);
+    // at least `need` bytes; `want` bytes where there is room for them
+    GemmWorkspace gemm_ws(size_t need, size_t want = 0);
+    // give back the buffers that only speed up products (called when a
+    // reservation does not fit); true if any was held
+    bool release_optional();
 
     // Autotuner: time the candidate plane kernels on a few bands of this
     // k-point and keep the fastest (once per plan and precision).
@@ -142,7 +152,10 @@ class Context {
     template <typename R> int local_kernel();
 
   private:
+    size_t ws_gemm_need_ = 0;     // largest `need` of gemm_ws
+    size_t ws_gemm_refused_ = 0;  // smallest `want` the device had no room for (0: none)
     void build_plan();
+    void pack_beta64();
 };
 
 // convert an exception into a status code and message

@@ -274,7 +274,7 @@ template <typename R> class Davidson {
     // ------------------------------------------------------------ GEMM
     void gemm(bool conj, int M, int N, int K, T alpha, const T* A, long lda, const T* B, long ldb, T beta,
               T* C, long ldc) {
-        GemmWorkspace ws = c_.gemm_ws(conj ? cgemm_workspace_bytes<R>(M, N, K) : 0);
+        GemmWorkspace ws = c_.gemm_ws(conj ? cgemm_workspace_bytes<R>(M, N, K) : 0, cgemm_wanted_bytes<R>(conj, M, N, K));
         cgemm<R>(st_, conj, M, N, K, alpha, A, lda, B, ldb, beta, C, ldc, ws);
     }
     // inner products A^H B (K = npw): on a Gamma-only k-point the real
@@ -403,7 +403,7 @@ template <typename R> class Davidson {
             if (st == 0 && publish) whost_.assign(wread_.begin(), wread_.begin() + nvec);
             return st;
         }
-        GemmWorkspace gws = c_.gemm_ws(cgemm_workspace_bytes<double>(n, n, n));
+        GemmWorkspace gws = c_.gemm_ws(cgemm_workspace_bytes<double>(n, n, n), cgemm_wanted_bytes<double>(true, n, n, n));
         // the lowest nvec eigenvalues come back in the solve's own status read
         wread_.assign(n, 0.0);
         const int info = dense::hegv(st_, n, H, S, ld, w_, evec_, nvec, dscratch_, gws, &c_.hegv_graphs,
@@ -529,7 +529,8 @@ template <typename R> class Davidson {
         const size_t pb = (size_t)P * nv * sizeof(T);
         c_.ws_bm.reserve(&c_, pb);
         c_.ws_bp.reserve(&c_, pb);
-        GemmWorkspace ws = c_.gemm_ws(cgemm_workspace_bytes<R>(P, nv, len));
+        GemmWorkspace ws = c_.gemm_ws(cgemm_workspace_bytes<R>(P, nv, len),
+                                      nonlocal_wanted_bytes<R>(c_.overlap<R>(), len, nv));
         apply_nonlocal<R>(st_, c_.overlap<R>(), len, nv, in, len, out, len, c_.ws_bm.as<T>(), c_.ws_bp.as<T>(), ws);
         if (gamma_) {
             gamma_unpack<T><<<gamma_blocks((long)npw_ * nv), 256, 0, st_>>>(npw_, count, ghphi_, nfull, sv, npw_);

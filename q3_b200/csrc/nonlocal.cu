@@ -1,3 +1,5 @@
+#include <algorithm>
+#include <cstdint>
 #include <type_traits>
 // Kleinman-Bylander term and small elementwise helpers.
 //
@@ -47,6 +49,17 @@ inline int grid_for(long n) { return stride_grid(n, 16); }
 
 }  // namespace
 
+template <typename R> size_t nonlocal_wanted_bytes(const NonlocalData<R>& nl, int npw, int nvec) {
+    size_t b = 0;
+    if constexpr (std::is_same<R, double>::value) {
+        if (nl.zm_overlap.tiles && zmod::worth(true, nl.nproj, nvec, npw, true))
+            b = zmod::workspace_bytes(true, nl.nproj, nvec, npw, true);
+        if (nl.zm_accum.tiles && zmod::worth(false, npw, nvec, nl.nproj, true))
+            b = std::max(b, zmod::workspace_bytes(false, npw, nvec, nl.nproj, true));
+    }
+    return b;
+}
+
 template <typename R>
 void apply_nonlocal(cudaStream_t st, const NonlocalData<R>& nl, int npw, int nvec,
                     const cplx_t<R>* psi, long ldpsi, cplx_t<R>* hpsi, long ldh, cplx_t<R>* Bm,
@@ -60,6 +73,10 @@ void apply_nonlocal(cudaStream_t st, const NonlocalData<R>& nl, int npw, int nve
             tc::cgemm_packed(st, true, nl.nproj, nvec, npw, one, nl.beta_overlap, psi, ldpsi, zero, Bm, nl.nproj, ws);
         else
             cgemm<R>(st, true, nl.nproj, nvec, npw, one, nl.beta, npw, psi, ldpsi, zero, Bm, nl.nproj, ws);
+    } else if (nl.zm_overlap.tiles && zmod::worth(true, nl.nproj, nvec, npw, true) && ws.ptr &&
+               ws.bytes >= zmod::workspace_bytes(true, nl.nproj, nvec, npw, true) &&
+               reinterpret_cast<uintptr_t>(psi) % 16 == 0) {
+        zmod::zgemm(st, true, nl.nproj, nvec, npw, one, nullptr, 0, &nl.zm_overlap, psi, ldpsi, zero, Bm, nl.nproj, ws);
     } else {
         cgemm<R>(st, true, nl.nproj, nvec, npw, one, nl.beta, npw, psi, ldpsi, zero, Bm, nl.nproj, ws);
     }
@@ -75,6 +92,9 @@ void apply_nonlocal(cudaStream_t st, const NonlocalData<R>& nl, int npw, int nve
             tc::cgemm_packed(st, false, npw, nvec, nl.nproj, one, nl.beta_accum, Bp, nl.nproj, one, hpsi, ldh, ws);
         else
             cgemm<R>(st, false, npw, nvec, nl.nproj, one, nl.beta, npw, Bp, nl.nproj, one, hpsi, ldh, ws);
+    } else if (nl.zm_accum.tiles && zmod::worth(false, npw, nvec, nl.nproj, true) && ws.ptr &&
+               ws.bytes >= zmod::workspace_bytes(false, npw, nvec, nl.nproj, true)) {
+        zmod::zgemm(st, false, npw, nvec, nl.nproj, one, nullptr, 0, &nl.zm_accum, Bp, nl.nproj, one, hpsi, ldh, ws);
     } else {
         cgemm<R>(st, false, npw, nvec, nl.nproj, one, nl.beta, npw, Bp, nl.nproj, one, hpsi, ldh, ws);
     }
@@ -94,6 +114,8 @@ template void apply_nonlocal<double>(cudaStream_t, const NonlocalData<double>&, 
 template void apply_nonlocal<float>(cudaStream_t, const NonlocalData<float>&, int, int,
                                     const float2*, long, float2*, long, float2*, float2*,
                                     const GemmWorkspace&, PhaseTimer*);
+template size_t nonlocal_wanted_bytes<double>(const NonlocalData<double>&, int, int);
+template size_t nonlocal_wanted_bytes<float>(const NonlocalData<float>&, int, int);
 template void convert<double, float>(cudaStream_t, long, const double2*, float2*);
 template void convert<float, double>(cudaStream_t, long, const float2*, double2*);
 template void convert<double, double>(cudaStream_t, long, const double2*, double2*);

@@ -4,6 +4,7 @@
 #include "cgemm.cuh"
 #include "common.cuh"
 #include "hpsi_local.cuh"
+#include "zgemm_mod.cuh"
 
 namespace q3b {
 
@@ -17,7 +18,13 @@ template <typename R> struct NonlocalData {
     // FP32 only: beta pre-split into the tensor-core kernel's A tiles, for
     // beta^H psi (rows = projectors) and for beta B' (rows = plane waves)
     tc::PackedA beta_overlap{}, beta_accum{};
+    // FP64 only: beta as residue tiles for the same two products (may be empty)
+    zmod::PackedA zm_overlap{}, zm_accum{};
 };
+
+// workspace with which both projector products of nvec bands run on the
+// residue tiles (0: they do not, at this size or for these projectors)
+template <typename R> size_t nonlocal_wanted_bytes(const NonlocalData<R>& nl, int npw, int nvec);
 
 // hpsi += beta D beta^H psi.  Bm, Bp: nproj x nvec scratch each.
 template <typename R>

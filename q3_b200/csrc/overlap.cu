@@ -38,7 +38,8 @@ void apply_s_device(Context& c, const double2* psi, double2* spsi, int nvec, int
         const size_t pb = (size_t)P * nvec * sizeof(double2);
         c.ws_bm.reserve(&c, pb);
         c.ws_bp.reserve(&c, pb);
-        GemmWorkspace ws = c.gemm_ws(cgemm_workspace_bytes<double>(P, nvec, npw));
+        GemmWorkspace ws = c.gemm_ws(cgemm_workspace_bytes<double>(P, nvec, npw),
+                                     nonlocal_wanted_bytes<double>(c.overlap<double>(), npw, nvec));
         apply_nonlocal<double>(c.stream, c.overlap<double>(), npw, nvec, psi, npw, spsi, npw,
                                c.ws_bm.as<double2>(), c.ws_bp.as<double2>(), ws);
     } else if (precision == Q3B_MIXED) {

@@ -24,6 +24,7 @@
 #include "context.cuh"
 #include "davidson.cuh"
 #include "dense.cuh"
+#include "zgemm_mod.cuh"
 #include "q3b.h"
 
 namespace q3b {
@@ -72,6 +73,12 @@ size_t estimate_bytes(const Job& j) {
     b += std::min<size_t>(48ull << 20, (size_t)j.nb * j.n3 * (size_t)j.n1 * j.n2 / 4 * sizeof(double2));
     // projectors: FP64, FP32 and the two packed tensor-core copies (16 B each)
     b += (size_t)j.npw * j.nproj * (sizeof(double2) + sizeof(float2) + 32);
+    // the projectors' residue tiles and the workspace of the largest FP64 products
+    const int P = j.nproj, nb = (int)maxn64 / 2;
+    if (P > 0 && zmod::worth(true, P, P / 2, j.npw, true))
+        b += zmod::packed_a_bytes(P, j.npw) + zmod::packed_a_bytes(j.npw, P);
+    b += std::max(cgemm_wanted_bytes<double>(true, (int)maxn64, nb, j.npw),
+                  cgemm_wanted_bytes<double>(false, j.npw, nb, (int)maxn64));
     b += 2 * N * (sizeof(double) + sizeof(float));  // V/N in two layouts
     b += 2 * (size_t)j.nproj * j.nb * sizeof(double2) + (16ull << 20);
     return b + b / 5;

@@ -50,14 +50,16 @@ void require_started(const q3b::Context& c) {
 // H (n x n) and S (n x n), ld n, on the device
 void start_project_dev(q3b::Context& c, double2* H, double2* S) {
     const int n = c.start_n, npw = c.start_npw;
-    q3b::GemmWorkspace g = c.gemm_ws(q3b::cgemm_workspace_bytes<double>(n, n, npw));
+    q3b::GemmWorkspace g = c.gemm_ws(q3b::cgemm_workspace_bytes<double>(n, n, npw),
+                                     q3b::cgemm_wanted_bytes<double>(true, n, n, npw));
     q3b::cgemm<double>(c.stream, true, n, n, npw, kOne, chi_of(c), npw, hchi_of(c), npw, kZero, H, n, g);
     q3b::cgemm<double>(c.stream, true, n, n, npw, kOne, chi_of(c), npw, chi_of(c), npw, kZero, S, n, g);
 }
 
 void start_rotate_dev(q3b::Context& c, const double2* C, int ldc, int nb, double2* bands) {
     const int n = c.start_n, npw = c.start_npw;
-    q3b::GemmWorkspace g = c.gemm_ws(q3b::cgemm_workspace_bytes<double>(npw, nb, n));
+    q3b::GemmWorkspace g = c.gemm_ws(q3b::cgemm_workspace_bytes<double>(npw, nb, n),
+                                     q3b::cgemm_wanted_bytes<double>(false, npw, nb, n));
     q3b::cgemm<double>(c.stream, false, npw, nb, n, kOne, chi_of(c), npw, C, ldc, kZero, bands, npw, g);
 }
 
@@ -117,7 +119,8 @@ int q3b_starting_subspace(q3b_context* ctx, const q3b_cplx128* chi_host, int nch
         start_project_dev(c, H, S);
         c.ws_dense.reserve(&c, q3b::dense::hegv_scratch_bytes(n));
         q3b::dense::Scratch ws{c.ws_dense.as<char>(), c.ws_dense.bytes, 0};
-        q3b::GemmWorkspace g = c.gemm_ws(q3b::cgemm_workspace_bytes<double>(n, n, n));
+        q3b::GemmWorkspace g = c.gemm_ws(q3b::cgemm_workspace_bytes<double>(n, n, n),
+                                         q3b::cgemm_wanted_bytes<double>(true, n, n, n));
         const int info = q3b::dense::hegv(c.stream, n, H, S, n, w, Z, nb, ws, g, &c.hegv_graphs);
         if (info != 0)
             throw q3b::Status(Q3B_ERR_LINALG, "overlap of the starting vectors is not positive definite (info " +

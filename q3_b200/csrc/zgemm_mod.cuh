@@ -1,0 +1,33 @@
+// FP64 complex GEMMs on the integer tensor cores; see zgemm_mod.cu.
+#pragma once
+
+#include "cgemm.cuh"
+
+namespace q3b {
+namespace zmod {
+
+// An operand scaled to integers and reduced modulo each modulus, as the tiles
+// of 128 rows x 128 K the kernel copies, for operands used many times (a
+// k-point's projectors).  Rows are M of the product, K its reduction index.
+struct PackedA {
+    const unsigned char* tiles = nullptr;
+    const int* exps = nullptr;  // power of two each row was scaled by
+    int M = 0, K = 0;
+};
+size_t packed_a_bytes(int M, int K);
+size_t packed_a_exps(int M);  // ints
+// kmajor: element (m, k) at A[m * lda + k] (the "C,N" operand); else at A[m + k * lda]
+void pack_a(cudaStream_t st, int M, int K, const double2* A, long lda, bool kmajor, unsigned char* tiles, int* exps);
+
+// whether the product is faster here than on the FP64 units
+bool worth(bool conj_a, int M, int N, int K, bool packed);
+size_t workspace_bytes(bool conj_a, int M, int N, int K, bool packed);
+
+// C = alpha op(A) B + beta C as cgemm<double>; `pk` replaces A when given.
+// ws holds at least workspace_bytes(...).
+void zgemm(cudaStream_t st, bool conj_a, int M, int N, int K, double2 alpha, const double2* A, long lda,
+           const PackedA* pk, const double2* B, long ldb, double2 beta, double2* C, long ldc,
+           const GemmWorkspace& ws);
+
+}  // namespace zmod
+}  // namespace q3b
