@@ -469,7 +469,8 @@ void Context::build_plan() {
         if (gcol[g] >= 0) start[col_id[gcol[g]] + 1]++;
     for (int s = 0; s < S; ++s) start[s + 1] += start[s];
     const int nent = start[S];
-    std::vector<int> eg(nent), ew3(nent), es(nent), fill(start.begin(), start.end() - 1);
+    constexpr int kStickGroup = 32;
+    std::vector<int> eg(nent), ew3(nent), es(nent), ea(nent), fill(start.begin(), start.end() - 1);
     for (int g = 0; g < k.npw; ++g) {
         if (gcol[g] < 0) continue;
         const int s = col_id[gcol[g]];
@@ -477,11 +478,13 @@ void Context::build_plan() {
         eg[e] = g;
         ew3[e] = gw3[g];
         es[e] = s;
+        ea[e] = (s % kStickGroup) * p3 + gw3[g];
     }
     upload(this, k.stick_start, start.data(), start.size());
     upload(this, k.entry_g, eg.data(), eg.size());
     upload(this, k.entry_w3, ew3.data(), ew3.size());
     upload(this, k.entry_stick, es.data(), es.size());
+    upload(this, k.entry_at, ea.data(), ea.size());
     upload(this, k.stick_pos, stick_pos.data(), stick_pos.size());
     upload(this, k.row_base, rows.data(), rows.size());
     upload(this, k.unmapped, unm.data(), unm.size());
@@ -515,13 +518,14 @@ void Context::build_plan() {
         lp.nb2 = f[3];
         lp.na3 = f[4];
         lp.nb3 = f[5];
-        lp.sg = 32;
+        lp.sg = kStickGroup;
         lp.plane_threads = 256;
         lp.nunmapped = static_cast<int>(unm.size());
         lp.stick_start = k.stick_start.as<int>();
         lp.entry_g = k.entry_g.as<int>();
         lp.entry_w3 = k.entry_w3.as<int>();
         lp.entry_stick = k.entry_stick.as<int>();
+        lp.entry_at = k.entry_at.as<int>();
         lp.stick_pos = k.stick_pos.as<int>();
         lp.row_base = k.row_base.as<int>();
         lp.unmapped_g = k.unmapped.as<int>();

@@ -311,15 +311,16 @@ __global__ void __launch_bounds__(256, 2) planes_density(LocalPlan<double> p, co
 }
 
 // rho[(w1*N2 + w2)*N3 + w3] += sum over groups (in order) of the partial at
-// the digit-reversed positions of (w1, w2, w3)
-__global__ void density_reduce(LocalPlan<double> p, int groups, const double* partial, double* rho) {
+// the positions of (w1, w2, w3): digit-reversed, w1 only where w1_reversed
+__global__ void density_reduce(LocalPlan<double> p, int groups, const double* partial, double* rho,
+                               int w1_reversed) {
     const long n = (long)p.n1 * p.n2 * p.n3;
     const long nplane = (long)p.n1 * p.n2;
     for (long idx = blockIdx.x * (long)blockDim.x + threadIdx.x; idx < n; idx += (long)gridDim.x * blockDim.x) {
         const int w3 = static_cast<int>(idx % p.n3);
         const int w2 = static_cast<int>((idx / p.n3) % p.n2);
         const int w1 = static_cast<int>(idx / ((long)p.n3 * p.n2));
-        const int q1 = p.nb1 * (w1 % p.na1) + w1 / p.na1;
+        const int q1 = w1_reversed ? p.nb1 * (w1 % p.na1) + w1 / p.na1 : w1;
         const int q2 = p.nb2 * (w2 % p.na2) + w2 / p.na2;
         const int q3 = p.nb3 * (w3 % p.na3) + w3 / p.na3;
         const long off = (long)q3 * nplane + (long)q1 * p.n2 + q2;
@@ -366,33 +367,81 @@ void PhaseTimer::collect(double* ms, int* count) {
     }
 }
 
+namespace {
+
+// The passes by the kernels for compile-time lengths (planes_sq.cuh) where the
+// plan has them, else by the general ones above.
+inline bool sq_planes(const LocalPlan<double>& p, double2* X, int nb, cudaStream_t st) {
+    return psq::f64_small_planes(p, X, nb, st) || psq::f64_large_planes(p, X, nb, st);
+}
+inline bool sq_planes(const LocalPlan<float>& p, float2* X, int nb, cudaStream_t st) {
+    return psq::f32_small_planes(p, X, nb, st) || psq::f32_large_planes(p, X, nb, st);
+}
+inline bool sq_back(const LocalPlan<double>& p, const double2* psi, long ld, double2* X, int nb, cudaStream_t st) {
+    return psq::f64_small_back(p, psi, ld, X, nb, st) || psq::f64_large_back(p, psi, ld, X, nb, st);
+}
+inline bool sq_back(const LocalPlan<float>& p, const float2* psi, long ld, float2* X, int nb, cudaStream_t st) {
+    return psq::f32_small_back(p, psi, ld, X, nb, st) || psq::f32_large_back(p, psi, ld, X, nb, st);
+}
+inline bool sq_fwd(const LocalPlan<double>& p, const double2* X, const double2* psi, long ld, double2* h, long ldh,
+                   int nb, cudaStream_t st) {
+    return psq::f64_small_fwd(p, X, psi, ld, h, ldh, nb, st) || psq::f64_large_fwd(p, X, psi, ld, h, ldh, nb, st);
+}
+inline bool sq_fwd(const LocalPlan<float>& p, const float2* X, const float2* psi, long ld, float2* h, long ldh,
+                   int nb, cudaStream_t st) {
+    return psq::f32_small_fwd(p, X, psi, ld, h, ldh, nb, st) || psq::f32_large_fwd(p, X, psi, ld, h, ldh, nb, st);
+}
+
+template <typename R>
+void run_sticks_backward(const LocalPlan<R>& p, const cplx_t<R>* psi, long ldpsi, cplx_t<R>* X, int nb,
+                         cudaStream_t st) {
+    const dim3 grid(ceil_div(p.nsticks, p.sg), nb);
+    if (sq_back(p, psi, ldpsi, X, nb, st)) {
+    } else if (p.na3 <= kSmallR && p.nb3 <= kSmallR) {
+        sticks_backward<R, kSmallR><<<grid, kStickThreads, stick_smem_bytes(p), st>>>(p, psi, ldpsi, X);
+    } else {
+        sticks_backward<R, 16><<<grid, kStickThreads, stick_smem_bytes(p), st>>>(p, psi, ldpsi, X);
+    }
+    Q3B_LAUNCH_CHECK();
+}
+
+template <typename R>
+void run_sticks_forward(const LocalPlan<R>& p, const cplx_t<R>* X, const cplx_t<R>* psi, long ldpsi,
+                        cplx_t<R>* hpsi, long ldh, int nb, cudaStream_t st) {
+    const dim3 grid(ceil_div(p.nsticks, p.sg), nb);
+    if (sq_fwd(p, X, psi, ldpsi, hpsi, ldh, nb, st)) {
+    } else if (p.na3 <= kSmallR && p.nb3 <= kSmallR) {
+        sticks_forward<R, kSmallR><<<grid, kStickThreads, stick_smem_bytes(p), st>>>(p, X, psi, ldpsi, hpsi, ldh);
+    } else {
+        sticks_forward<R, 16><<<grid, kStickThreads, stick_smem_bytes(p), st>>>(p, X, psi, ldpsi, hpsi, ldh);
+    }
+    Q3B_LAUNCH_CHECK();
+}
+
+}  // namespace
+
 template <typename R>
 void apply_local(cudaStream_t st, const LocalPlan<R>& p, const cplx_t<R>* psi, long ldpsi,
                  cplx_t<R>* hpsi, long ldh, int nvec, cplx_t<R>* X, int chunk, PhaseTimer* tm) {
     if (nvec <= 0) return;
     set_smem_limits<R>();
     if (chunk < 1) chunk = 1;
-    const size_t smem_s = stick_smem_bytes(p);
     const size_t smem_p = plane_smem_bytes(p);
-    const int nsg = ceil_div(p.nsticks, p.sg);
     for (int b0 = 0; b0 < nvec; b0 += chunk) {
         const int nb = nvec - b0 < chunk ? nvec - b0 : chunk;
         const cplx_t<R>* ps = psi + (long)b0 * ldpsi;
         cplx_t<R>* hs = hpsi + (long)b0 * ldh;
         if (p.nsticks > 0) {
             if (tm) tm->begin(PhaseTimer::STICKS_BACKWARD);
-            const bool small3 = p.na3 <= kSmallR && p.nb3 <= kSmallR;
-            if (small3)
-                sticks_backward<R, kSmallR><<<dim3(nsg, nb), kStickThreads, smem_s, st>>>(p, ps, ldpsi, X);
-            else
-                sticks_backward<R, 16><<<dim3(nsg, nb), kStickThreads, smem_s, st>>>(p, ps, ldpsi, X);
-            Q3B_LAUNCH_CHECK();
+            run_sticks_backward<R>(p, ps, ldpsi, X, nb, st);
             if (tm) tm->end();
             if (tm) tm->begin(PhaseTimer::PLANES);
             const dim3 gp(p.n3, nb);
             const bool small12 = p.na1 <= kSmallR && p.nb1 <= kSmallR && p.na2 <= kSmallR && p.nb2 <= kSmallR;
             if (p.variant > 0 && launch_planes_reg<R>(p, X, nb, p.variant, st, p.err)) {
                 // the register kernel took the plane pass
+            } else if (sq_planes(p, X, nb, st)) {
+                // a kernel for this plane size
             } else if (small12) {
                 if (p.plane_threads >= 512) launch_planes<R, 512, kSmallR>(gp, smem_p, st, p, X);
                 else if (p.plane_threads >= 256) launch_planes<R, 256, kSmallR>(gp, smem_p, st, p, X);
@@ -405,11 +454,7 @@ void apply_local(cudaStream_t st, const LocalPlan<R>& p, const cplx_t<R>* psi, l
             Q3B_LAUNCH_CHECK();
             if (tm) tm->end();
             if (tm) tm->begin(PhaseTimer::STICKS_FORWARD);
-            if (small3)
-                sticks_forward<R, kSmallR><<<dim3(nsg, nb), kStickThreads, smem_s, st>>>(p, X, ps, ldpsi, hs, ldh);
-            else
-                sticks_forward<R, 16><<<dim3(nsg, nb), kStickThreads, smem_s, st>>>(p, X, ps, ldpsi, hs, ldh);
-            Q3B_LAUNCH_CHECK();
+            run_sticks_forward<R>(p, X, ps, ldpsi, hs, ldh, nb, st);
             if (tm) tm->end();
         }
     }
@@ -423,6 +468,12 @@ void apply_local(cudaStream_t st, const LocalPlan<R>& p, const cplx_t<R>* psi, l
 }
 
 namespace {
+
+inline bool sq_density(const LocalPlan<double>& p, const double2* X, int nb, const double* w, double* partial,
+                       int groups, cudaStream_t st, int* per_sm) {
+    return psq::f64_small_density(p, X, nb, w, partial, groups, st, per_sm) ||
+           psq::f64_large_density(p, X, nb, w, partial, groups, st, per_sm);
+}
 
 // the partial slabs of the density stay below this many bytes, so that they
 // stay in L2 beside a stick chunk (48 MB) while the bands add into them
@@ -453,7 +504,8 @@ int density_groups(const LocalPlan<double>& p, int nvec) {
     if (nvec < 1) return 1;
     set_density_limits();
     int per_sm = 0, dev = 0, sms = 0;
-    if (density_small_factors(p))
+    if (sq_density(p, nullptr, 0, nullptr, nullptr, 0, nullptr, &per_sm)) {
+    } else if (density_small_factors(p))
         Q3B_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, planes_density<kSmallR>, 256,
                                                                plane_smem_bytes(p)));
     else
@@ -483,24 +535,18 @@ void accumulate_density(cudaStream_t st, const LocalPlan<double>& p, const doubl
     set_smem_limits<double>();
     set_density_limits();
     if (chunk < 1) chunk = 1;
-    const size_t smem_s = stick_smem_bytes(p);
     const size_t smem_p = plane_smem_bytes(p);
-    const int nsg = ceil_div(p.nsticks, p.sg);
-    const bool small3 = p.na3 <= kSmallR && p.nb3 <= kSmallR;
     const bool small12 = density_small_factors(p);
     Q3B_CUDA(cudaMemsetAsync(partial, 0, (size_t)groups * p.n1 * p.n2 * p.n3 * sizeof(double), st));
     for (int b0 = 0; b0 < nvec; b0 += chunk) {
         const int nb = nvec - b0 < chunk ? nvec - b0 : chunk;
         const double2* ps = psi + (long)b0 * ldpsi;
-        if (small3)
-            sticks_backward<double, kSmallR><<<dim3(nsg, nb), kStickThreads, smem_s, st>>>(p, ps, ldpsi, X);
-        else
-            sticks_backward<double, 16><<<dim3(nsg, nb), kStickThreads, smem_s, st>>>(p, ps, ldpsi, X);
-        Q3B_LAUNCH_CHECK();
+        run_sticks_backward<double>(p, ps, ldpsi, X, nb, st);
         const int gb = nb < groups ? nb : groups;
         // every chunk adds into the same slabs; a chunk with fewer bands than
         // groups leaves the remaining slabs as they are
-        if (small12)
+        if (sq_density(p, X, nb, w + b0, partial, gb, st, nullptr)) {
+        } else if (small12)
             planes_density<kSmallR><<<dim3(p.n3, gb), 256, smem_p, st>>>(p, X, nb, w + b0, partial, gb);
         else
             planes_density<16><<<dim3(p.n3, gb), 256, smem_p, st>>>(p, X, nb, w + b0, partial, gb);
@@ -509,7 +555,9 @@ void accumulate_density(cudaStream_t st, const LocalPlan<double>& p, const doubl
     const long n = (long)p.n1 * p.n2 * p.n3;
     int blocks = ceil_div(n, 256);
     if (blocks > 4096) blocks = 4096;
-    density_reduce<<<blocks, 256, 0, st>>>(p, groups, partial, rho);
+    int unused = 0;
+    const int reversed = sq_density(p, nullptr, 0, nullptr, nullptr, 0, nullptr, &unused) ? 0 : 1;
+    density_reduce<<<blocks, 256, 0, st>>>(p, groups, partial, rho, reversed);
     Q3B_LAUNCH_CHECK();
 }
 

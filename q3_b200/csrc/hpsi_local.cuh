@@ -32,6 +32,7 @@ template <typename R> struct LocalPlan {
     const int* entry_g;      // G index (caller's order) of each sphere entry
     const int* entry_w3;
     const int* entry_stick;
+    const int* entry_at;     // (stick % sg) * p3 + w3: its place in its block's lines
     const int* stick_pos;    // w1*p2 + w2
     const int* row_base;     // w1*p2 of each used row
     const int* unmapped_g;
@@ -62,6 +63,27 @@ template <typename R> struct LocalPlan {
 bool has_planes_reg(int n1, int n2, int lanes);
 template <typename R>
 bool launch_planes_reg(const LocalPlan<R>& p, cplx_t<R>* X, int nb, int lanes, cudaStream_t st, int* err);
+
+// the kernels for compile-time lengths (planes_sq.cuh): false where this plan's
+// plane or line length has none
+namespace psq {
+#define Q3B_SQ_DECLARE(NAME, R)                                                                          \
+    bool NAME##_planes(const LocalPlan<R>& p, cplx_t<R>* X, int nb, cudaStream_t st);                    \
+    bool NAME##_back(const LocalPlan<R>& p, const cplx_t<R>* psi, long ldpsi, cplx_t<R>* X, int nb,      \
+                     cudaStream_t st);                                                                   \
+    bool NAME##_fwd(const LocalPlan<R>& p, const cplx_t<R>* X, const cplx_t<R>* psi, long ldpsi,         \
+                    cplx_t<R>* hpsi, long ldh, int nb, cudaStream_t st);
+Q3B_SQ_DECLARE(f64_small, double)
+Q3B_SQ_DECLARE(f64_large, double)
+Q3B_SQ_DECLARE(f32_small, float)
+Q3B_SQ_DECLARE(f32_large, float)
+#undef Q3B_SQ_DECLARE
+// density planes (nb > 0), or the blocks an SM holds of them (nb == 0, *per_sm)
+bool f64_small_density(const LocalPlan<double>& p, const double2* X, int nb, const double* w, double* partial,
+                       int groups, cudaStream_t st, int* per_sm);
+bool f64_large_density(const LocalPlan<double>& p, const double2* X, int nb, const double* w, double* partial,
+                       int groups, cudaStream_t st, int* per_sm);
+}  // namespace psq
 
 // bytes of the stick buffer per band
 template <typename R> inline size_t sticks_bytes_per_band(const LocalPlan<R>& p) {
