@@ -9,119 +9,146 @@
 namespace q3b {
 namespace {
 
-constexpr int kBM = 64;
-constexpr int kBN = 64;
 constexpr int kThreads = 256;
+constexpr int kBK = 16;      // K per stage
+constexpr int kStages = 4;
+constexpr int kKP = kBK + 1;  // pitch of [m][k] and [n][k]
 
-template <typename R> struct GemmTile;
-template <> struct GemmTile<double> { static constexpr int BK = 8; };
-template <> struct GemmTile<float> { static constexpr int BK = 16; };
+// one complex value, global -> shared (zeros where not valid)
+template <typename T> __device__ __forceinline__ void cp_async(T* dst, const T* src, bool valid) {
+    const uint32_t d = static_cast<uint32_t>(__cvta_generic_to_shared(dst));
+    if constexpr (sizeof(T) == 16) {
+        const int n = valid ? 16 : 0;
+        asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(d), "l"(src), "r"(n) : "memory");
+    } else {
+        const int n = valid ? 8 : 0;
+        asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;" ::"r"(d), "l"(src), "r"(n) : "memory");
+    }
+}
+__device__ __forceinline__ void cp_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+template <int N> __device__ __forceinline__ void cp_wait() {
+    asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory");
+}
 
-// One BM x BN tile of C per block (64x64, or 32x32 for small products),
-// (BM/16) x (BN/16) complex outputs per thread.  With kchunk < K the block
-// handles K range [z*kchunk, (z+1)*kchunk) and writes its raw sum to part[z]
-// (ld M); otherwise it applies alpha/beta into C.
-template <typename R, bool CONJ_A, int BM = kBM, int BN = kBN>
+template <typename R, int TM, int TN> struct PipeTile {
+    static constexpr int bm = 16 * TM, bn = 16 * TN;
+    static constexpr int a_pitch_n = bm + 4;  // [k][m]
+    static constexpr int a_stage = kBK * a_pitch_n > bm * kKP ? kBK * a_pitch_n : bm * kKP;
+    static constexpr int b_stage = bn * kKP;
+    static constexpr size_t smem = (size_t)kStages * (a_stage + b_stage) * sizeof(cplx_t<R>);
+};
+
+// Products too small for the large tiles below: bm x bn tiles of C (32 x 16, 32 x 32
+// or 64 x 64), TM x TN outputs a thread, K in four cp.async stages of 16, so that
+// a block's K range is a few global latencies long.  With splits > 1 a block takes
+// one range of K and leaves its sums in `part`; the last block of a tile to finish
+// adds them in the order of the ranges (a fixed order, whichever block it is) and
+// clears the tile's counter for the next product, so no second launch is needed.
+// Bound: latency.  The 32 x 32 form it replaces staged 8 of K through registers
+// and summed the splits in a kernel of its own: 96 x 48 x 3000 (C,N) took 25 us,
+// 3000 x 48 x 96 (N,N) 19 us.
+template <typename R, bool CONJ_A, int TM, int TN>
 __global__ void __launch_bounds__(kThreads)
-cgemm_kernel(int M, int N, int K, cplx_t<R> alpha, const cplx_t<R>* __restrict__ A, long lda,
-             const cplx_t<R>* __restrict__ B, long ldb, cplx_t<R> beta, cplx_t<R>* C, long ldc,
-             int kchunk, cplx_t<R>* part) {
+cgemm_pipe(int M, int N, int K, cplx_t<R> alpha, const cplx_t<R>* __restrict__ A, long lda,
+           const cplx_t<R>* __restrict__ B, long ldb, cplx_t<R> beta, cplx_t<R>* C, long ldc, int kchunk,
+           cplx_t<R>* part, unsigned* counters) {
     using T = cplx_t<R>;
-    constexpr int BK = GemmTile<R>::BK;
-    constexpr int TM = BM / 16, TN = BN / 16;  // outputs per thread
-    constexpr int LA = (BK * BM + kThreads - 1) / kThreads;  // complex loads per thread, A tile
-    constexpr int LB = (BK * BN + kThreads - 1) / kThreads;
-    __shared__ T As[2][BK][BM + 1];
-    __shared__ T Bs[2][BK][BN + 1];
-
-    const int tid = threadIdx.x;
-    const int tx = tid % 16, ty = tid / 16;
+    using S = PipeTile<R, TM, TN>;
+    extern __shared__ __align__(16) unsigned char zsm[];
+    __shared__ int s_last;
+    T* As = reinterpret_cast<T*>(zsm);
+    T* Bs = As + kStages * S::a_stage;
+    const int tid = threadIdx.x, tx = tid % 16, ty = tid / 16;
     // N tiles run fastest: the blocks that share an A tile run together
-    const int m0 = blockIdx.y * BM, n0 = blockIdx.x * BN;
-    const int kbeg = blockIdx.z * kchunk;
-    const int kend = min(K, kbeg + kchunk);
+    const int m0 = blockIdx.y * S::bm, n0 = blockIdx.x * S::bn;
+    const int kbeg = blockIdx.z * kchunk, kend = min(K, kbeg + kchunk);
+    const int nk = kend > kbeg ? (kend - kbeg + kBK - 1) / kBK : 0;
+
+    auto fill = [&](int kb, int s) {
+        const int k0 = kbeg + kb * kBK;
+        T* as = As + s * S::a_stage;
+        T* bs = Bs + s * S::b_stage;
+#pragma unroll
+        for (int r = 0; r < S::bm * kBK / kThreads; ++r) {
+            const int idx = tid + r * kThreads;
+            const int k = CONJ_A ? idx % kBK : idx / S::bm, m = CONJ_A ? idx / kBK : idx % S::bm;
+            const int gk = k0 + k, gm = m0 + m;
+            const bool ok = gk < kend && gm < M;
+            cp_async(CONJ_A ? as + m * kKP + k : as + k * S::a_pitch_n + m,
+                     ok ? (CONJ_A ? A + gk + (long)gm * lda : A + gm + (long)gk * lda) : A, ok);
+        }
+#pragma unroll
+        for (int r = 0; r < S::bn * kBK / kThreads; ++r) {
+            const int idx = tid + r * kThreads;
+            const int k = idx % kBK, n = idx / kBK;
+            const int gk = k0 + k, gn = n0 + n;
+            const bool ok = gk < kend && gn < N;
+            cp_async(bs + n * kKP + k, ok ? B + gk + (long)gn * ldb : B, ok);
+        }
+    };
 
     T acc[TM][TN];
 #pragma unroll
     for (int i = 0; i < TM; ++i)
 #pragma unroll
         for (int j = 0; j < TN; ++j) acc[i][j] = czero<T>();
-
-    T ra[LA], rb[LB];
-    auto load = [&](int k0) {
 #pragma unroll
-        for (int r = 0; r < LA; ++r) {
-            const int idx = tid + r * kThreads;
-            int k, m;
-            if (CONJ_A) {
-                k = idx % BK;
-                m = idx / BK;
-            } else {
-                m = idx % BM;
-                k = idx / BM;
-            }
-            const int gk = k0 + k, gm = m0 + m;
-            T v = czero<T>();
-            if (idx < BK * BM && gk < kend && gm < M) {
-                v = CONJ_A ? conj2(A[gk + (long)gm * lda]) : A[gm + (long)gk * lda];
-            }
-            ra[r] = v;
-        }
-#pragma unroll
-        for (int r = 0; r < LB; ++r) {
-            const int idx = tid + r * kThreads;
-            const int k = idx % BK, n = idx / BK;
-            const int gk = k0 + k, gn = n0 + n;
-            rb[r] = (idx < BK * BN && gk < kend && gn < N) ? B[gk + (long)gn * ldb] : czero<T>();
-        }
-    };
-    auto store = [&](int buf) {
-#pragma unroll
-        for (int r = 0; r < LA; ++r) {
-            const int idx = tid + r * kThreads;
-            if (idx >= BK * BM) continue;
-            int k, m;
-            if (CONJ_A) {
-                k = idx % BK;
-                m = idx / BK;
-            } else {
-                m = idx % BM;
-                k = idx / BM;
-            }
-            As[buf][k][m] = ra[r];
-        }
-#pragma unroll
-        for (int r = 0; r < LB; ++r) {
-            const int idx = tid + r * kThreads;
-            if (idx >= BK * BN) continue;
-            Bs[buf][idx % BK][idx / BK] = rb[r];
-        }
-    };
-
-    int buf = 0;
-    if (kbeg < kend) {
-        load(kbeg);
-        store(0);
+    for (int s = 0; s < kStages - 1; ++s) {
+        if (s < nk) fill(s, s);
+        cp_commit();
     }
-    __syncthreads();
-    for (int k0 = kbeg; k0 < kend; k0 += BK) {
-        const bool more = (k0 + BK) < kend;
-        if (more) load(k0 + BK);
+    for (int kb = 0; kb < nk; ++kb) {
+        cp_wait<kStages - 2>();
+        __syncthreads();  // stage kb is complete for everyone; stage kb - 1 is free
+        const int nxt = kb + kStages - 1;
+        if (nxt < nk) fill(nxt, nxt % kStages);
+        cp_commit();
+        const T* as = As + (kb % kStages) * S::a_stage;
+        const T* bs = Bs + (kb % kStages) * S::b_stage;
 #pragma unroll
-        for (int kk = 0; kk < BK; ++kk) {
+        for (int kk = 0; kk < kBK; ++kk) {
             T a[TM], b[TN];
 #pragma unroll
-            for (int i = 0; i < TM; ++i) a[i] = As[buf][kk][ty + 16 * i];
+            for (int i = 0; i < TM; ++i) {
+                const T v = CONJ_A ? as[(ty + 16 * i) * kKP + kk] : as[kk * S::a_pitch_n + ty + 16 * i];
+                a[i] = CONJ_A ? conj2(v) : v;
+            }
 #pragma unroll
-            for (int j = 0; j < TN; ++j) b[j] = Bs[buf][kk][tx + 16 * j];
+            for (int j = 0; j < TN; ++j) b[j] = bs[(tx + 16 * j) * kKP + kk];
 #pragma unroll
             for (int i = 0; i < TM; ++i)
 #pragma unroll
                 for (int j = 0; j < TN; ++j) cfma(acc[i][j], a[i], b[j]);
         }
-        if (more) store(buf ^ 1);
+    }
+    cp_wait<0>();
+
+    if (gridDim.z > 1) {
+        const int tile = blockIdx.y * gridDim.x + blockIdx.x, tiles = gridDim.x * gridDim.y;
+        T* mine = part + ((size_t)blockIdx.z * tiles + tile) * (S::bm * S::bn) + tid;
+#pragma unroll
+        for (int i = 0; i < TM; ++i)
+#pragma unroll
+            for (int j = 0; j < TN; ++j) __stcg(mine + (i * TN + j) * kThreads, acc[i][j]);
+        __threadfence();
         __syncthreads();
-        buf ^= 1;
+        if (tid == 0) s_last = atomicAdd(counters + tile, 1u) == gridDim.z - 1;
+        __syncthreads();
+        if (!s_last) return;
+        __threadfence();
+        const T* first = part + (size_t)tile * (S::bm * S::bn) + tid;
+        const size_t step = (size_t)tiles * (S::bm * S::bn);
+#pragma unroll
+        for (int i = 0; i < TM; ++i)
+#pragma unroll
+            for (int j = 0; j < TN; ++j) acc[i][j] = czero<T>();
+#pragma unroll 4
+        for (int z = 0; z < (int)gridDim.z; ++z)
+#pragma unroll
+            for (int i = 0; i < TM; ++i)
+#pragma unroll
+                for (int j = 0; j < TN; ++j) acc[i][j] = acc[i][j] + __ldcg(first + z * step + (i * TN + j) * kThreads);
+        if (tid == 0) counters[tile] = 0;
     }
 
     const bool use_beta = (beta.x != R(0) || beta.y != R(0));
@@ -133,14 +160,10 @@ cgemm_kernel(int M, int N, int K, cplx_t<R> alpha, const cplx_t<R>* __restrict__
         for (int j = 0; j < TN; ++j) {
             const int gn = n0 + tx + 16 * j;
             if (gn >= N) continue;
-            if (part) {
-                part[(long)blockIdx.z * M * N + (long)gn * M + gm] = acc[i][j];
-            } else {
-                T v = cmul(alpha, acc[i][j]);
-                T* c = C + gm + (long)gn * ldc;
-                if (use_beta) v = v + cmul(beta, *c);
-                *c = v;
-            }
+            T v = cmul(alpha, acc[i][j]);
+            T* c = C + gm + (long)gn * ldc;
+            if (use_beta) v = v + cmul(beta, *c);
+            *c = v;
         }
     }
 }
@@ -164,15 +187,6 @@ template <int TM> struct Shape {   // BM = 16 TM rows of C per block
     static constexpr size_t smem = (size_t)STAGES * (a_stage + b_stage) * sizeof(double2);
 };
 
-__device__ __forceinline__ void cp16(void* dst, const void* src, bool valid) {
-    const uint32_t d = static_cast<uint32_t>(__cvta_generic_to_shared(dst));
-    const int n = valid ? 16 : 0;  // 0 bytes read: the 16 bytes are zero-filled
-    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(d), "l"(src), "r"(n) : "memory");
-}
-__device__ __forceinline__ void cp_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
-template <int N> __device__ __forceinline__ void cp_wait() {
-    asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory");
-}
 }  // namespace big
 
 template <bool CONJ_A, int TM>
@@ -206,12 +220,12 @@ zgemm_big(int M, int N, int K, double2 alpha, const double2* __restrict__ A, lon
                 const int k = idx % BK, m = idx / BK;
                 const int gk = k0 + k, gm = m0 + m;
                 const bool ok = gk < kend && gm < M;
-                cp16(as + m * KP + k, ok ? A + gk + (long)gm * lda : A, ok);
+                cp_async(as + m * KP + k, ok ? A + gk + (long)gm * lda : A, ok);
             } else {       // A is M x K: each k holds BM consecutive m
                 const int m = idx % BM, k = idx / BM;
                 const int gk = k0 + k, gm = m0 + m;
                 const bool ok = gk < kend && gm < M;
-                cp16(as + k * A_PITCH_N + m, ok ? A + gm + (long)gk * lda : A, ok);
+                cp_async(as + k * A_PITCH_N + m, ok ? A + gm + (long)gk * lda : A, ok);
             }
         }
         // B: BK x BN complex, 2 per thread; each n holds BK consecutive k
@@ -221,7 +235,7 @@ zgemm_big(int M, int N, int K, double2 alpha, const double2* __restrict__ A, lon
             const int k = idx % BK, n = idx / BK;
             const int gk = k0 + k, gn = n0 + n;
             const bool ok = gk < kend && gn < N;
-            cp16(bs + n * KP + k, ok ? B + gk + (long)gn * ldb : B, ok);
+            cp_async(bs + n * KP + k, ok ? B + gk + (long)gn * ldb : B, ok);
         }
     };
 
@@ -323,29 +337,64 @@ __global__ void splitk_reduce(int M, int N, int splits, const cplx_t<R>* __restr
     }
 }
 
-// Products whose 64x64 tiling has fewer tiles than the GPU has SMs (the
-// subspace eigensolver's n x n x n products up to n = 767) run on 32x32 tiles:
-// four times the blocks and a quarter of the serial K loop per block.
-inline bool small_tiles(int M, int N) { return (long)ceil_div(M, kBM) * ceil_div(N, kBN) < device_sms(); }
-
-// K splits for a product with `tiles` output tiles (never more than for
-// 64x64 tiles, which size the workspace)
-inline int choose_splits_for(int tiles, int K) {
-    const int target = 2 * device_sms();
-    int s = ceil_div(target, tiles);
-    const int kmax = ceil_div(K, 128);
-    if (s > kmax) s = kmax;
-    if (s < 1) s = 1;
-    if (s > 64) s = 64;
-    return s;
+// Clocks a product takes on the busiest SM, for choosing tiles and K ranges: a
+// block of a bm x bn tile spends 4 bm bn / 64 clocks of the FP64 units on a step
+// of K, at the share of their rate its kernel reaches (0.6 here, 0.72 with the
+// large tiles, both measured), and about `start` steps before and after them.
+constexpr double kPipeRate = 0.6, kBigRate = 0.72;
+constexpr int kPipeStart = 48, kBigStart = 30;
+inline double busiest(long blocks, int k, int start, int bm, int bn, double rate) {
+    const long sms = device_sms(), waves = (blocks + sms - 1) / sms;
+    return (double)waves * (k + start) * (bm * bn / 16.0) / rate;
 }
 
-template <typename R> int choose_splits(int M, int N, int K) {
-    return choose_splits_for(ceil_div(M, kBM) * ceil_div(N, kBN), K);
+// The tile and the K ranges of a product on the pipelined tiles.
+//   tile: 64 x 64 or 32 x 32, whichever takes fewer clocks; 32 x 16 where 32
+//     columns would leave a quarter or more of them empty;
+//   ranges (C,N only): the count with the least clocks, each costing two steps of K
+//     for its share of the sum.  At most 64, of at least 32 steps, and as many tiles
+//     as there are counters.
+struct PipePlan {
+    int tm, tn, splits, kchunk;
+    size_t part;   // complex values of the partial sums
+    double clocks;
+};
+PipePlan pipe_plan(bool conj_a, int M, int N, int K) {
+    PipePlan best{2, 2, 1, K, 0, -1.0};
+    auto consider = [&](int tm, int tn) {
+        const int bm = 16 * tm, bn = 16 * tn;
+        const long tiles = (long)ceil_div(M, bm) * ceil_div(N, bn);
+        for (int s = 1; s == 1 || (conj_a && tiles <= GemmWorkspace::kCounters && s <= 64 && K >= 32 * s); ++s) {
+            const double c = busiest(tiles * s, ceil_div(K, s), kPipeStart, bm, bn, kPipeRate) +
+                             (s > 1 ? 2.0 * s * (bm * bn / 16.0) : 0.0);
+            if (best.clocks >= 0.0 && c >= best.clocks) continue;
+            best = PipePlan{tm, tn, 1, K, 0, c};
+            if (s > 1) {
+                best.kchunk = ceil_div(ceil_div(K, s), kBK) * kBK;
+                best.splits = ceil_div(K, best.kchunk);
+                best.part = best.splits > 1 ? (size_t)best.splits * tiles * (256 * tm * tn) : 0;
+            }
+        }
+    };
+    consider(2, ceil_div(N, 16) * 16 * 4 <= ceil_div(N, 32) * 32 * 3 ? 1 : 2);
+    consider(4, 4);
+    return best;
 }
 
-// FP64 products of at least one 128 x 64 tile take zgemm_big
-inline bool big_tiles(int M, int N) { return M >= big::BM && N >= big::BN; }
+template <typename R, bool CONJ_A, int TM, int TN>
+void pipe_run(cudaStream_t st, dim3 grid, int M, int N, int K, cplx_t<R> alpha, const cplx_t<R>* A, long lda,
+              const cplx_t<R>* B, long ldb, cplx_t<R> beta, cplx_t<R>* C, long ldc, int kchunk, cplx_t<R>* part,
+              unsigned* counters) {
+    constexpr size_t smem = PipeTile<R, TM, TN>::smem;
+    static PerDeviceOnce once;
+    once.run([] {
+        Q3B_CUDA(cudaFuncSetAttribute(cgemm_pipe<R, CONJ_A, TM, TN>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                      (int)PipeTile<R, TM, TN>::smem));
+    });
+    cgemm_pipe<R, CONJ_A, TM, TN><<<grid, kThreads, smem, st>>>(M, N, K, alpha, A, lda, B, ldb, beta, C, ldc, kchunk,
+                                                                part, counters);
+    Q3B_LAUNCH_CHECK();
+}
 
 // K splits of a large-tile C,N product: at most 64, at most one per 256 of K,
 // and a workspace of at most 64 MB
@@ -355,6 +404,35 @@ inline int big_max_splits(int M, int N, int K) {
     long s = std::min<long>(64, ceil_div(K, 256));
     s = std::min(s, by_ws);
     return s < 1 ? 1 : static_cast<int>(s);
+}
+
+// The tile height (128 or 96 rows) and K ranges of zgemm_big: the least rows of
+// work per SM over whole waves; a C,N product splits K into as many chunks as fill
+// whole waves (at least two, at most 64).
+struct BigPlan {
+    int tm, splits;
+    double clocks;
+};
+BigPlan big_plan(bool conj_a, int M, int N, int K) {
+    BigPlan best{8, 1, -1.0};
+    const int most = conj_a ? big_max_splits(M, N, K) : 1;
+    for (int tm : {8, 6}) {
+        const long tiles = (long)ceil_div(M, 16 * tm) * ceil_div(N, big::BN);
+        for (int s = 1; s <= most; ++s) {
+            const double c = busiest(tiles * s, ceil_div(K, s), kBigStart, 16 * tm, big::BN, kBigRate);
+            if (best.clocks < 0.0 || c < best.clocks) best = BigPlan{tm, s, c};
+        }
+    }
+    // the split sums' own kernel, about 5 us
+    if (best.splits > 1) best.clocks += 1e4;
+    return best;
+}
+
+// FP64 products of at least one 128 x 64 tile take the large tiles where these
+// are the faster: 23847 x 256 x 512 (N,N) and 256 x 128 x 12000 (C,N) do;
+// 3000 x 96 x 96 (38 us there), 128 x 64 x 6000 (87) and 160 x 80 x 9000 (89) do not
+inline bool big_tiles(bool conj_a, int M, int N, int K) {
+    return M >= big::BM && N >= big::BN && big_plan(conj_a, M, N, K).clocks < pipe_plan(conj_a, M, N, K).clocks;
 }
 
 template <bool CONJ_A, int TM>
@@ -373,45 +451,12 @@ void zgemm_big_run(cudaStream_t st, dim3 grid, int M, int N, int K, double2 alph
     Q3B_LAUNCH_CHECK();
 }
 
-// One 256-thread block of zgemm_big per SM, so the launch runs in waves of
-// `sms` blocks.  The tile height (128 or 96 rows) is the one with the least
-// rows of work per SM over whole waves; a C,N product splits K into as many
-// chunks as fill whole waves (at least two, at most 64).
 void zgemm_big_launch(cudaStream_t st, bool conj_a, int M, int N, int K, double2 alpha, const double2* A,
                       long lda, const double2* B, long ldb, double2 beta, double2* C, long ldc,
                       const GemmWorkspace& ws) {
-    const int sms = device_sms();
-    auto waves = [&](long units) { return (units + sms - 1) / sms; };
-    const int t128 = ceil_div(M, 128) * ceil_div(N, big::BN), t96 = ceil_div(M, 96) * ceil_div(N, big::BN);
-    int splits = 1, tm = 8, tiles = t128;
-    if (conj_a) {
-        // the waves of split blocks, per tile height
-        auto best_split = [&](int t, int& s_out) {
-            long best = -1;
-            const int kmax = big_max_splits(M, N, K);
-            for (int s = 1; s <= kmax; ++s) {
-                const long cost = waves((long)t * s) * ((long)ceil_div(K, s));  // K steps of the busiest SM
-                if (best < 0 || cost < best) {
-                    best = cost;
-                    s_out = s;
-                }
-            }
-            return best;
-        };
-        int s128 = 1, s96 = 1;
-        const long c128 = best_split(t128, s128) * 128, c96 = best_split(t96, s96) * 96;
-        if (c96 < c128) {
-            tm = 6;
-            splits = s96;
-            tiles = t96;
-        } else {
-            splits = s128;
-        }
-    } else if (waves(t96) * 96 < waves(t128) * 128) {
-        tm = 6;
-        tiles = t96;
-    }
-    (void)tiles;
+    const BigPlan plan = big_plan(conj_a, M, N, K);
+    const int tm = plan.tm;
+    int splits = plan.splits;
     const size_t need = (size_t)splits * M * N * sizeof(double2);
     if (splits > 1 && (ws.ptr == nullptr || ws.bytes < need)) splits = 1;
     int kchunk = K;
@@ -446,10 +491,17 @@ void zgemm_big_launch(cudaStream_t st, bool conj_a, int M, int N, int K, double2
 bool use_tensor_cores(int M, int N, int K) { return (double)M * N * K >= kTensorCoreMinMacs; }
 
 template <typename R> size_t cgemm_workspace_bytes(int M, int N, int K) {
-    const int s = std::max(choose_splits<R>(M, N, K), big_max_splits(M, N, K));
-    const size_t simt = s > 1 ? (size_t)s * M * N * sizeof(cplx_t<R>) : 0;
+    size_t simt = pipe_plan(true, M, N, K).part * sizeof(cplx_t<R>);
     if constexpr (std::is_same<R, float>::value) return std::max(simt, tc::workspace_bytes(M, N, K));
+    const int s = big_max_splits(M, N, K);
+    if (big_tiles(true, M, N, K) && s > 1) simt = std::max(simt, (size_t)s * M * N * sizeof(cplx_t<R>));
     return simt;
+}
+
+double fp64_units_seconds(bool conj_a, int M, int N, int K) {
+    double clocks = pipe_plan(conj_a, M, N, K).clocks;
+    if (M >= big::BM && N >= big::BN) clocks = std::min(clocks, big_plan(conj_a, M, N, K).clocks);
+    return clocks / 1.93e9 + 4e-6;
 }
 
 template <typename R> size_t cgemm_wanted_bytes(bool conj_a, int M, int N, int K) {
@@ -465,7 +517,6 @@ void cgemm(cudaStream_t st, bool conj_a, int M, int N, int K, cplx_t<R> alpha, c
            const GemmWorkspace& ws) {
     using T = cplx_t<R>;
     if (M <= 0 || N <= 0) return;
-    constexpr int BK = GemmTile<R>::BK;
     if constexpr (std::is_same<R, float>::value) {
         // small products stay on the CUDA cores: a tensor-core block takes a
         // whole SM's shared memory, which small problems, often several at
@@ -489,48 +540,31 @@ void cgemm(cudaStream_t st, bool conj_a, int M, int N, int K, cplx_t<R> alpha, c
             zmod::zgemm(st, conj_a, M, N, K, alpha, A, lda, nullptr, B, ldb, beta, C, ldc, ws);
             return;
         }
-        if (big_tiles(M, N) && reinterpret_cast<uintptr_t>(A) % 16 == 0 &&
+        if (big_tiles(conj_a, M, N, K) && reinterpret_cast<uintptr_t>(A) % 16 == 0 &&
             reinterpret_cast<uintptr_t>(B) % 16 == 0) {
             zgemm_big_launch(st, conj_a, M, N, K, alpha, A, lda, B, ldb, beta, C, ldc, ws);
             return;
         }
     }
-    const bool small = small_tiles(M, N);
-    const int bm = small ? 32 : kBM;
-    int splits = conj_a ? choose_splits_for(ceil_div(M, bm) * ceil_div(N, bm), K) : 1;
-    size_t need = (size_t)splits * M * N * sizeof(T);
-    if (splits > 1 && (ws.ptr == nullptr || ws.bytes < need)) splits = 1;
-    int kchunk = K;
-    if (splits > 1) {
-        kchunk = ceil_div(K, splits);
-        kchunk = ceil_div(kchunk, BK) * BK;
-        splits = ceil_div(K, kchunk);
+    PipePlan p = pipe_plan(conj_a, M, N, K);
+    if (p.splits > 1 && (!ws.ptr || !ws.counters || ws.bytes < p.part * sizeof(T))) {
+        p.splits = 1;
+        p.kchunk = K;
     }
-    if (ceil_div(M, bm) > 65535) throw std::runtime_error("complex GEMM: M too large");
-    dim3 grid(ceil_div(N, bm), ceil_div(M, bm), splits);
-    T* part = splits > 1 ? static_cast<T*>(ws.ptr) : nullptr;
-    if (small) {
-        if (conj_a)
-            cgemm_kernel<R, true, 32, 32><<<grid, kThreads, 0, st>>>(M, N, K, alpha, A, lda, B, ldb, beta,
-                                                                    C, ldc, kchunk, part);
+    if (ceil_div(M, 16 * p.tm) > 65535) throw std::runtime_error("complex GEMM: M too large");
+    const dim3 grid(ceil_div(N, 16 * p.tn), ceil_div(M, 16 * p.tm), p.splits);
+    T* part = p.splits > 1 ? static_cast<T*>(ws.ptr) : nullptr;
+    auto run = [&](auto conj) {
+        constexpr bool CA = decltype(conj)::value;
+        if (p.tm == 4)
+            pipe_run<R, CA, 4, 4>(st, grid, M, N, K, alpha, A, lda, B, ldb, beta, C, ldc, p.kchunk, part, ws.counters);
+        else if (p.tn == 2)
+            pipe_run<R, CA, 2, 2>(st, grid, M, N, K, alpha, A, lda, B, ldb, beta, C, ldc, p.kchunk, part, ws.counters);
         else
-            cgemm_kernel<R, false, 32, 32><<<grid, kThreads, 0, st>>>(M, N, K, alpha, A, lda, B, ldb,
-                                                                     beta, C, ldc, kchunk, part);
-    } else if (conj_a) {
-        cgemm_kernel<R, true><<<grid, kThreads, 0, st>>>(M, N, K, alpha, A, lda, B, ldb, beta, C,
-                                                         ldc, kchunk, part);
-    } else {
-        cgemm_kernel<R, false><<<grid, kThreads, 0, st>>>(M, N, K, alpha, A, lda, B, ldb, beta, C,
-                                                          ldc, kchunk, part);
-    }
-    Q3B_LAUNCH_CHECK();
-    if (splits > 1) {
-        const long total = (long)M * N;
-        int blocks = ceil_div(total, 256);
-        if (blocks > 4096) blocks = 4096;
-        splitk_reduce<R><<<blocks, 256, 0, st>>>(M, N, splits, part, alpha, beta, C, ldc);
-        Q3B_LAUNCH_CHECK();
-    }
+            pipe_run<R, CA, 2, 1>(st, grid, M, N, K, alpha, A, lda, B, ldb, beta, C, ldc, p.kchunk, part, ws.counters);
+    };
+    if (conj_a) run(std::true_type{});
+    else run(std::false_type{});
 }
 
 double measure_dfma_tflops(cudaStream_t st) {

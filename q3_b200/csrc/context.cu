@@ -145,6 +145,8 @@ Context::Context(int dev, size_t hbm_budget) : device(dev), budget(hbm_budget) {
     stream = own_stream;
     err_word.reserve(this, 4 * sizeof(int));
     Q3B_CUDA(cudaMemsetAsync(err_word.ptr, 0, 4 * sizeof(int), stream));
+    gemm_counters.reserve(this, GemmWorkspace::kCounters * sizeof(unsigned));
+    Q3B_CUDA(cudaMemsetAsync(gemm_counters.ptr, 0, gemm_counters.bytes, stream));
     Q3B_CUDA(cudaStreamSynchronize(stream));
 }
 
@@ -182,7 +184,7 @@ GemmWorkspace Context::gemm_ws(size_t need, size_t want) {
         if (!ws_gemm.try_reserve(this, want) && in_budget) ws_gemm_refused_ = want;
     }
     ws_gemm.reserve(this, need);
-    return GemmWorkspace{ws_gemm.ptr, ws_gemm.bytes};
+    return GemmWorkspace{ws_gemm.ptr, ws_gemm.bytes, gemm_counters.as<unsigned>()};
 }
 
 bool Context::release_optional() {

@@ -82,6 +82,7 @@ class Context {
     std::vector<double> v_host;     // V(r) as given, reference layout
     DevBuf v64, v32;                // V/N, [w3 pos][w1][w2 pos] (see LocalPlan::vplane)
     DevBuf v64nat, v32nat;          // V/N, [w3 pos][w1][w2] (LocalPlan::vnat)
+    DevBuf gemm_counters;           // GemmWorkspace::counters of this context's products
     DevBuf err_word;                // device error word of this context's kernels (bounded waits)
 
     KPoint kp;

@@ -822,24 +822,20 @@ void pack_a(cudaStream_t st, int M, int K, const double2* A, long lda, bool kmaj
 }
 
 // Estimated times of both paths, from runs of q3b_gemm on shapes of the 8- to
-// 128-atom cells (B200, 1965 MHz).  Here: 19 ps per packed entry, 60 ns per tile
-// and K block, 10 ps per output, and 40 us of launches.  On the FP64 units:
-// 23 TFLOP/s on tiles of 64 x 64 (13 for narrow ones), the split sums' 15 us, and
-// 0.29 us per K of an unsplit product, however few its tiles.  Measured, here
-// against there: 23847 x 256 x 512 (N,N) 0.49 ms against 1.12, 512 x 256 x 23847
-// (C,N) 0.53 against 0.97, 1024 x 512 x 62669 3.6 against 10.2; the two meet near
-// 23847 x 64 x 512 (0.33 against 0.33) and 12000 x 128 x 256 (0.15 against 0.17).
-// With A packed before (the projectors), beta Q beta^H psi of 90 bands of the
-// 64-atom cell takes 0.39 ms against 1.14.
+// 128-atom cells (B200, 1965 MHz): here 19 ps per packed entry, 60 ns per 128 x 64
+// tile and K block, 10 ps per output, and 40 us of launches; on the FP64 units as
+// their own tiles are chosen.  Measured, here against there: 23847 x 256 x 512
+// (N,N) 0.49 ms against 1.12, 512 x 256 x 23847 (C,N) 0.53 against 0.97,
+// 1024 x 512 x 62669 3.6 against 10.2; the two meet near 23847 x 64 x 512 (0.33
+// against 0.33) and 12000 x 128 x 256 (0.15 against 0.17).  With A packed before
+// (the projectors), beta Q beta^H psi of 90 bands of the 64-atom cell takes 0.39 ms
+// against 1.14.
 bool worth(bool conj_a, int M, int N, int K, bool packed) {
     if (M < 64 || N < 16 || K < 64) return false;
     const double tiles = (double)ceil_div(M, 2 * BM) * (narrow(N) ? 2 : 4 * ceil_div(N, 128)) * ceil_div(K, BK);
     const double entries = (double)K * N + (packed ? 0.0 : (double)M * K);
     const double here = 40e-6 + 19e-12 * entries + 60e-9 * tiles + 10e-12 * (double)M * N;
-    const double flops = 8.0 * ceil_div(M, 64) * ceil_div(N, 64) * 4096.0 * K;
-    const double rate = M >= 128 && (N >= 64 || conj_a) ? 23e12 : 13e12;
-    const double there = conj_a ? flops / rate + 15e-6 : std::fmax(flops / rate, 0.29e-6 * K);
-    return here < there;
+    return here < fp64_units_seconds(conj_a, M, N, K);
 }
 
 size_t workspace_bytes(bool conj_a, int M, int N, int K, bool packed) {
