@@ -281,48 +281,52 @@ __global__ void copy_matrix(int n, const double2* src, int lds, double2* dst, in
 
 inline int grid_for(long n) { return stride_grid(n, 8); }
 
-// ------------------------------------------------------------ grid barrier
-// One monotonic arrival counter: the e-th barrier of a launch completes when
-// the counter reaches e * nblocks.  Every wait is bounded (about 2 s of
-// clock), after which the kernel records an error and all blocks leave.
-__device__ unsigned& grid_epoch() {
-    __shared__ unsigned s_epoch;
-    return s_epoch;
+// ------------------------------------------------------------ exchange between blocks
+// A published complex value is 32 bytes: each of its four 32-bit words beside a
+// word that holds the step it belongs to, so a reader that sees the step in
+// every pair has the value, with no fence and no separate flag to wait for (8-byte
+// halves of a vector access are single copies).  Steps count from 1; the buffers
+// are zeroed before the launch.
+struct Published {
+    uint4 re, im;  // {low word, step, high word, step}
+};
+__device__ __forceinline__ void publish(Published* at, double2 v, unsigned step) {
+    const unsigned r0 = __double2loint(v.x), r1 = __double2hiint(v.x), i0 = __double2loint(v.y),
+                   i1 = __double2hiint(v.y);
+    asm volatile("st.volatile.global.v4.u32 [%0], {%1, %2, %3, %2};" ::"l"(&at->re), "r"(r0), "r"(step), "r"(r1)
+                 : "memory");
+    asm volatile("st.volatile.global.v4.u32 [%0], {%1, %2, %3, %2};" ::"l"(&at->im), "r"(i0), "r"(step), "r"(i1)
+                 : "memory");
 }
-__device__ __forceinline__ void grid_sync_init() {
-    if (threadIdx.x == 0) grid_epoch() = 0;
+__device__ __forceinline__ uint4 load_pairs(const uint4* at) {
+    uint4 v;
+    asm volatile("ld.volatile.global.v4.u32 {%0, %1, %2, %3}, [%4];"
+                 : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w)
+                 : "l"(at)
+                 : "memory");
+    return v;
 }
-__device__ __forceinline__ bool grid_sync(unsigned* bar, unsigned nblocks, int* err) {
-    __shared__ int s_ok;
-    unsigned& s_epoch = grid_epoch();
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        const unsigned epoch = s_epoch + 1;  // barriers this block has entered
-        s_epoch = epoch;
-        __threadfence();
-        atomicAdd(bar, 1u);
-        const unsigned target = epoch * nblocks;
-        int ok = 1;
-        const long long t0 = clock64();
-        while (true) {
-            unsigned cur;
-            asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(cur) : "l"(bar) : "memory");
-            if (cur >= target) break;
-            if (vload(err)) {
-                ok = 0;
-                break;
-            }
-            if (clock64() - t0 > (1LL << 32)) {
-                atomicExch(err, 1);
-                ok = 0;
-                break;
-            }
+// one look: true with the value once it is there
+__device__ __forceinline__ bool look(const Published* at, unsigned step, double2& v) {
+    const uint4 a = load_pairs(&at->re), b = load_pairs(&at->im);
+    v = mk(__hiloint2double(a.z, a.x), __hiloint2double(b.z, b.x));
+    return a.y == step && a.w == step && b.y == step && b.w == step;
+}
+// Every wait is bounded (about 2 s of clock), after which the kernel records an
+// error and all blocks leave.
+struct Patience {
+    long long t0;
+    unsigned spins;
+    __device__ __forceinline__ bool exhausted(int* err) {
+        if ((++spins & 255u) != 0) return false;
+        if (vload(err)) return true;
+        if (clock64() - t0 > (1LL << 32)) {
+            atomicExch(err, 1);
+            return true;
         }
-        s_ok = ok;
+        return false;
     }
-    __syncthreads();
-    return s_ok != 0;
-}
+};
 
 // ------------------------------------------------------------------ hetrd
 // A (n x n, ld n, full Hermitian; read once) reduced to tridiagonal form by
@@ -333,50 +337,65 @@ __device__ __forceinline__ bool grid_sync(unsigned* bar, unsigned nblocks, int* 
 // shared memory for the whole reduction, and its columns of W too when they
 // fit (`w_in_smem`), else in global memory.
 //
-// One grid barrier per column step.  Before it, every block publishes its
-// entries of p = tau A v and its share of v^H p, and the owner of column k+1
-// publishes that column as it stands before step k's update.  After it, every
-// block reads the three together (one L2 latency), forms w, and applies step
-// k's rank-2 update to its own copy of column k+1, which is the next step's
-// Householder input: no block waits for another between the barriers.  The
-// published vectors are double-buffered by step parity; a block can run at
-// most one step ahead of another (the next barrier holds it), so nothing is
-// overwritten while it is still being read.  Every wait is bounded.
-__global__ void __launch_bounds__(256, 1)
+// One exchange per column step.  Every block publishes its entries of
+// p = tau A v as its warps form them, and the owner of column k+1 publishes that
+// column as it stands before step k's update; every block polls for all of
+// both, forms w, and applies step k's rank-2 update to its own copy of column
+// k+1, which is the next step's Householder input.  While the first eight warps
+// form p the other eight apply the reflector to the block's columns of W, which
+// needs no exchange.  The published vectors are double-buffered by step parity:
+// `seen` tells that a block has done with the step before, and nobody goes on
+// to write the step after before all have said so.  Bound: the chain of
+// latencies of a step (two block sums, the reflector's square root and
+// division, one L2 write and read, the update), not work: 3.9 us at n = 96 and
+// 5.5 us at n = 512 with a counting grid barrier between the writes and
+// reads, which cost a fence, an atomic and a second L2 read, and W after it.
+constexpr int kHetrdThreads = 512;
+constexpr int kHetrdEntries = 3;  // of a vector a thread holds: orders up to 1536
+__global__ void __launch_bounds__(kHetrdThreads, 1)
 hetrd_smem(int n, int cpb, int w_in_smem, const double2* A, double* d, double2* e, double2* W,
-           double2* xpre2, double2* pbuf2, double2* partial2, unsigned* bar, int* err) {
+           Published* xpre2, Published* pbuf2, unsigned* seen, int* err) {
     extern __shared__ __align__(16) unsigned char smem[];
     double2* cols = reinterpret_cast<double2*>(smem);   // cpb columns of A
-    double2* sv = cols + (size_t)cpb * n;              // v
-    double2* sw = sv + n;                              // w
+    double2* sv2 = cols + (size_t)cpb * n;             // v, by step parity
+    double2* sw = sv2 + 2 * (size_t)n;                 // w
     double2* sx = sw + n;                              // column k, rows k.. (the next v)
     double2* wsm = sx + n;                             // cpb columns of W (if w_in_smem)
-    __shared__ double red[8];
-    __shared__ double2 redc[8];
-    __shared__ double s_tau;
+    constexpr int WARPS = kHetrdThreads / 32, HALF = WARPS / 2;
+    __shared__ double red[WARPS], redp[WARPS];
+    __shared__ double2 s_p0;
+    __shared__ int s_stop;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int G = gridDim.x, b = blockIdx.x;
     const int owned = b < n ? (n - b + G - 1) / G : 0;
-    grid_sync_init();
+    if (tid == 0) s_stop = 0;
     auto wcol = [&](int jj) -> double2* { return w_in_smem ? wsm + (size_t)jj * n : W + (size_t)(b + G * jj) * n; };
     for (int jj = 0; jj < owned; ++jj) {
         const int c = b + G * jj;
         double2* wc = wcol(jj);
-        for (int r = tid; r < n; r += blockDim.x) {
+        for (int r = tid; r < n; r += kHetrdThreads) {
             cols[(size_t)jj * n + r] = A[r + (size_t)c * n];
             wc[r] = (r == c) ? mk(1.0, 0.0) : mk(0.0, 0.0);
         }
     }
-    for (int r = tid; r < n; r += blockDim.x) sx[r] = A[r];  // column 0
+    for (int r = tid; r < n; r += kHetrdThreads) sx[r] = A[r];  // column 0
     __syncthreads();
     for (int k = 0; k + 1 < n; ++k) {
         const int m = n - k - 1;
         const int par = k & 1;
-        double2* pbuf = pbuf2 + (size_t)par * n;
-        double2* partial = partial2 + (size_t)par * G;
-        double2* xpre = xpre2 + (size_t)par * n;
+        const unsigned step = k + 1;
+        Published* pbuf = pbuf2 + (size_t)par * n;
+        Published* xpre = xpre2 + (size_t)par * n;
+        double2* sv = sv2 + (size_t)par * n;
+        // this block has read everything of the step before
+        if (tid == 0) *const_cast<volatile unsigned*>(seen + b) = step;
+        // the owner of column k+1 publishes it as it stands before this step
+        if ((k + 1) % G == b) {
+            const double2* col = cols + (size_t)((k + 1) / G) * n + (k + 1);
+            for (int j = tid; j < m; j += kHetrdThreads) publish(&xpre[j], col[j], step);
+        }
         double part = 0.0;
-        for (int j = tid; j < m; j += blockDim.x) {
+        for (int j = tid; j < m; j += kHetrdThreads) {
             const double2 x = sx[k + 1 + j];
             sv[j] = x;
             if (j > 0) part += x.x * x.x + x.y * x.y;
@@ -384,94 +403,118 @@ hetrd_smem(int n, int cpb, int w_in_smem, const double2* A, double* d, double2* 
         part = warp_sum(part);
         if (lane == 0) red[warp] = part;
         __syncthreads();
-        if (tid == 0) {
-            double sigma = 0.0;
-            for (int q = 0; q < 8; ++q) sigma += red[q];
-            const double2 x0 = sv[0];
-            double t = 0.0;
-            double2 alpha = x0;
-            if (m > 1 && sigma > 0.0) {
-                const double ax0 = hypot(x0.x, x0.y);
-                const double nrm = sqrt(sigma + ax0 * ax0);
-                alpha = ax0 > 0.0 ? mk(-nrm * x0.x / ax0, -nrm * x0.y / ax0) : mk(-nrm, 0.0);
-                const double2 v0 = x0 - alpha;
-                t = 2.0 / (sigma + v0.x * v0.x + v0.y * v0.y);
-                sv[0] = v0;
-            }
-            s_tau = t;
-            if (b == 0) {
-                d[k] = sx[k].x;
-                e[k] = alpha;
-            }
+        // the reflector, by every thread: v = x - alpha e_0 with alpha = -|x| x_0 / |x_0|,
+        // tau = 2 / |v|^2 = 1 / (|x|^2 + |x| |x_0|)
+        double sigma = 0.0;
+#pragma unroll
+        for (int q = 0; q < WARPS; ++q) sigma += red[q];
+        const double2 x0 = sx[k + 1];
+        double tk = 0.0;
+        double2 alpha = x0;
+        if (m > 1 && sigma > 0.0) {
+            const double a2 = x0.x * x0.x + x0.y * x0.y, n2 = sigma + a2, nrm = sqrt(n2);
+            // (below 1e-290 the square is no longer accurate, and x_0 counts for nothing)
+            const double ra = a2 > 1e-290 ? rsqrt(a2) : 0.0, ax0 = a2 * ra;
+            alpha = ra > 0.0 ? mk(-nrm * (x0.x * ra), -nrm * (x0.y * ra)) : mk(-nrm, 0.0);
+            tk = 1.0 / fma(nrm, ax0, n2);
+            if (tid == 0) sv[0] = x0 - alpha;
         }
-        // the owner of column k+1 publishes it as it stands before this step
-        if ((k + 1) % G == b) {
-            const double2* col = cols + (size_t)((k + 1) / G) * n + (k + 1);
-            for (int j = tid; j < m; j += blockDim.x) xpre[j] = col[j];
-        }
-        __syncthreads();
-        const double tk = s_tau;
-        // p_i = tau (column i)^H v for the owned columns i > k; this block's share of v^H p
-        double2 acc = mk(0.0, 0.0);
-        if (tk != 0.0) {
-            for (int jj = warp; jj < owned; jj += 8) {
-                const int i = b + G * jj;
-                if (i <= k) continue;
-                const double2* col = cols + (size_t)jj * n + (k + 1);
-                double2 sacc = mk(0.0, 0.0);
-                for (int j = lane; j < m; j += 32) sacc = sacc + cmulc(col[j], sv[j]);
-                sacc = warp_sum(sacc);
-                const double2 p = mk(tk * sacc.x, tk * sacc.y);
-                if (lane == 0) pbuf[i] = p;
-                acc = acc + cmulc(sv[i - k - 1], p);
-            }
-        }
-        if (lane == 0) redc[warp] = acc;
-        __syncthreads();
-        if (tid == 0) {
-            double2 sacc = mk(0.0, 0.0);
-            for (int q = 0; q < 8; ++q) sacc = sacc + redc[q];
-            partial[b] = sacc;
-        }
-        if (!grid_sync(bar, G, err)) return;
-        // column k+1 before the update, p and the shares, read together
-        for (int j = tid; j < m; j += blockDim.x) {
-            sx[k + 1 + j] = __ldcg(&xpre[j]);
-            if (tk != 0.0) sw[j] = __ldcg(&pbuf[k + 1 + j]);
-        }
-        if (tk != 0.0 && warp == 0) {
-            double2 sacc = mk(0.0, 0.0);
-            for (int q = lane; q < G; q += 32) sacc = sacc + __ldcg(&partial[q]);
-            sacc = warp_sum(sacc);
-            if (lane == 0) redc[0] = sacc;
+        if (b == 0 && tid == 0) {
+            d[k] = sx[k].x;
+            e[k] = alpha;
         }
         __syncthreads();
         if (tk != 0.0) {
-            const double half = 0.5 * tk * redc[0].x;  // v^H p is real
-            for (int j = tid; j < m; j += blockDim.x) {
-                const double2 p = sw[j];
-                sw[j] = mk(p.x - half * sv[j].x, p.y - half * sv[j].y);
-            }
-            __syncthreads();
-            // the next step's column: A[k+1+j, k+1] -= v_j conj(w_0) + w_j conj(v_0)
-            {
-                const double2 v0 = sv[0], w0 = sw[0];
-                for (int j = tid; j < m; j += blockDim.x) {
-                    const double2 u = cmul(sv[j], conj2(w0)) + cmul(sw[j], conj2(v0));
-                    sx[k + 1 + j] = sx[k + 1 + j] - u;
+            if (warp < HALF) {
+                // p_i = tau (column i)^H v for the owned columns i > k
+                for (int jj = warp; jj < owned; jj += HALF) {
+                    const int i = b + G * jj;
+                    if (i <= k) continue;
+                    const double2* col = cols + (size_t)jj * n + (k + 1);
+                    double2 sacc = mk(0.0, 0.0);
+                    for (int j = lane; j < m; j += 32) sacc = sacc + cmulc(col[j], sv[j]);
+                    sacc = warp_sum(sacc);
+                    if (lane == 0) publish(&pbuf[i], mk(tk * sacc.x, tk * sacc.y), step);
+                }
+            } else {
+                // W[k+1:, i] -= tau v (v^H W[k+1:, i])
+                for (int jj = warp - HALF; jj < owned; jj += HALF) {
+                    double2* wc = wcol(jj) + (k + 1);
+                    double2 sacc = mk(0.0, 0.0);
+                    for (int j = lane; j < m; j += 32) sacc = sacc + cmulc(sv[j], wc[j]);
+                    sacc = warp_sum(sacc);
+                    const double2 f = mk(tk * sacc.x, tk * sacc.y);
+                    for (int j = lane; j < m; j += 32) wc[j] = wc[j] - cmul(sv[j], f);
                 }
             }
-            for (int jj = warp; jj < owned; jj += 8) {
+        }
+        // column k+1 before the update, p, and that every block has done with the step before
+        double2 xr[kHetrdEntries], pr[kHetrdEntries];
+        {
+            Patience patience{clock64(), 0};
+            bool stop = false;
+            unsigned todo = 0;
+#pragma unroll
+            for (int u = 0; u < kHetrdEntries; ++u)
+                if (tid + u * kHetrdThreads < m) todo |= (tk != 0.0 ? 3u : 1u) << (2 * u);
+            bool wait_seen = tid < G;
+            while ((todo || wait_seen) && !stop) {
+#pragma unroll
+                for (int u = 0; u < kHetrdEntries; ++u) {
+                    const int j = tid + u * kHetrdThreads;
+                    if ((todo >> (2 * u)) & 1u)
+                        if (look(&xpre[j], step, xr[u])) todo &= ~(1u << (2 * u));
+                    if ((todo >> (2 * u)) & 2u)
+                        if (look(&pbuf[k + 1 + j], step, pr[u])) todo &= ~(2u << (2 * u));
+                }
+                if (wait_seen && *const_cast<volatile unsigned*>(seen + tid) >= step) wait_seen = false;
+                if (todo || wait_seen) stop = patience.exhausted(err);
+            }
+            if (stop) s_stop = 1;
+        }
+        double vp = 0.0;  // v^H p is real
+        if (tk != 0.0) {
+#pragma unroll
+            for (int u = 0; u < kHetrdEntries; ++u) {
+                const int j = tid + u * kHetrdThreads;
+                if (j < m) vp += sv[j].x * pr[u].x + sv[j].y * pr[u].y;
+            }
+            if (tid == 0) s_p0 = pr[0];
+            vp = warp_sum(vp);
+            if (lane == 0) redp[warp] = vp;
+        }
+        __syncthreads();
+        if (s_stop) return;
+        double half = 0.0;
+        double2 v0 = mk(0.0, 0.0), w0 = v0;
+        if (tk != 0.0) {
+#pragma unroll
+            for (int q = 0; q < WARPS; ++q) half += redp[q];
+            half *= 0.5 * tk;
+            v0 = sv[0];
+            w0 = mk(s_p0.x - half * v0.x, s_p0.y - half * v0.y);
+        }
+        // w = p - (tau / 2) (v^H p) v, and the next step's column:
+        // A[k+1+j, k+1] -= v_j conj(w_0) + w_j conj(v_0)
+#pragma unroll
+        for (int u = 0; u < kHetrdEntries; ++u) {
+            const int j = tid + u * kHetrdThreads;
+            if (j >= m) continue;
+            double2 x = xr[u];
+            if (tk != 0.0) {
+                const double2 v = sv[j], w = mk(pr[u].x - half * v.x, pr[u].y - half * v.y);
+                sw[j] = w;
+                x = x - (cmul(v, conj2(w0)) + cmul(w, conj2(v0)));
+            }
+            sx[k + 1 + j] = x;
+        }
+        __syncthreads();
+        if (tk != 0.0) {
+            // A[j, i] -= v_j conj(w_i) + w_j conj(v_i); the next step's first barrier
+            // comes before anyone writes what is read here
+            for (int jj = warp; jj < owned; jj += WARPS) {
                 const int i = b + G * jj;
-                // W column: W[k+1:, i'] -= tau v (v^H W[k+1:, i'])
-                double2* wc = wcol(jj) + (k + 1);
-                double2 sacc = mk(0.0, 0.0);
-                for (int j = lane; j < m; j += 32) sacc = sacc + cmulc(sv[j], wc[j]);
-                sacc = warp_sum(sacc);
-                const double2 f = mk(tk * sacc.x, tk * sacc.y);
-                for (int j = lane; j < m; j += 32) wc[j] = wc[j] - cmul(sv[j], f);
                 if (i <= k) continue;
-                // A[j, i] -= v_j conj(w_i) + w_j conj(v_i)
                 const double2 vi = sv[i - k - 1], wi = sw[i - k - 1];
                 double2* col = cols + (size_t)jj * n + (k + 1);
                 for (int j = lane; j < m; j += 32) {
@@ -480,8 +523,10 @@ hetrd_smem(int n, int cpb, int w_in_smem, const double2* A, double* d, double2* 
                 }
             }
         }
-        __syncthreads();
+        // the owner of the next column reads it whole at the top of the loop
+        if ((k + 2) % G == b) __syncthreads();
     }
+    __syncthreads();
     if (b == 0 && tid == 0) {
         d[n - 1] = sx[n - 1].x;
         e[n - 1] = mk(0.0, 0.0);
@@ -489,7 +534,7 @@ hetrd_smem(int n, int cpb, int w_in_smem, const double2* A, double* d, double2* 
     if (w_in_smem) {
         for (int jj = 0; jj < owned; ++jj) {
             const int c = b + G * jj;
-            for (int r = tid; r < n; r += blockDim.x) W[r + (size_t)c * n] = wsm[(size_t)jj * n + r];
+            for (int r = tid; r < n; r += kHetrdThreads) W[r + (size_t)c * n] = wsm[(size_t)jj * n + r];
         }
     }
 }
@@ -912,8 +957,7 @@ struct HeevPlan {
     double* d;
     double2* e;
     double2* W;
-    double2* xpre;
-    double2* pbuf;
+    Published *xpre, *pbuf;  // two steps' parities each
     double* ea;
     double* e2;
     double2* phase;
@@ -921,9 +965,10 @@ struct HeevPlan {
     double* Y;
     double* work;
     double2* Yc;
-    double2* partial;
-    unsigned* bar;
+    unsigned* seen;
     int* err;
+    void* zeroed;            // xpre, pbuf, seen and err
+    size_t zeroed_bytes;
     int G = 1, cpb = 1, w_in_smem = 0;
     size_t smem = 0;
 };
@@ -936,8 +981,6 @@ HeevPlan heev_plan(int n, int nvec, Scratch& ws) {
     p.d = ws.take<double>(n);
     p.e = ws.take<double2>(n);
     p.W = ws.take<double2>((size_t)n * n);
-    p.xpre = ws.take<double2>(2 * (size_t)n);
-    p.pbuf = ws.take<double2>(2 * (size_t)n);
     p.ea = ws.take<double>(n);
     p.e2 = ws.take<double>(n);
     p.phase = ws.take<double2>(n);
@@ -956,22 +999,25 @@ HeevPlan heev_plan(int n, int nvec, Scratch& ws) {
     // blocks: about 8 columns each, at most one per SM; columns (and W) in shared memory
     p.G = std::max(1, std::min(nsm, (n + 7) / 8));
     p.cpb = (n + p.G - 1) / p.G;
-    const size_t limit = 200 * 1024;
-    p.smem = ((size_t)p.cpb * n + 3 * (size_t)n) * sizeof(double2);
-    if (p.smem > limit)
+    const size_t limit = 224 * 1024;
+    p.smem = ((size_t)p.cpb * n + 4 * (size_t)n) * sizeof(double2);
+    if (!order_supported(n))
         throw Status(Q3B_ERR_INVALID, "subspace of order " + std::to_string(n) + " too large for the eigensolver");
     p.w_in_smem = (p.smem + (size_t)p.cpb * n * sizeof(double2) <= limit) ? 1 : 0;
     if (p.w_in_smem) p.smem += (size_t)p.cpb * n * sizeof(double2);
-    p.partial = ws.take<double2>(2 * (size_t)p.G);
-    p.bar = ws.take<unsigned>(2);
-    p.err = ws.take<int>(1);
+    p.zeroed_bytes = 4 * (size_t)n * sizeof(Published) + ((size_t)p.G + 1) * sizeof(unsigned);
+    p.xpre = reinterpret_cast<Published*>(ws.take<double2>(p.zeroed_bytes / sizeof(double2) + 1));
+    p.zeroed = p.xpre;
+    p.pbuf = p.xpre + 2 * (size_t)n;
+    p.seen = reinterpret_cast<unsigned*>(p.pbuf + 2 * (size_t)n);
+    p.err = reinterpret_cast<int*>(p.seen + p.G);
     static PerDeviceOnce once;
     once.run([limit] {
         cudaFuncSetAttribute(hetrd_smem, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)limit);
         cudaFuncSetAttribute(tridiag_invit_smem, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kInvitSmemLimit);
     });
     int per_sm = 0;
-    Q3B_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, hetrd_smem, 256, p.smem));
+    Q3B_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, hetrd_smem, kHetrdThreads, p.smem));
     if (per_sm < 1 || per_sm * nsm < p.G) throw Status(Q3B_ERR_INVALID, "eigensolver blocks cannot be co-resident");
     return p;
 }
@@ -980,19 +1026,19 @@ HeevPlan heev_plan(int n, int nvec, Scratch& ws) {
 void heev_launch(cudaStream_t st, const HeevPlan& p, const double2* A, double* w, double2* Z,
                  const GemmWorkspace& gws) {
     const int n = p.n, nvec = p.nvec;
-    Q3B_CUDA(cudaMemsetAsync(p.bar, 0, 2 * sizeof(unsigned), st));
-    Q3B_CUDA(cudaMemsetAsync(p.err, 0, sizeof(int), st));
+    Q3B_CUDA(cudaMemsetAsync(p.zeroed, 0, p.zeroed_bytes, st));
     {
         int nn = n, cpb = p.cpb, wis = p.w_in_smem;
         const double2* Ac = A;
         double* d = p.d;
-        double2 *e = p.e, *W = p.W, *xpre = p.xpre, *pbuf = p.pbuf, *partial = p.partial;
-        unsigned* bar = p.bar;
+        double2 *e = p.e, *W = p.W;
+        Published *xpre = p.xpre, *pbuf = p.pbuf;
+        unsigned* seen = p.seen;
         int* err = p.err;
-        void* args[] = {&nn, &cpb, &wis, &Ac, &d, &e, &W, &xpre, &pbuf, &partial, &bar, &err};
+        void* args[] = {&nn, &cpb, &wis, &Ac, &d, &e, &W, &xpre, &pbuf, &seen, &err};
         cudaLaunchConfig_t cfg = {};
         cfg.gridDim = dim3(p.G);
-        cfg.blockDim = dim3(256);
+        cfg.blockDim = dim3(kHetrdThreads);
         cfg.dynamicSmemBytes = p.smem;
         cfg.stream = st;
         cudaLaunchAttribute attr[1];
