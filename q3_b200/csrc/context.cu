@@ -191,7 +191,7 @@ bool Context::release_optional() {
     // callers ask for the GEMM workspace after all their other buffers, so no
     // product that still has to be issued holds its address here
     bool any = false;
-    for (DevBuf* b : {&kp.beta_zm_overlap, &kp.beta_zm_accum}) {
+    for (DevBuf* b : {&kp.beta_zm_overlap, &kp.beta_zm_accum, &kp.beta_hs_overlap, &kp.beta_hs_accum}) {
         any = any || b->ptr;
         b->release();
     }
@@ -586,10 +586,6 @@ void Context::prepare_kpoint(int npw, const int32_t* g2g, const double* ke, cons
             for (size_t i = 0; i < nb; ++i) b32[i] = make_float2((float)beta[i].x, (float)beta[i].y);
             upload(this, kp.beta32, b32.data(), nb);
         }
-        kp.beta_pk_overlap.reserve(this, tc::packed_a_bytes(nproj, npw));
-        kp.beta_pk_accum.reserve(this, tc::packed_a_bytes(npw, nproj));
-        tc::pack_a(stream, nproj, npw, kp.beta32.as<float2>(), npw, true, kp.beta_pk_overlap.as<unsigned char>());
-        tc::pack_a(stream, npw, nproj, kp.beta32.as<float2>(), npw, false, kp.beta_pk_accum.as<unsigned char>());
         std::vector<int> ps(nproj), pz(nproj), po(nproj);
         std::vector<double> d64;
         size_t doff = 0;
@@ -616,25 +612,49 @@ void Context::prepare_kpoint(int npw, const int32_t* g2g, const double* ke, cons
         kp.dpk_len = d64.size();
     }
     build_plan();
-    pack_beta64();
+    pack_projectors();
     kp.valid = true;
 }
 
-// Residue tiles of the projectors for <beta|psi> and beta B', where a block of
-// bands of usual size (half the projectors, as four bands an atom make) runs
-// its products on them.
-void Context::pack_beta64() {
-    kp.beta_zm_overlap.release();
-    kp.beta_zm_accum.release();
+// The projectors as the tensor-core products of <beta|psi> and beta B' take
+// them, in both precisions.  FP32: FP16 tiles from kHalfMinMacs complex
+// multiply-adds of a block of usual size (half the projectors, as four bands an
+// atom make), TF32 tiles below.  The FP16 form packs the bands as well (two
+// launches) and works in 256 rows: both products of a block took 204 us against 300
+// at 64 atoms (3.1e9), 155 against 142 at 48 (1.3e9), 77 against 42 at 19 (8e7);
+// with half the 64-atom cell's bands 157 against 167, with a quarter 122 against
+// 122.  FP64: residue tiles where the products of such a block run on them.
+// Without room for FP16 or residue tiles the products take the projectors as they
+// are.
+constexpr double kHalfMinMacs = 2e9;
+void Context::pack_projectors() {
+    for (DevBuf* b : {&kp.beta_zm_overlap, &kp.beta_zm_accum, &kp.beta_hs_overlap, &kp.beta_hs_accum}) b->release();
     const int P = kp.nproj, npw = kp.npw;
-    if (P <= 0 || !zmod::worth(true, P, P / 2, npw, true)) return;
-    const size_t to = zmod::packed_a_bytes(P, npw), ta = zmod::packed_a_bytes(npw, P);
-    if (!kp.beta_zm_overlap.try_reserve(this, to + zmod::packed_a_exps(P) * sizeof(int))) return;
-    if (!kp.beta_zm_accum.try_reserve(this, ta + zmod::packed_a_exps(npw) * sizeof(int))) return;
-    unsigned char* o = kp.beta_zm_overlap.as<unsigned char>();
-    unsigned char* a = kp.beta_zm_accum.as<unsigned char>();
-    zmod::pack_a(stream, P, npw, kp.beta64.as<double2>(), npw, true, o, reinterpret_cast<int*>(o + to));
-    zmod::pack_a(stream, npw, P, kp.beta64.as<double2>(), npw, false, a, reinterpret_cast<int*>(a + ta));
+    if (P <= 0) return;
+    auto pack = [&](auto convert_rows, DevBuf& buf, size_t tiles, size_t exps, const auto* beta, int M, int K, bool kmajor) {
+        if (!buf.try_reserve(this, tiles + exps * sizeof(int))) return;
+        unsigned char* t = buf.as<unsigned char>();
+        convert_rows(stream, M, K, beta, npw, kmajor, t, reinterpret_cast<int*>(t + tiles));
+    };
+    if (0.5 * P * P * npw >= kHalfMinMacs) {
+        pack(half2x::pack_a, kp.beta_hs_overlap, half2x::packed_a_bytes(P, npw), half2x::packed_a_exps(P),
+             kp.beta32.as<float2>(), P, npw, true);
+        pack(half2x::pack_a, kp.beta_hs_accum, half2x::packed_a_bytes(npw, P), half2x::packed_a_exps(npw),
+             kp.beta32.as<float2>(), npw, P, false);
+        kp.beta_pk_overlap.release();
+        kp.beta_pk_accum.release();
+    } else {
+        kp.beta_pk_overlap.reserve(this, tc::packed_a_bytes(P, npw));
+        kp.beta_pk_accum.reserve(this, tc::packed_a_bytes(npw, P));
+        tc::pack_a(stream, P, npw, kp.beta32.as<float2>(), npw, true, kp.beta_pk_overlap.as<unsigned char>());
+        tc::pack_a(stream, npw, P, kp.beta32.as<float2>(), npw, false, kp.beta_pk_accum.as<unsigned char>());
+    }
+    if (zmod::worth(true, P, P / 2, npw, true)) {
+        pack(zmod::pack_a, kp.beta_zm_overlap, zmod::packed_a_bytes(P, npw), zmod::packed_a_exps(P),
+             kp.beta64.as<double2>(), P, npw, true);
+        pack(zmod::pack_a, kp.beta_zm_accum, zmod::packed_a_bytes(npw, P), zmod::packed_a_exps(npw),
+             kp.beta64.as<double2>(), npw, P, false);
+    }
 }
 
 template <> const LocalPlan<double>& Context::local_plan<double>() const { return kp.lp64; }
@@ -655,10 +675,16 @@ template <> NonlocalData<double> Context::nonlocal<double>() const {
 template <> NonlocalData<float> Context::nonlocal<float>() const {
     NonlocalData<float> d{kp.nproj, kp.beta32.as<float2>(), kp.pstart.as<int>(),
                           kp.psize.as<int>(), kp.poff.as<int>(), kp.dpk32.as<float>()};
-    if (kp.nproj > 0) {
+    if (kp.beta_pk_overlap.ptr)
         d.beta_overlap = tc::PackedA{kp.beta_pk_overlap.as<unsigned char>(), kp.nproj, kp.npw};
-        d.beta_accum = tc::PackedA{kp.beta_pk_accum.as<unsigned char>(), kp.npw, kp.nproj};
-    }
+    if (kp.beta_pk_accum.ptr) d.beta_accum = tc::PackedA{kp.beta_pk_accum.as<unsigned char>(), kp.npw, kp.nproj};
+    auto packed = [](const DevBuf& b, int M, int K) {
+        if (!b.ptr) return half2x::PackedA{};
+        const unsigned char* t = b.as<unsigned char>();
+        return half2x::PackedA{t, reinterpret_cast<const int*>(t + half2x::packed_a_bytes(M, K)), M, K};
+    };
+    d.hs_overlap = packed(kp.beta_hs_overlap, kp.nproj, kp.npw);
+    d.hs_accum = packed(kp.beta_hs_accum, kp.npw, kp.nproj);
     return d;
 }
 

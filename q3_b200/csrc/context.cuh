@@ -51,7 +51,10 @@ struct KPoint {
     std::vector<double> ke_host;
     DevBuf ke64, ke32;
     DevBuf beta64, beta32;
-    DevBuf beta_pk_overlap, beta_pk_accum;  // beta32 as packed tensor-core A tiles
+    DevBuf beta_pk_overlap, beta_pk_accum;  // beta32 as TF32 tensor-core A tiles
+    // or, for large sets, as FP16 tiles, each followed by its rows' exponents
+    // (these, like the next, empty where memory is short)
+    DevBuf beta_hs_overlap, beta_hs_accum;
     // beta64 as residue tiles for the FP64 products, each followed by its rows'
     // exponents; empty for small sets and where memory is short
     DevBuf beta_zm_overlap, beta_zm_accum;
@@ -156,7 +159,7 @@ class Context {
     size_t ws_gemm_need_ = 0;     // largest `need` of gemm_ws
     size_t ws_gemm_refused_ = 0;  // smallest `want` the device had no room for (0: none)
     void build_plan();
-    void pack_beta64();
+    void pack_projectors();
 };
 
 // convert an exception into a status code and message

@@ -56,8 +56,19 @@ template <typename R> size_t nonlocal_wanted_bytes(const NonlocalData<R>& nl, in
             b = zmod::workspace_bytes(true, nl.nproj, nvec, npw, true);
         if (nl.zm_accum.tiles && zmod::worth(false, npw, nvec, nl.nproj, true))
             b = std::max(b, zmod::workspace_bytes(false, npw, nvec, nl.nproj, true));
+    } else if (use_tensor_cores(nl.nproj, nvec, npw)) {
+        if (nl.hs_overlap.tiles) b = half2x::workspace_bytes(true, nl.nproj, nvec, npw);
+        if (nl.hs_accum.tiles) b = std::max(b, half2x::workspace_bytes(false, npw, nvec, nl.nproj));
     }
     return b;
+}
+
+// whether an FP32 projector product runs on the FP16 tiles (beta^H psi
+// with `overlap`, else beta B')
+static bool on_half_tiles(const NonlocalData<float>& nl, bool overlap, int npw, int nvec, const GemmWorkspace& ws) {
+    if (!use_tensor_cores(nl.nproj, nvec, npw) || !ws.ptr) return false;
+    return overlap ? nl.hs_overlap.tiles && ws.bytes >= half2x::workspace_bytes(true, nl.nproj, nvec, npw)
+                   : nl.hs_accum.tiles && ws.bytes >= half2x::workspace_bytes(false, npw, nvec, nl.nproj);
 }
 
 template <typename R>
@@ -69,7 +80,9 @@ void apply_nonlocal(cudaStream_t st, const NonlocalData<R>& nl, int npw, int nve
     const T one = mk(R(1), R(0)), zero = mk(R(0), R(0));
     if (tm) tm->begin(PhaseTimer::PROJ_OVERLAP);
     if constexpr (std::is_same<R, float>::value) {
-        if (nl.beta_overlap.tiles && use_tensor_cores(nl.nproj, nvec, npw))
+        if (on_half_tiles(nl, true, npw, nvec, ws))
+            half2x::cgemm(st, true, nl.nproj, nvec, npw, one, nl.hs_overlap, psi, ldpsi, zero, Bm, nl.nproj, ws);
+        else if (nl.beta_overlap.tiles && use_tensor_cores(nl.nproj, nvec, npw))
             tc::cgemm_packed(st, true, nl.nproj, nvec, npw, one, nl.beta_overlap, psi, ldpsi, zero, Bm, nl.nproj, ws);
         else
             cgemm<R>(st, true, nl.nproj, nvec, npw, one, nl.beta, npw, psi, ldpsi, zero, Bm, nl.nproj, ws);
@@ -88,7 +101,9 @@ void apply_nonlocal(cudaStream_t st, const NonlocalData<R>& nl, int npw, int nve
     if (tm) tm->end();
     if (tm) tm->begin(PhaseTimer::PROJ_ACCUM);
     if constexpr (std::is_same<R, float>::value) {
-        if (nl.beta_accum.tiles && use_tensor_cores(npw, nvec, nl.nproj))
+        if (on_half_tiles(nl, false, npw, nvec, ws))
+            half2x::cgemm(st, false, npw, nvec, nl.nproj, one, nl.hs_accum, Bp, nl.nproj, one, hpsi, ldh, ws);
+        else if (nl.beta_accum.tiles && use_tensor_cores(npw, nvec, nl.nproj))
             tc::cgemm_packed(st, false, npw, nvec, nl.nproj, one, nl.beta_accum, Bp, nl.nproj, one, hpsi, ldh, ws);
         else
             cgemm<R>(st, false, npw, nvec, nl.nproj, one, nl.beta, npw, Bp, nl.nproj, one, hpsi, ldh, ws);

@@ -2,6 +2,7 @@
 #pragma once
 
 #include "cgemm.cuh"
+#include "cgemm_half.cuh"
 #include "common.cuh"
 #include "hpsi_local.cuh"
 #include "zgemm_mod.cuh"
@@ -15,9 +16,11 @@ template <typename R> struct NonlocalData {
     const int* psize = nullptr;       // size of p's atom block
     const int* poff = nullptr;        // offset of p's block in dpk
     const R* dpk = nullptr;           // packed column-major D blocks (Ry)
-    // FP32 only: beta pre-split into the tensor-core kernel's A tiles, for
-    // beta^H psi (rows = projectors) and for beta B' (rows = plane waves)
+    // FP32 only: beta pre-split into the TF32 kernel's A tiles, for beta^H psi
+    // (rows = projectors) and for beta B' (rows = plane waves), or, for large sets,
+    // into FP16 tiles (each may be empty)
     tc::PackedA beta_overlap{}, beta_accum{};
+    half2x::PackedA hs_overlap{}, hs_accum{};
     // FP64 only: beta as residue tiles for the same two products (may be empty)
     zmod::PackedA zm_overlap{}, zm_accum{};
 };

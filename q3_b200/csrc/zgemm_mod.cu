@@ -32,11 +32,14 @@
 #include <type_traits>
 #include <utility>
 
+#include "umma_pair.cuh"
 #include "zgemm_mod.cuh"
 
 namespace q3b {
 namespace zmod {
 namespace {
+
+using namespace umma;
 
 constexpr int NMOD = 15;
 constexpr int kMod[NMOD] = {256, 255, 253, 251, 247, 241, 239, 233, 229, 227, 223, 217, 211, 199, 197};
@@ -108,7 +111,7 @@ constexpr int A_TILE = 2 * BM * BK;   // real plane, imaginary plane
 constexpr int STAGES = 4;
 constexpr int EPI_WARPS = 8;
 constexpr int THREADS = 32 * (EPI_WARPS + 2);
-constexpr uint32_t TMEM_COLS = 512;   // two buffers of at most 256 accumulator columns
+// TMEM: two buffers of at most 256 accumulator columns
 // BC: complex columns a CTA holds of its pair's 2 BC (64, or 32 for narrow products)
 template <int BC> struct Cols {
     static constexpr int b_tile = 3 * BC * BK;      // three planes, see pack_rows
@@ -286,64 +289,15 @@ __global__ void __launch_bounds__(256) pack_rows(int R, int K, const double2* __
                     else neg[q] = m * 0x01010101u - w[q];
                 }
             }
-            const uint4 v = make_uint4(w[0], w[1], w[2], w[3]);
             unsigned char* at = dst + (size_t)i * TILE;
-            *reinterpret_cast<uint4*>(at + (AS == kPackB ? p + 1 : p) * PLANE) = v;
+            *reinterpret_cast<uint4*>(at + (AS == kPackB ? p + 1 : p) * PLANE) = make_uint4(w[0], w[1], w[2], w[3]);
             if (p == negated)
                 *reinterpret_cast<uint4*>(at + (AS == kPackB ? 0 : 2) * PLANE) = make_uint4(neg[0], neg[1], neg[2], neg[3]);
         }
     });
 }
 
-// ------------------------------------------------------------------ device helpers
-__device__ __forceinline__ uint32_t smem_u32(const void* p) {
-    return static_cast<uint32_t>(__cvta_generic_to_shared(p));
-}
-__device__ __forceinline__ void mbar_init(uint64_t* bar, uint32_t count) {
-    asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_u32(bar)), "r"(count) : "memory");
-}
-__device__ __forceinline__ void mbar_arrive_tx(uint64_t* bar, uint32_t bytes) {
-    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(smem_u32(bar)), "r"(bytes)
-                 : "memory");
-}
-__device__ __forceinline__ bool mbar_try_wait(uint64_t* bar, uint32_t parity) {
-    uint32_t ok;
-    asm volatile(
-        "{\n\t.reg .pred p;\n\t"
-        "mbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\n\t"
-        "selp.u32 %0, 1, 0, p;\n\t}\n"
-        : "=r"(ok)
-        : "r"(smem_u32(bar)), "r"(parity)
-        : "memory");
-    return ok != 0;
-}
-// Bounded wait on an mbarrier phase; false (and the error word set) on timeout.
-// `heed`: give up as soon as another wait has timed out.
-__device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, int* err, bool heed = true) {
-    for (int i = 0; i < (1 << 22); ++i) {
-        if (mbar_try_wait(bar, parity)) return true;
-        if (heed && (i & 63) == 63 && *reinterpret_cast<volatile int*>(err)) return false;
-        if (i > 4096) __nanosleep(64);
-    }
-    atomicExch(err, 1);
-    return false;
-}
-__device__ __forceinline__ void bulk_copy_g2s(void* dst, const void* src, uint32_t bytes, uint64_t* bar) {
-    asm volatile(
-        "cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(
-            smem_u32(dst)),
-        "l"(src), "r"(bytes), "r"(smem_u32(bar))
-        : "memory");
-}
-__device__ __forceinline__ void tc_fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
-__device__ __forceinline__ void tc_fence_after() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
-
-// K-major, SWIZZLE_128B, rows of 128 bytes, 8-row groups 1024 bytes apart
-__device__ __forceinline__ uint64_t smem_desc(uint32_t addr) {
-    return static_cast<uint64_t>((addr >> 4) & 0x3FFF) | (static_cast<uint64_t>(1) << 16) |
-           (static_cast<uint64_t>((1024 >> 4) & 0x3FFF) << 32) | (static_cast<uint64_t>(1) << 46) |
-           (static_cast<uint64_t>(2) << 61);
-}
+// ------------------------------------------------------------------ products
 __device__ __forceinline__ void mma_i8(uint32_t d, uint64_t a, uint64_t b, uint32_t instr, uint32_t accumulate) {
     asm volatile(
         "{\n\t.reg .pred p;\n\t"
@@ -352,38 +306,6 @@ __device__ __forceinline__ void mma_i8(uint32_t d, uint64_t a, uint64_t b, uint3
         "l"(a), "l"(b), "r"(instr), "r"(accumulate)
         : "memory");
 }
-// arrive on this barrier of both CTAs once the MMAs issued so far are done
-__device__ __forceinline__ void mma_commit_pair(uint64_t* bar) {
-    asm volatile(
-        "tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;" ::"r"(
-            smem_u32(bar)),
-        "h"(static_cast<uint16_t>(3))
-        : "memory");
-}
-__device__ __forceinline__ uint32_t cluster_rank() {
-    uint32_t r;
-    asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
-    return r;
-}
-// arrive on the leader's (rank 0) copy of a barrier
-__device__ __forceinline__ void mbar_arrive_leader(uint64_t* bar) {
-    asm volatile(
-        "{\n\t.reg .b32 a;\n\t"
-        "mapa.shared::cluster.u32 a, %0, 0;\n\t"
-        "mbarrier.arrive.release.cluster.shared::cluster.b64 _, [a];\n\t}\n" ::"r"(smem_u32(bar))
-        : "memory");
-}
-__device__ __forceinline__ void cluster_sync() {
-    asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
-}
-__device__ __forceinline__ void tmem_ld8(uint32_t addr, uint32_t* r) {
-    asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
-                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7])
-                 : "r"(addr));
-}
-__device__ __forceinline__ void tmem_wait_ld() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
-
-// ------------------------------------------------------------------ products
 // A pair of CTAs (one TPC) works on output tiles of 256 rows x 2 BC columns with
 // cta_group::2 MMAs: each CTA holds 128 rows of A and BC columns of B in its
 // shared memory, and its 128 rows of the accumulator, [re | im] of one half of
@@ -449,12 +371,7 @@ zmod_gemm(Units un, int total, const unsigned char* __restrict__ A, const unsign
         mbar_init(&done_bar, 1);
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
-    if (warp == 0) {
-        asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&tmem_slot)),
-                     "r"(TMEM_COLS)
-                     : "memory");
-        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
-    }
+    if (warp == 0) tmem_alloc_pair(&tmem_slot);
     tc_fence_before();
     __syncthreads();
     cluster_sync();  // both CTAs' barriers and TMEM are ready
@@ -586,9 +503,7 @@ zmod_gemm(Units un, int total, const unsigned char* __restrict__ A, const unsign
     tc_fence_before();
     __syncthreads();
     cluster_sync();  // no CTA leaves while the other may still read or signal it
-    if (warp == 0) {
-        asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(TMEM_COLS) : "memory");
-    }
+    if (warp == 0) tmem_free_pair(tmem);
 }
 
 // ------------------------------------------------------------------ recombination

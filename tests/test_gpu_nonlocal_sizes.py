@@ -1,0 +1,55 @@
+"""The projector products of H|psi> (FP32 on split FP16 tiles, FP64 on residue tiles or the FP64
+units, by size) on their own: no potential, no kinetic energy, no plane wave on the grid, so
+that H psi = beta D beta^H psi.
+
+Bounds per entry, S = sum |beta| |D| sum |beta| |psi| over projectors and plane waves: FP32
+4e-6 S (each product within 2e-6 of its sum of magnitudes, test_gpu_gemm.py's bar, and each
+operand within 2^-22 of itself or 2^-39 of the largest in its row); FP64 2e-13 S.
+"""
+import numpy as np
+import pytest
+
+from q3_b200._lib import FP64, MIXED
+
+pytestmark = pytest.mark.gpu
+
+# edges of 256-row, 128-column and 64-column tiles and of 64 and 128 of K, on the FP16 tiles (from
+# 2e9 multiply-adds of half as many bands as projectors) and, first and last, the TF32 ones
+SIZES = [(5000, 136, 130), (12289, 640, 130), (4097, 1032, 65), (2100, 1400, 257), (23847, 512, 33), (769, 640, 257)]
+
+
+def _inputs(npw, nproj, nvec, graded):
+    rng = np.random.default_rng(npw + nproj + nvec)
+    beta = rng.standard_normal((npw, nproj)) + 1j * rng.standard_normal((npw, nproj))
+    psi = rng.standard_normal((npw, nvec)) + 1j * rng.standard_normal((npw, nvec))
+    if graded:  # projectors and bands fall off along the plane waves, and differ in size
+        fall = np.exp(-16.0 * np.linspace(0.0, 1.0, npw))[:, None]
+        beta *= fall * 10.0 ** rng.uniform(-3, 3, nproj)[None, :]
+        psi *= fall ** 0.25 * 10.0 ** rng.uniform(-6, 3, nvec)[None, :]
+    d = rng.uniform(-1.0, 1.0, (nproj // 8, 8, 8))
+    return beta, psi, d + d.transpose(0, 2, 1)
+
+
+@pytest.mark.parametrize("graded", [False, True], ids=["normal", "graded"])
+@pytest.mark.parametrize("npw,nproj,nvec", SIZES)
+def test_projector_products(cuda_device, npw, nproj, nvec, graded):
+    import torch
+    from q3_b200.applicator import PlanewaveHamiltonianApplicator
+    beta, psi, d = _inputs(npw, nproj, nvec, graded)
+    ap = PlanewaveHamiltonianApplicator()
+    ap.update_potential(np.zeros(16 ** 3), (16, 16, 16))
+    ap.prepare_kpoint(0, npw, np.full(npw, -1, np.int32), np.zeros(npw), beta,
+                      np.arange(0, nproj + 1, 8, dtype=np.int32), d.transpose(0, 2, 1).reshape(-1))
+    x = torch.from_numpy(np.ascontiguousarray(psi.T)).cuda()
+    inner = beta.conj().T @ psi
+    want = beta @ np.einsum("aij,ajv->aiv", d, inner.reshape(nproj // 8, 8, nvec)).reshape(nproj, nvec)
+    mag = np.abs(beta) @ np.einsum("aij,ajv->aiv", np.abs(d), (np.abs(beta).T @ np.abs(psi)).reshape(
+        nproj // 8, 8, nvec)).reshape(nproj, nvec)
+    if graded:  # 2^-39 of the largest entry of a row, against entries of its tail
+        mag = np.maximum(mag, 1e-6 * np.max(mag, axis=0))
+    for precision, tol in ((MIXED, 4e-6), (FP64, 2e-13)):
+        y = torch.full_like(x, np.nan)
+        ap.apply_batch(x, y, nvec, precision)
+        torch.cuda.synchronize()
+        got = y.cpu().numpy().T
+        assert np.max(np.abs(got - want) / mag) < tol, precision
