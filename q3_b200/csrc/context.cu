@@ -460,10 +460,13 @@ void Context::build_plan() {
         col_id[order[i]] = i;
         stick_pos[i] = (order[i] / n2) * p2 + order[i] % n2;
     }
+    std::vector<short> row_map;
     for (int w1 = 0; w1 < n1; ++w1)
         for (int w2 = 0; w2 < n2; ++w2)
             if (col_id[w1 * n2 + w2] >= 0) {
                 rows.push_back(w1 * p2);
+                if (n1 <= 128 && n2 <= 128)
+                    for (int c = 0; c < n2; ++c) row_map.push_back(static_cast<short>(col_id[w1 * n2 + c]));
                 break;
             }
     std::vector<int> start(S + 1, 0);
@@ -489,6 +492,7 @@ void Context::build_plan() {
     upload(this, k.entry_at, ea.data(), ea.size());
     upload(this, k.stick_pos, stick_pos.data(), stick_pos.size());
     upload(this, k.row_base, rows.data(), rows.size());
+    upload(this, k.row_map, row_map.data(), row_map.size());
     upload(this, k.unmapped, unm.data(), unm.size());
     if (intervals) upload(this, k.row_iv, ivs.data(), ivs.size());
     else k.row_iv.release();
@@ -530,6 +534,7 @@ void Context::build_plan() {
         lp.entry_at = k.entry_at.as<int>();
         lp.stick_pos = k.stick_pos.as<int>();
         lp.row_base = k.row_base.as<int>();
+        lp.row_map = k.row_map.as<short>();
         lp.unmapped_g = k.unmapped.as<int>();
         lp.tw1 = tw[0].as<TT>();
         lp.tw2 = tw[1].as<TT>();

@@ -35,6 +35,7 @@ template <typename R> struct LocalPlan {
     const int* entry_at;     // (stick % sg) * p3 + w3: its place in its block's lines
     const int* stick_pos;    // w1*p2 + w2
     const int* row_base;     // w1*p2 of each used row
+    const short* row_map;    // [used row][w2]: the stick there, or -1 (grids up to 128 x 128)
     const int* unmapped_g;
     const T* tw1;            // w_n^m = exp(-2 pi i m/n), one table per axis
     const T* tw2;

@@ -13,11 +13,11 @@
 // 80 registers, so that an SM holds 24 warps of it instead of 16.  Bound: the
 // latency of the passes (shared memory, FP64 or FP32 arithmetic) between barriers.
 // Plane pass of 64 bands, general kernel against this, each at its best block:
-//   40^3, 48 bands   FP64 45.3 -> 35.1 us    FP32 29.0 -> 22.6 us
-//   54^3, 77 bands   FP64 133.5 -> 110.8     FP32 86.1 -> 69.6
-//   64^3, 65 bands   FP64 162.2 -> 129.3     FP32 104.6 -> 82.3
-//   80^3             FP64 334.6 -> 267.2     FP32 188.7 -> 151.6
-//   108^3, 32 bands  FP64 525.5 -> 433.2     FP32 286.9 -> 209.6
+//   40^3, 48 bands   FP64 45.3 -> 33.1 us    FP32 29.0 -> 21.0 us
+//   54^3, 77 bands   FP64 133.5 -> 100.9     FP32 86.1 -> 61.7
+//   64^3, 65 bands   FP64 162.2 -> 133.4     FP32 104.6 -> 80.4
+//   80^3             FP64 334.6 -> 242.5     FP32 188.7 -> 139.5
+//   108^3, 32 bands  FP64 525.5 -> 406.8     FP32 286.9 -> 205.4
 #pragma once
 
 #include "fft_core.cuh"
@@ -94,28 +94,35 @@ template <typename R, int N> struct PlaneSmem {
     }
 };
 
-// Sticks of one plane into its rows, rows backward, the columns' first pass
-// backward.  Only the rows that hold sticks are read before they are written.
-// Ends with a barrier.
+// The rows' outer passes take their values from the stick buffer and leave them
+// there, element by element through the plan's map from (row, w2) to sticks
+// (LocalPlan::row_map), so no row is cleared, filled or emptied by passes of its
+// own: six barriers a plane instead of ten (80^3, 64 bands: FP64 267 -> 243 us,
+// FP32 152 -> 140; the density of the 64-atom cell 875 -> 824).  Their items run
+// along q first, so that neighbouring lanes meet neighbouring sticks.
+template <int NT, int NB, typename F> __device__ __forceinline__ void items_along_row(int nrows, const F& f) {
+#pragma unroll 1
+    for (int it = threadIdx.x; it < nrows * NB; it += NT) f(it / NB, it % NB);
+}
+
+// Rows backward from the sticks of one plane, the columns' first pass backward.
+// Only the rows that hold sticks are written and read.  Ends with a barrier.
 template <typename R, int N, int NT>
 __device__ __forceinline__ void plane_in(const LocalPlan<R>& p, const PlaneSmem<R, N>& s, const cplx_t<R>* xp) {
     using T = cplx_t<R>;
     using G = Geometry<R, N>;
     constexpr int NA = G::NA, NB = G::NB, P = G::PITCH;
-    const int tid = threadIdx.x, nrows = p.nrows;
-    for (int r = tid >> 5; r < nrows; r += NT / 32) {
-        T* row = s.plane + s.rowb[r];
-        for (int c = tid & 31; c < N; c += 32) row[c] = czero<T>();
-    }
-    __syncthreads();
-    for (int i = tid; i < p.nsticks; i += NT) s.plane[p.stick_pos[i]] = xp[i];
-    __syncthreads();
-    items<NT>(nrows, NB, [&](int l, int q) {
+    const int nrows = p.nrows;
+    items_along_row<NT, NB>(nrows, [&](int l, int q) {
         T* b = s.plane + s.rowb[l] + q;
         const T* w = s.twa + q * NA;
+        const short* at = p.row_map + l * N + q;
+        int from[NA];
         T x[NA];
 #pragma unroll
-        for (int r = 0; r < NA; ++r) x[r] = b[NB * r];
+        for (int r = 0; r < NA; ++r) from[r] = at[NB * r];
+#pragma unroll
+        for (int r = 0; r < NA; ++r) x[r] = from[r] >= 0 ? xp[from[r]] : czero<T>();
         fft::dft<NA, +1>(x, w, 0);
 #pragma unroll
         for (int k = 0; k < NA; ++k) b[NB * k] = k ? cmulc(w[k], x[k]) : x[k];
@@ -153,7 +160,7 @@ __global__ void __launch_bounds__(NT, MINB) planes_sq(LocalPlan<R> p, cplx_t<R>*
     extern __shared__ __align__(16) unsigned char smem[];
     PlaneSmem<R, N> s;
     s.template init<NT>(p, smem);
-    const int tid = threadIdx.x, i3 = blockIdx.x, band = blockIdx.y, nrows = p.nrows;
+    const int i3 = blockIdx.x, band = blockIdx.y, nrows = p.nrows;
     T* xp = X + ((long)band * p.n3 + i3) * p.xpitch;
     plane_in<R, N, NT>(p, s, xp);
     // columns: the rest of backward, V, forward (only the stick rows are wanted of it)
@@ -199,17 +206,20 @@ __global__ void __launch_bounds__(NT, MINB) planes_sq(LocalPlan<R> p, cplx_t<R>*
         for (int k = 0; k < NB; ++k) b[k] = k ? cmul(x[k], w[k]) : x[k];
     });
     __syncthreads();
-    items<NT>(nrows, NB, [&](int l, int q) {
-        T* b = s.plane + s.rowb[l] + q;
+    items_along_row<NT, NB>(nrows, [&](int l, int q) {
+        const T* b = s.plane + s.rowb[l] + q;
+        const short* at = p.row_map + l * N + q;
+        int to[NA];
         T x[NA];
+#pragma unroll
+        for (int r = 0; r < NA; ++r) to[r] = at[NB * r];
 #pragma unroll
         for (int r = 0; r < NA; ++r) x[r] = b[NB * r];
         fft::dft<NA, -1>(x, s.twa, 0);
 #pragma unroll
-        for (int k = 0; k < NA; ++k) b[NB * k] = x[k];
+        for (int k = 0; k < NA; ++k)
+            if (to[k] >= 0) xp[to[k]] = x[k];
     });
-    __syncthreads();
-    for (int i = tid; i < p.nsticks; i += NT) xp[i] = s.plane[p.stick_pos[i]];
 }
 
 // Charge density of one band group on one plane (density_reduce in
