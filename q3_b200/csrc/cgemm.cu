@@ -52,6 +52,7 @@ __global__ void __launch_bounds__(kThreads)
 cgemm_pipe(int M, int N, int K, cplx_t<R> alpha, const cplx_t<R>* __restrict__ A, long lda,
            const cplx_t<R>* __restrict__ B, long ldb, cplx_t<R> beta, cplx_t<R>* C, long ldc, int kchunk,
            cplx_t<R>* part, unsigned* counters) {
+    chain_begin();
     using T = cplx_t<R>;
     using S = PipeTile<R, TM, TN>;
     extern __shared__ __align__(16) unsigned char zsm[];
@@ -194,6 +195,7 @@ __global__ void __launch_bounds__(big::THREADS, 1)
 zgemm_big(int M, int N, int K, double2 alpha, const double2* __restrict__ A, long lda,
           const double2* __restrict__ B, long ldb, double2 beta, double2* C, long ldc, int kchunk,
           double2* part) {
+    chain_begin();
     using namespace big;
     constexpr int BM = Shape<TM>::bm, A_PITCH_N = Shape<TM>::a_pitch_n, A_STAGE = Shape<TM>::a_stage,
                   B_STAGE = Shape<TM>::b_stage;
@@ -321,6 +323,7 @@ __global__ void __launch_bounds__(256) dfma_probe(int iters, double seed, double
 template <typename R>
 __global__ void splitk_reduce(int M, int N, int splits, const cplx_t<R>* __restrict__ part,
                               cplx_t<R> alpha, cplx_t<R> beta, cplx_t<R>* C, long ldc) {
+    chain_begin();
     using T = cplx_t<R>;
     const long total = (long)M * N;
     const bool use_beta = (beta.x != R(0) || beta.y != R(0));
@@ -391,7 +394,7 @@ void pipe_run(cudaStream_t st, dim3 grid, int M, int N, int K, cplx_t<R> alpha, 
         Q3B_CUDA(cudaFuncSetAttribute(cgemm_pipe<R, CONJ_A, TM, TN>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                       (int)PipeTile<R, TM, TN>::smem));
     });
-    cgemm_pipe<R, CONJ_A, TM, TN><<<grid, kThreads, smem, st>>>(M, N, K, alpha, A, lda, B, ldb, beta, C, ldc, kchunk,
+    launch_chained(cgemm_pipe<R, CONJ_A, TM, TN>, grid, kThreads, smem, st, M, N, K, alpha, A, lda, B, ldb, beta, C, ldc, kchunk,
                                                                 part, counters);
     Q3B_LAUNCH_CHECK();
 }
@@ -446,7 +449,7 @@ void zgemm_big_run(cudaStream_t st, dim3 grid, int M, int N, int K, double2 alph
         Q3B_CUDA(cudaFuncSetAttribute(zgemm_big<CONJ_A, TM>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                       (int)big::Shape<TM>::smem));
     });
-    zgemm_big<CONJ_A, TM><<<grid, big::THREADS, smem, st>>>(M, N, K, alpha, A, lda, B, ldb, beta, C, ldc, kchunk,
+    launch_chained(zgemm_big<CONJ_A, TM>, grid, big::THREADS, smem, st, M, N, K, alpha, A, lda, B, ldb, beta, C, ldc, kchunk,
                                                              part);
     Q3B_LAUNCH_CHECK();
 }
@@ -480,7 +483,7 @@ void zgemm_big_launch(cudaStream_t st, bool conj_a, int M, int N, int K, double2
         const long total = (long)M * N;
         int blocks = ceil_div(total, 256);
         if (blocks > 4096) blocks = 4096;
-        splitk_reduce<double><<<blocks, 256, 0, st>>>(M, N, splits, part, alpha, beta, C, ldc);
+        launch_chained(splitk_reduce<double>, blocks, 256, 0, st, M, N, splits, part, alpha, beta, C, ldc);
         Q3B_LAUNCH_CHECK();
     }
 }
@@ -529,7 +532,7 @@ void cgemm(cudaStream_t st, bool conj_a, int M, int N, int K, cplx_t<R> alpha, c
     if (K <= 0) {
         // C = beta * C
         dim3 g(ceil_div((long)M * N, 256));
-        splitk_reduce<R><<<g, 256, 0, st>>>(M, N, 0, nullptr, alpha, beta, C, ldc);
+        launch_chained(splitk_reduce<R>, g, 256, 0, st, M, N, 0, nullptr, alpha, beta, C, ldc);
         Q3B_LAUNCH_CHECK();
         return;
     }

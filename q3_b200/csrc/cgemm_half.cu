@@ -67,6 +67,7 @@ __device__ __forceinline__ int exponent_for(float mx) {
 __device__ __forceinline__ float larger(float mx, float2 v) { return fmaxf(mx, fmaxf(fabsf(v.x), fabsf(v.y))); }
 
 __global__ void __launch_bounds__(256) exps_kmajor(int R, int K, const float2* __restrict__ X, long ld, int* exps) {
+    chain_begin();
     const int r = blockIdx.x;
     float mx = 0.f;
     if (r < R) {
@@ -90,6 +91,7 @@ __global__ void __launch_bounds__(256) exps_kmajor(int R, int K, const float2* _
 }
 
 __global__ void __launch_bounds__(256) exps_mmajor(int R, int K, const float2* __restrict__ X, long ld, int* exps) {
+    chain_begin();
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, r = blockIdx.x * 32 + lane;
     float mx = 0.f;
     if (r < R) {
@@ -126,6 +128,7 @@ constexpr int PACK_PITCH = 8 * 9 + 1;  // float2 per row: chunks of 8 + 1, odd i
 template <bool KMAJOR, int ROWS, int AS>
 __global__ void __launch_bounds__(256) pack_rows(int R, int K, const float2* __restrict__ X, long ld,
                                                  const int* __restrict__ exps, int nkb, unsigned char* out) {
+    chain_begin();
     __shared__ float2 s[PACK_ROWS * PACK_PITCH];
     const int tid = threadIdx.x, kb = blockIdx.y, k0 = kb * BK, r0 = blockIdx.x * PACK_ROWS;
     float2 in[PACK_ROWS * BK / 256];
@@ -214,6 +217,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(THREADS, 1)
 half_gemm(Units un, int total, int M, int N, const unsigned char* __restrict__ A, const unsigned char* __restrict__ B,
           const int* __restrict__ ea, const int* __restrict__ eb, float2 alpha, float2 beta, float2* C, long ldc,
           float2* part, int* err) {
+    chain_begin();
     constexpr int B_TILE = Cols<BC>::b_tile, STAGE = A_TILE + B_TILE, PLANE = Cols<BC>::plane;
     extern __shared__ __align__(1024) unsigned char smem_raw[];
     __shared__ __align__(8) uint64_t full_bar[STAGES], peer_full[STAGES], empty_bar[STAGES], acc_full[2], acc_empty[2],
@@ -391,6 +395,7 @@ half_gemm(Units un, int total, int M, int N, const unsigned char* __restrict__ A
 // C = alpha * sum_z part[z] + beta * C, the ranges in order
 __global__ void sum_ranges(int M, int N, int ranges, const float2* __restrict__ part, float2 alpha, float2 beta,
                            float2* C, long ldc) {
+    chain_begin();
     const long total = (long)M * N;
     const bool use_beta = (beta.x != 0.f || beta.y != 0.f);
     for (long i = blockIdx.x * (long)blockDim.x + threadIdx.x; i < total; i += (long)gridDim.x * blockDim.x) {
@@ -461,10 +466,10 @@ template <bool KMAJOR, int ROWS, int AS>
 void pack_operand(cudaStream_t st, int R, int K, const float2* X, long ld, unsigned char* tiles, int* exps) {
     const int padded = ceil_div(R, 2 * ROWS) * 2 * ROWS, nkb = ceil_div(K, BK);
     if (nkb > 65535) throw std::runtime_error("tensor-core GEMM: operand too large to pack");
-    if (KMAJOR) exps_kmajor<<<padded, 256, 0, st>>>(R, K, X, ld, exps);
-    else exps_mmajor<<<padded / 32, 256, 0, st>>>(R, K, X, ld, exps);
+    if (KMAJOR) launch_chained(exps_kmajor, padded, 256, 0, st, R, K, X, ld, exps);
+    else launch_chained(exps_mmajor, padded / 32, 256, 0, st, R, K, X, ld, exps);
     Q3B_LAUNCH_CHECK();
-    pack_rows<KMAJOR, ROWS, AS><<<dim3(padded / PACK_ROWS, nkb), 256, 0, st>>>(R, K, X, ld, exps, nkb, tiles);
+    launch_chained(pack_rows<KMAJOR, ROWS, AS>, dim3(padded / PACK_ROWS, nkb), 256, 0, st, R, K, X, ld, exps, nkb, tiles);
     Q3B_LAUNCH_CHECK();
 }
 
@@ -475,12 +480,12 @@ void run(cudaStream_t st, const Plan& p, int M, int N, int K, float2 alpha, cons
     const long units = (long)p.mt * p.nt * p.splits, pairs = device_sms() / 2 > 0 ? device_sms() / 2 : 1;
     if (units > 0x7fffffffL) throw std::runtime_error("tensor-core GEMM: too large");
     const int grid = 2 * static_cast<int>(units < pairs ? units : pairs);
-    half_gemm<CONJ_A, BC><<<grid, THREADS, Cols<BC>::smem, st>>>(Units{p.nt, p.mt, p.kb_per, p.nkb}, (int)units, M, N,
+    launch_chained(half_gemm<CONJ_A, BC>, grid, THREADS, Cols<BC>::smem, st, Units{p.nt, p.mt, p.kb_per, p.nkb}, (int)units, M, N,
                                                                  A.tiles, bt, A.exps, eb, alpha, beta, C, ldc, part,
                                                                  tc::error_word());
     Q3B_LAUNCH_CHECK();
     if (part) {
-        sum_ranges<<<stride_grid((long)M * N, 16), 256, 0, st>>>(M, N, p.splits, part, alpha, beta, C, ldc);
+        launch_chained(sum_ranges, stride_grid((long)M * N, 16), 256, 0, st, M, N, p.splits, part, alpha, beta, C, ldc);
         Q3B_LAUNCH_CHECK();
     }
 }

@@ -349,6 +349,7 @@ __global__ void __launch_bounds__(THREADS, 1)
 cgemm_tc_kernel(int M, int N, int K, float2 alpha, const float2* __restrict__ A, long lda,
                 const unsigned char* __restrict__ Apk, const float2* __restrict__ B, long ldb, float2 beta,
                 float2* C, long ldc, int kchunk, float2* part, int* err) {
+    chain_begin();
     extern __shared__ __align__(1024) unsigned char smem_raw[];
     __shared__ __align__(8) uint64_t full_bar[STAGES];
     __shared__ __align__(8) uint64_t empty_bar[STAGES];
@@ -525,6 +526,7 @@ cgemm_tc_kernel(int M, int N, int K, float2 alpha, const float2* __restrict__ A,
 
 __global__ void splitk_sum(int M, int N, int splits, const float2* __restrict__ part, float2 alpha, float2 beta,
                            float2* C, long ldc) {
+    chain_begin();
     const long total = (long)M * N;
     const bool use_beta = (beta.x != 0.f || beta.y != 0.f);
     for (long idx = blockIdx.x * (long)blockDim.x + threadIdx.x; idx < total; idx += (long)gridDim.x * blockDim.x) {
@@ -630,7 +632,7 @@ void launch(cudaStream_t st, bool conj_a, int M, int N, int K, float2 alpha, con
     dim3 grid(ceil_div(N, BN), ceil_div(M, BM), splits);
     float2* part = splits > 1 ? static_cast<float2*>(ws.ptr) : nullptr;
 #define Q3B_TC_LAUNCH(CA, PA)                                                                             \
-    cgemm_tc_kernel<CA, PA><<<grid, THREADS, SMEM_BYTES, st>>>(M, N, K, alpha, A, lda, Apk, B, ldb, beta, C, \
+    launch_chained(cgemm_tc_kernel<CA, PA>, grid, THREADS, SMEM_BYTES, st, M, N, K, alpha, A, lda, Apk, B, ldb, beta, C, \
                                                                ldc, kchunk, part, err)
     if (Apk) {
         if (conj_a) Q3B_TC_LAUNCH(true, true);
@@ -645,7 +647,7 @@ void launch(cudaStream_t st, bool conj_a, int M, int N, int K, float2 alpha, con
         const long total = (long)M * N;
         int blocks = ceil_div(total, 256);
         if (blocks > 4096) blocks = 4096;
-        splitk_sum<<<blocks, 256, 0, st>>>(M, N, splits, part, alpha, beta, C, ldc);
+        launch_chained(splitk_sum, blocks, 256, 0, st, M, N, splits, part, alpha, beta, C, ldc);
         Q3B_LAUNCH_CHECK();
     }
 }

@@ -85,6 +85,41 @@ void count_launch();
         Q3B_CUDA(cudaGetLastError()); \
     } while (0)
 
+// Launches in chains.  A kernel started by launch_chained may be set up on the
+// SMs while its predecessor on the stream still runs; it begins with
+// chain_begin(), which waits until the predecessor has finished and its writes
+// are visible, and only then lets its own successor be set up.  So every
+// kernel still sees what a plain launch would, without the launch latency
+// between two short kernels.  chain_begin() returns at once in a kernel that was
+// launched plainly.
+//
+// Only a grid of at most one block an SM lets its successor in early: the blocks
+// of a successor that comes while some SMs are full settle on the others instead
+// of spreading over all of them, and where a product has one block for each SM
+// that costs more than the latency.  H|psi> launched plainly, let in by any grid of
+// up to four blocks an SM, and as it is: eight atoms 75.7, 85.5 and 68.4 us, two
+// atoms 37.4, 34.1 and 34.4.  Grids above kChainBlocks are launched plainly.
+constexpr int kEarlyBlocks = 148, kChainBlocks = 4 * 148;
+__device__ __forceinline__ void chain_begin() {
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    if ((unsigned long long)gridDim.x * gridDim.y * gridDim.z <= kEarlyBlocks)
+        asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+}
+template <typename... P, typename... A>
+inline void launch_chained(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, A&&... args) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = grid;
+    cfg.blockDim = block;
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = st;
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = at;
+    cfg.numAttrs = (unsigned long long)grid.x * grid.y * grid.z <= kChainBlocks ? 1 : 0;
+    Q3B_CUDA(cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...));
+}
+
 // Pinned host memory of the calling host thread, at least `bytes` long, for
 // small device->host reads (status words, eigenvalues, norms).  A read into
 // pageable memory is staged by the driver through memory it shares between

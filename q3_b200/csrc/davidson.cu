@@ -50,6 +50,7 @@ inline int grid_for(long n) { return stride_grid(n, 16); }
 template <typename R>
 __global__ void precondition_kernel(int npw, int ncols, const double* __restrict__ ke,
                                     const double* __restrict__ eps, cplx_t<R>* X) {
+    chain_begin();
     const long total = (long)npw * ncols;
     for (long idx = blockIdx.x * (long)blockDim.x + threadIdx.x; idx < total;
          idx += (long)gridDim.x * blockDim.x) {
@@ -71,6 +72,7 @@ template <typename R>
 __global__ void pack_coefficients(int n, int ncols, const double2* __restrict__ evec,
                                   const int* __restrict__ idx, const double* __restrict__ w,
                                   cplx_t<R>* out, cplx_t<R>* outneg, double* eps) {
+    chain_begin();
     const long total = (long)n * ncols;
     for (long t = blockIdx.x * (long)blockDim.x + threadIdx.x; t < total;
          t += (long)gridDim.x * blockDim.x) {
@@ -87,6 +89,7 @@ __global__ void pack_coefficients(int n, int ncols, const double2* __restrict__ 
 
 template <typename R>
 __global__ void unit_vectors(int npw, int count, const int* __restrict__ gidx, cplx_t<R>* V) {
+    chain_begin();
     const long total = (long)npw * count;
     for (long t = blockIdx.x * (long)blockDim.x + threadIdx.x; t < total;
          t += (long)gridDim.x * blockDim.x) {
@@ -98,6 +101,7 @@ __global__ void unit_vectors(int npw, int count, const int* __restrict__ gidx, c
 
 template <typename R>
 __global__ void scale_vector(long n, cplx_t<R>* v, double s) {
+    chain_begin();
     for (long i = blockIdx.x * (long)blockDim.x + threadIdx.x; i < n; i += (long)gridDim.x * blockDim.x) {
         cplx_t<R> x = v[i];
         x.x = static_cast<R>(x.x * s);
@@ -109,6 +113,7 @@ __global__ void scale_vector(long n, cplx_t<R>* v, double s) {
 // dst (double2, ld ldd) = src (R, ld lds), an M x N block
 template <typename R>
 __global__ void widen_block(int M, int N, const cplx_t<R>* __restrict__ src, int lds, double2* dst, int ldd) {
+    chain_begin();
     const long total = (long)M * N;
     for (long t = blockIdx.x * (long)blockDim.x + threadIdx.x; t < total;
          t += (long)gridDim.x * blockDim.x) {
@@ -120,6 +125,7 @@ __global__ void widen_block(int M, int N, const cplx_t<R>* __restrict__ src, int
 
 template <typename R>
 __global__ void narrow_block(int M, int N, const double2* __restrict__ src, int lds, cplx_t<R>* dst, int ldd) {
+    chain_begin();
     const long total = (long)M * N;
     for (long t = blockIdx.x * (long)blockDim.x + threadIdx.x; t < total;
          t += (long)gridDim.x * blockDim.x) {
@@ -133,6 +139,7 @@ __global__ void narrow_block(int M, int N, const double2* __restrict__ src, int 
 // gamma the half-sphere norm sqrt(2 sum |x|^2 - |x_0|^2)
 template <typename R>
 __global__ void column_norms(int npw, const cplx_t<R>* __restrict__ X, double* out, int gamma = 0) {
+    chain_begin();
     const cplx_t<R>* x = X + (long)blockIdx.x * npw;
     double s = 0.0;
     for (int g = threadIdx.x; g < npw; g += blockDim.x) {
@@ -162,6 +169,7 @@ __global__ void column_norms(int npw, const cplx_t<R>* __restrict__ X, double* o
 template <typename T>
 __global__ void gamma_inner_fix(int M, int N, const T* __restrict__ A, long lda, const T* __restrict__ B, long ldb,
                                 T* C, long ldc) {
+    chain_begin();
     const long total = (long)M * N;
     for (long t = blockIdx.x * (long)blockDim.x + threadIdx.x; t < total; t += (long)gridDim.x * blockDim.x) {
         const int i = static_cast<int>(t % M), j = static_cast<int>(t / M);
@@ -173,6 +181,7 @@ __global__ void gamma_inner_fix(int M, int N, const T* __restrict__ A, long lda,
 }
 
 __global__ void set_identity(int n, double2* E) {
+    chain_begin();
     const long total = (long)n * n;
     for (long t = blockIdx.x * (long)blockDim.x + threadIdx.x; t < total; t += (long)gridDim.x * blockDim.x)
         E[t] = (t % n == t / n) ? mk(1.0, 0.0) : mk(0.0, 0.0);
@@ -282,7 +291,7 @@ template <typename R> class Davidson {
     void inner(int M, int N, const T* A, const T* B, T* C, long ldc) {
         gemm(true, M, N, npw_, one(), A, npw_, B, npw_, zero(), C, ldc);
         if (gamma_) {
-            gamma_inner_fix<T><<<grid_for((long)M * N), 256, 0, st_>>>(M, N, A, npw_, B, npw_, C, ldc);
+            launch_chained(gamma_inner_fix<T>, grid_for((long)M * N), 256, 0, st_, M, N, A, npw_, B, npw_, C, ldc);
             Q3B_LAUNCH_CHECK();
         }
     }
@@ -296,7 +305,7 @@ template <typename R> class Davidson {
         T* Tc = V_ + (size_t)start * npw_;
         T* STc = SV_ + (size_t)start * npw_;
         if (gamma_) {
-            gamma_real_origin<T><<<1, 256, 0, st_>>>(ncand, Tc, npw_);
+            launch_chained(gamma_real_origin<T>, 1, 256, 0, st_, ncand, Tc, npw_);
             Q3B_LAUNCH_CHECK();
         }
         apply_overlap(start, ncand);                                    // serial.hpp:62-68
@@ -334,7 +343,7 @@ template <typename R> class Davidson {
                 inner(nex, 1, Tc, v, coef_, nex);
                 gemm(false, npw_, 1, nex, mone(), Tc, npw_, coef_, nex, one(), v, npw_);
             }
-            column_norms<R><<<1, 256, 0, st_>>>(npw_, v, norms_, gamma_ ? 1 : 0);
+            launch_chained(column_norms<R>, 1, 256, 0, st_, npw_, v, norms_, gamma_ ? 1 : 0);
             Q3B_LAUNCH_CHECK();
             double* hb = static_cast<double*>(host_readback(sizeof(double)));
             Q3B_CUDA(cudaMemcpyAsync(hb, norms_, sizeof(double), cudaMemcpyDeviceToHost, st_));
@@ -342,7 +351,7 @@ template <typename R> class Davidson {
             const double nrm = hb[0];
             const double n2 = nrm * nrm;
             if (n2 > kNormThreshold) {
-                scale_vector<R><<<grid_for(npw_), 256, 0, st_>>>(npw_, v, 1.0 / nrm);
+                launch_chained(scale_vector<R>, grid_for(npw_), 256, 0, st_, npw_, v, 1.0 / nrm);
                 Q3B_LAUNCH_CHECK();
                 ++accepted;
             }
@@ -417,13 +426,13 @@ template <typename R> class Davidson {
         int ncand = std::min<int>(static_cast<int>(bands.size()), maxcand);
         if (ncand <= 0) return 0;
         upload_async(idx_, bands.data(), ncand * sizeof(int), st_);
-        pack_coefficients<R><<<grid_for((long)basis * ncand), 256, 0, st_>>>(basis, ncand, evec_, idx_, w_,
+        launch_chained(pack_coefficients<R>, grid_for((long)basis * ncand), 256, 0, st_, basis, ncand, evec_, idx_, w_,
                                                                              cpack_, cneg_, eps_);
         Q3B_LAUNCH_CHECK();
         T* Rc = V_ + (size_t)basis * npw_;
         gemm(false, npw_, ncand, basis, one(), SV_, npw_, cneg_, basis, zero(), Rc, npw_);  // -(SV)c eps
         gemm(false, npw_, ncand, basis, one(), HV_, npw_, cpack_, basis, one(), Rc, npw_);  // + (HV)c
-        precondition_kernel<R><<<grid_for((long)npw_ * ncand), 256, 0, st_>>>(npw_, ncand, ke_, eps_, Rc);
+        launch_chained(precondition_kernel<R>, grid_for((long)npw_ * ncand), 256, 0, st_, npw_, ncand, ke_, eps_, Rc);
         Q3B_LAUNCH_CHECK();
         return ncand;
     }
@@ -485,12 +494,12 @@ template <typename R> class Davidson {
         std::vector<int> all(nb_);
         std::iota(all.begin(), all.end(), 0);
         upload_async(idx_, all.data(), nb_ * sizeof(int), st_);
-        pack_coefficients<R><<<grid_for((long)basis * nb_), 256, 0, st_>>>(basis, nb_, evec_, idx_, w_, cpack_,
+        launch_chained(pack_coefficients<R>, grid_for((long)basis * nb_), 256, 0, st_, basis, nb_, evec_, idx_, w_, cpack_,
                                                                            cneg_, eps_);
         Q3B_LAUNCH_CHECK();
         gemm(false, npw_, nb_, basis, one(), SV_, npw_, cneg_, basis, zero(), tmp_, npw_);
         gemm(false, npw_, nb_, basis, one(), HV_, npw_, cpack_, basis, one(), tmp_, npw_);
-        column_norms<R><<<nb_, 256, 0, st_>>>(npw_, tmp_, norms_, gamma_ ? 1 : 0);
+        launch_chained(column_norms<R>, nb_, 256, 0, st_, npw_, tmp_, norms_, gamma_ ? 1 : 0);
         Q3B_LAUNCH_CHECK();
         double* h = static_cast<double*>(host_readback(nb_ * sizeof(double)));
         Q3B_CUDA(cudaMemcpyAsync(h, norms_, nb_ * sizeof(double), cudaMemcpyDeviceToHost, st_));
@@ -518,7 +527,7 @@ template <typename R> class Davidson {
         const T* in = v;
         T* out = sv;
         if (gamma_) {
-            gamma_pack<T><<<gamma_blocks((long)npw_ * nv), 256, 0, st_>>>(npw_, count, v, npw_, gphi_, nfull);
+            launch_chained(gamma_pack<T>, gamma_blocks((long)npw_ * nv), 256, 0, st_, npw_, count, v, npw_, gphi_, nfull);
             Q3B_LAUNCH_CHECK();
             in = gphi_;
             out = ghphi_;
@@ -533,7 +542,7 @@ template <typename R> class Davidson {
                                       nonlocal_wanted_bytes<R>(c_.overlap<R>(), len, nv));
         apply_nonlocal<R>(st_, c_.overlap<R>(), len, nv, in, len, out, len, c_.ws_bm.as<T>(), c_.ws_bp.as<T>(), ws);
         if (gamma_) {
-            gamma_unpack<T><<<gamma_blocks((long)npw_ * nv), 256, 0, st_>>>(npw_, count, ghphi_, nfull, sv, npw_);
+            launch_chained(gamma_unpack<T>, gamma_blocks((long)npw_ * nv), 256, 0, st_, npw_, count, ghphi_, nfull, sv, npw_);
             Q3B_LAUNCH_CHECK();
         }
     }
@@ -567,9 +576,9 @@ template <typename R> class Davidson {
             const double n2 = static_cast<double>(hb[0].x);
             if (n2 > kNormThreshold) {
                 const double inv = 1.0 / std::sqrt(n2);
-                scale_vector<R><<<grid_for(npw_), 256, 0, st_>>>(npw_, v, inv);
+                launch_chained(scale_vector<R>, grid_for(npw_), 256, 0, st_, npw_, v, inv);
                 Q3B_LAUNCH_CHECK();
-                scale_vector<R><<<grid_for(npw_), 256, 0, st_>>>(npw_, sv, inv);
+                launch_chained(scale_vector<R>, grid_for(npw_), 256, 0, st_, npw_, sv, inv);
                 Q3B_LAUNCH_CHECK();
                 ++accepted;
             }
@@ -582,11 +591,11 @@ template <typename R> class Davidson {
         if (gamma_) {
             // two bands per full-sphere vector (hamiltonian_applicator/serial.hpp:283-418)
             const int nfull = c_.kp.npw, np = (count + 1) / 2;
-            gamma_pack<T><<<gamma_blocks((long)npw_ * np), 256, 0, st_>>>(npw_, count, V_ + (size_t)first * npw_,
+            launch_chained(gamma_pack<T>, gamma_blocks((long)npw_ * np), 256, 0, st_, npw_, count, V_ + (size_t)first * npw_,
                                                                          npw_, gphi_, nfull);
             Q3B_LAUNCH_CHECK();
             c_.apply_h<R>(gphi_, nfull, ghphi_, nfull, np);
-            gamma_unpack<T><<<gamma_blocks((long)npw_ * np), 256, 0, st_>>>(npw_, count, ghphi_, nfull,
+            launch_chained(gamma_unpack<T>, gamma_blocks((long)npw_ * np), 256, 0, st_, npw_, count, ghphi_, nfull,
                                                                            HV_ + (size_t)first * npw_, npw_);
             Q3B_LAUNCH_CHECK();
         } else {
@@ -642,7 +651,7 @@ template <typename R> class Davidson {
             for (int band = start; band < nb_; ++band) gsel.push_back(order[band]);
             const int ncand = static_cast<int>(gsel.size());
             upload_async(idx_, gsel.data(), ncand * sizeof(int), st_);
-            unit_vectors<R><<<grid_for((long)npw_ * ncand), 256, 0, st_>>>(npw_, ncand, idx_,
+            launch_chained(unit_vectors<R>, grid_for((long)npw_ * ncand), 256, 0, st_, npw_, ncand, idx_,
                                                                            V_ + (size_t)basis * npw_);
             Q3B_LAUNCH_CHECK();
             basis += orthogonalize(basis, ncand);
@@ -671,7 +680,7 @@ template <typename R> class Davidson {
             int info = 0;
             if (reuse_collapse_ && basis == nb_) {
                 whost_ = collapse_w_;
-                set_identity<<<grid_for((long)nb_ * nb_), 256, 0, st_>>>(nb_, evec_);
+                launch_chained(set_identity, grid_for((long)nb_ * nb_), 256, 0, st_, nb_, evec_);
                 Q3B_LAUNCH_CHECK();
             } else {
                 info = diagonalize(basis, Hs_, Ss_, maxn_);
@@ -752,7 +761,7 @@ template <typename R> class Davidson {
         int info = 0;                                                     // :816-840
         if (reuse_collapse_ && basis == nb_) {
             whost_ = collapse_w_;
-            set_identity<<<grid_for((long)nb_ * nb_), 256, 0, st_>>>(nb_, evec_);
+            launch_chained(set_identity, grid_for((long)nb_ * nb_), 256, 0, st_, nb_, evec_);
             Q3B_LAUNCH_CHECK();
         } else {
             info = diagonalize(basis, Hs_, Ss_, maxn_);
@@ -773,7 +782,7 @@ template <typename R> class Davidson {
 
   private:
     void widen(int M, int N, const T* src, int lds, double2* dst, int ldd) {
-        widen_block<R><<<grid_for((long)M * N), 256, 0, st_>>>(M, N, src, lds, dst, ldd);
+        launch_chained(widen_block<R>, grid_for((long)M * N), 256, 0, st_, M, N, src, lds, dst, ldd);
         Q3B_LAUNCH_CHECK();
     }
     const T* narrowed(int M, int N, const double2* src, int lds, T* buf) {
@@ -784,7 +793,7 @@ template <typename R> class Davidson {
             (void)buf;
             return src;
         } else {
-            narrow_block<R><<<grid_for((long)M * N), 256, 0, st_>>>(M, N, src, lds, buf, M);
+            launch_chained(narrow_block<R>, grid_for((long)M * N), 256, 0, st_, M, N, src, lds, buf, M);
             Q3B_LAUNCH_CHECK();
             return buf;
         }

@@ -74,6 +74,7 @@ __device__ __forceinline__ void pivot_terms(double piv, int j, int bs, int r0, d
 
 __global__ void __launch_bounds__(1024, 1)
 potrf_diag(int n, int k, double2* A, int lda, double2* dinv, int* info) {
+    chain_begin();
     if (vload(info)) return;
     __shared__ double2 a[NB][NB + 1];  // a[c][r] = G(r, c)
     __shared__ double2 u[NB][NB + 1];  // u[c][r] = U(r, c)
@@ -125,6 +126,7 @@ potrf_diag(int n, int k, double2* A, int lda, double2* dinv, int* info) {
 // U(k, j) = U_kk^{-H} G(k, j) for every block column j > k
 __global__ void __launch_bounds__(256)
 potrf_panel(int n, int k, double2* A, int lda, const double2* dinv, const int* info) {
+    chain_begin();
     if (vload(info)) return;
     __shared__ double2 xk[NB][NB + 1];  // xk[c][r] = Xk(r, c)
     __shared__ double2 g[NB][NB + 1];   // g[c][t] = G(k_t, j_c)
@@ -148,6 +150,7 @@ potrf_panel(int n, int k, double2* A, int lda, const double2* dinv, const int* i
 
 // G(i, j) -= U(k, i)^H U(k, j) for k < i <= j
 __global__ void __launch_bounds__(256) potrf_update(int n, int k, double2* A, int lda, const int* info) {
+    chain_begin();
     if (vload(info)) return;
     const int i = k + 1 + blockIdx.x, j = k + 1 + blockIdx.y;
     if (i > j) return;
@@ -174,6 +177,7 @@ __global__ void __launch_bounds__(256) potrf_update(int n, int k, double2* A, in
 
 // ------------------------------------------------------------------ trtri
 __global__ void trtri_diag(int n, const double2* dinv, double2* U) {
+    chain_begin();
     const int k = blockIdx.x;
     const int r0 = k * NB, bs = min(NB, n - r0);
     for (int idx = threadIdx.x; idx < NB * NB; idx += blockDim.x) {
@@ -193,6 +197,7 @@ __global__ void trtri_diag(int n, const double2* dinv, double2* U) {
 // the current one is multiplied.
 __global__ void __launch_bounds__(256)
 trtri_level(int n, int m, int mode, const double2* U, int ldu, double2* Ui, double2* T) {
+    chain_begin();
     const int p = blockIdx.x, ti = blockIdx.y, tj = blockIdx.z;
     const int r1 = 2 * m * p, r2 = r1 + m;
     const int m2 = min(m, n - r2);
@@ -258,6 +263,7 @@ trtri_level(int n, int m, int mode, const double2* U, int ldu, double2* Ui, doub
 // ------------------------------------------------------------------ helpers
 // dst (n x n, ld n) = full Hermitian matrix from the upper triangle of src (ld lds)
 __global__ void hermitian_from_upper(int n, const double2* src, int lds, double2* dst) {
+    chain_begin();
     const long total = (long)n * n;
     for (long idx = blockIdx.x * (long)blockDim.x + threadIdx.x; idx < total;
          idx += (long)gridDim.x * blockDim.x) {
@@ -271,6 +277,7 @@ __global__ void hermitian_from_upper(int n, const double2* src, int lds, double2
 }
 
 __global__ void copy_matrix(int n, const double2* src, int lds, double2* dst, int ldd) {
+    chain_begin();
     const long total = (long)n * n;
     for (long idx = blockIdx.x * (long)blockDim.x + threadIdx.x; idx < total;
          idx += (long)gridDim.x * blockDim.x) {
@@ -544,6 +551,7 @@ hetrd_smem(int n, int cpb, int w_in_smem, const double2* A, double* d, double2* 
 // across lanes)
 __global__ void tridiag_prep(int n, const double* d, const double2* e, double* ea, double* e2,
                              double2* phase, double* bounds) {
+    chain_begin();
     const int lane = threadIdx.x;
     if (blockIdx.x != 0 || lane >= 32) return;
     const int chunk = (n + 31) / 32;
@@ -598,6 +606,7 @@ __global__ void tridiag_prep(int n, const double* d, const double2* e, double* e
 
 // Yc[:, c] = phase .* Y[:, c] (complex)
 __global__ void apply_phase(int n, int nvec, const double2* phase, const double* Y, double2* Yc) {
+    chain_begin();
     const long total = (long)n * nvec;
     for (long t = blockIdx.x * (long)blockDim.x + threadIdx.x; t < total; t += (long)gridDim.x * blockDim.x) {
         const int r = static_cast<int>(t % n);
@@ -615,6 +624,7 @@ constexpr int kShifts = 2;
 constexpr int kSturmSmemOrder = 3072;
 __global__ void tridiag_multisect(int n, const double* d, const double* e2, const double* bounds, double* w,
                                   int nw) {
+    chain_begin();
     extern __shared__ double sturm_smem[];
     if (n <= kSturmSmemOrder) {
         for (int k = threadIdx.x; k < n; k += blockDim.x) {
@@ -662,6 +672,7 @@ __global__ void tridiag_multisect(int n, const double* d, const double* e2, cons
 // gap of 1e-5 ||T|| (orthogonality ~1e-11 across clusters).
 __global__ void tridiag_invit(int n, const double* d, const double* ea, const double* w,
                               const double* bounds, int nvec, double* Y, double* work) {
+    chain_begin();
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= nvec) return;
     const double scale = fmax(bounds[2], 1e-300);
@@ -750,6 +761,7 @@ __global__ void tridiag_invit(int n, const double* d, const double* ea, const do
 // 41 bytes per thread and row.
 __global__ void tridiag_invit_smem(int n, const double* d, const double* ea, const double* w,
                                    const double* bounds, int nvec, double* Y) {
+    chain_begin();
     extern __shared__ __align__(16) unsigned char smem[];
     const int T = blockDim.x, tid = threadIdx.x;
     double* DL = reinterpret_cast<double*>(smem);
@@ -877,13 +889,13 @@ void potrf_launch(cudaStream_t st, int n, double2* A, int lda, const Chol& c) {
     const int nblk = ceil_div(n, NB);
     Q3B_CUDA(cudaMemsetAsync(c.info, 0, sizeof(int), st));
     for (int k = 0; k < nblk; ++k) {
-        potrf_diag<<<1, 1024, 0, st>>>(n, k, A, lda, c.dinv, c.info);
+        launch_chained(potrf_diag, 1, 1024, 0, st, n, k, A, lda, c.dinv, c.info);
         Q3B_LAUNCH_CHECK();
         const int m = nblk - k - 1;
         if (m > 0) {
-            potrf_panel<<<m, 256, 0, st>>>(n, k, A, lda, c.dinv, c.info);
+            launch_chained(potrf_panel, m, 256, 0, st, n, k, A, lda, c.dinv, c.info);
             Q3B_LAUNCH_CHECK();
-            potrf_update<<<dim3(m, m), 256, 0, st>>>(n, k, A, lda, c.info);
+            launch_chained(potrf_update, dim3(m, m), 256, 0, st, n, k, A, lda, c.info);
             Q3B_LAUNCH_CHECK();
         }
     }
@@ -900,14 +912,14 @@ int potrf_impl(cudaStream_t st, int n, double2* A, int lda, const Chol& c) {
 void trtri_impl(cudaStream_t st, int n, const double2* A, int lda, const Chol& c, double2* Ui) {
     const int nblk = ceil_div(n, NB);
     Q3B_CUDA(cudaMemsetAsync(Ui, 0, (size_t)n * n * sizeof(double2), st));
-    trtri_diag<<<nblk, 256, 0, st>>>(n, c.dinv, Ui);
+    launch_chained(trtri_diag, nblk, 256, 0, st, n, c.dinv, Ui);
     Q3B_LAUNCH_CHECK();
     for (int m = NB; m < n; m *= 2) {
         const int pairs = ceil_div(n, 2 * m);
         const dim3 grid(pairs, m / NB, m / NB);
-        trtri_level<<<grid, 256, 0, st>>>(n, m, 0, A, lda, Ui, c.tbuf);
+        launch_chained(trtri_level, grid, 256, 0, st, n, m, 0, A, lda, Ui, c.tbuf);
         Q3B_LAUNCH_CHECK();
-        trtri_level<<<grid, 256, 0, st>>>(n, m, 1, A, lda, Ui, c.tbuf);
+        launch_chained(trtri_level, grid, 256, 0, st, n, m, 1, A, lda, Ui, c.tbuf);
         Q3B_LAUNCH_CHECK();
     }
 }
@@ -1049,22 +1061,22 @@ void heev_launch(cudaStream_t st, const HeevPlan& p, const double2* A, double* w
         Q3B_CUDA(cudaLaunchKernelExC(&cfg, (const void*)hetrd_smem, args));
         Q3B_LAUNCH_CHECK();
     }
-    tridiag_prep<<<1, 32, 0, st>>>(n, p.d, p.e, p.ea, p.e2, p.phase, p.bounds);
+    launch_chained(tridiag_prep, 1, 32, 0, st, n, p.d, p.e, p.ea, p.e2, p.phase, p.bounds);
     Q3B_LAUNCH_CHECK();
     const int nw = nvec > 0 ? nvec : n;
     const size_t sturm_smem = n <= kSturmSmemOrder ? 2 * (size_t)n * sizeof(double) : 0;
-    tridiag_multisect<<<ceil_div((long)nw * 32, 256), 256, sturm_smem, st>>>(n, p.d, p.e2, p.bounds, w, nw);
+    launch_chained(tridiag_multisect, ceil_div((long)nw * 32, 256), 256, sturm_smem, st, n, p.d, p.e2, p.bounds, w, nw);
     Q3B_LAUNCH_CHECK();
     if (nvec > 0) {
         const int T = static_cast<int>(std::min<size_t>(64, kInvitSmemLimit / ((size_t)n * kInvitBytesPerRow)));
         if (T >= 1) {
             const size_t sm = (size_t)n * T * kInvitBytesPerRow;
-            tridiag_invit_smem<<<ceil_div(nvec, T), T, sm, st>>>(n, p.d, p.ea, w, p.bounds, nvec, p.Y);
+            launch_chained(tridiag_invit_smem, ceil_div(nvec, T), T, sm, st, n, p.d, p.ea, w, p.bounds, nvec, p.Y);
         } else {
-            tridiag_invit<<<ceil_div(nvec, 64), 64, 0, st>>>(n, p.d, p.ea, w, p.bounds, nvec, p.Y, p.work);
+            launch_chained(tridiag_invit, ceil_div(nvec, 64), 64, 0, st, n, p.d, p.ea, w, p.bounds, nvec, p.Y, p.work);
         }
         Q3B_LAUNCH_CHECK();
-        apply_phase<<<grid_for((long)n * nvec), 256, 0, st>>>(n, nvec, p.phase, p.Y, p.Yc);
+        launch_chained(apply_phase, grid_for((long)n * nvec), 256, 0, st, n, nvec, p.phase, p.Y, p.Yc);
         Q3B_LAUNCH_CHECK();
         const double2 one = mk(1.0, 0.0), zero = mk(0.0, 0.0);
         cgemm<double>(st, true, n, nvec, n, one, p.W, n, p.Yc, n, zero, Z, n, gws);   // Z = W^H (D Y)
@@ -1188,16 +1200,16 @@ int hegv(cudaStream_t st, int n, const double2* H, const double2* S, int ld, dou
     const HeevPlan hp = heev_plan(n, nvec, ws);
     auto issue = [&] {
         const double2 one = mk(1.0, 0.0), zero = mk(0.0, 0.0);
-        copy_matrix<<<grid_for((long)nn), 256, 0, st>>>(n, S, ld, Uw, n);
+        launch_chained(copy_matrix, grid_for((long)nn), 256, 0, st, n, S, ld, Uw, n);
         Q3B_LAUNCH_CHECK();
         potrf_launch(st, n, Uw, n, c);
         trtri_impl(st, n, Uw, n, c, Ui);
-        hermitian_from_upper<<<grid_for((long)nn), 256, 0, st>>>(n, H, ld, Hf);
+        launch_chained(hermitian_from_upper, grid_for((long)nn), 256, 0, st, n, H, ld, Hf);
         Q3B_LAUNCH_CHECK();
         cgemm<double>(st, false, n, n, n, one, Hf, n, Ui, n, zero, W, n, gws);     // H U^{-1}
         cgemm<double>(st, true, n, n, n, one, Ui, n, W, n, zero, Hf, n, gws);      // U^{-H} H U^{-1}
         // make it exactly Hermitian from its upper triangle
-        hermitian_from_upper<<<grid_for((long)nn), 256, 0, st>>>(n, Hf, n, W);
+        launch_chained(hermitian_from_upper, grid_for((long)nn), 256, 0, st, n, Hf, n, W);
         Q3B_LAUNCH_CHECK();
         heev_launch(st, hp, W, w, Zc, gws);
         if (nvec > 0) cgemm<double>(st, false, n, nvec, n, one, Ui, n, Zc, n, zero, Z, n, gws);

@@ -613,7 +613,8 @@ __device__ __forceinline__ void hegv_block_body(const BlockProblem& pr) {
     if (tid == 0) *pr.info = 0;
 }
 
-__global__ void __launch_bounds__(kBT, 1) hegv_block_one(BlockProblem p) { hegv_block_body(p); }
+__global__ void __launch_bounds__(kBT, 1) hegv_block_one(BlockProblem p) {
+    chain_begin(); hegv_block_body(p); }
 
 __global__ void __launch_bounds__(kBT, 1) hegv_block_many(const BlockProblem* ps, int count) {
     if ((int)blockIdx.x >= count) return;
@@ -624,7 +625,8 @@ __global__ void __launch_bounds__(kBT, 1) hegv_block_many(const BlockProblem* ps
 // Cholesky and inverse of one Gram matrix (the orthogonalisation's potrf +
 // trtri, subspace_manager/serial.hpp:334-339)
 __global__ void __launch_bounds__(kBT, 1)
-chol_inverse_block(int n, const double2* G, int ldg, double2* Uinv, int* info) {
+chol_inverse_one(int n, const double2* G, int ldg, double2* Uinv, int* info) {
+    chain_begin();
     extern __shared__ __align__(16) unsigned char sm[];
     const int P = pitch_of(n);
     double2* A = reinterpret_cast<double2*>(sm);
@@ -646,7 +648,7 @@ void set_block_attributes() {
                                       static_cast<int>(kSmemLimit)));
         Q3B_CUDA(cudaFuncSetAttribute(hegv_block_many, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                       static_cast<int>(kSmemLimit)));
-        Q3B_CUDA(cudaFuncSetAttribute(chol_inverse_block, cudaFuncAttributeMaxDynamicSharedMemorySize,
+        Q3B_CUDA(cudaFuncSetAttribute(chol_inverse_one, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                       static_cast<int>(kSmemLimit)));
     });
 }
@@ -676,14 +678,14 @@ void chol_inverse_block(cudaStream_t st, int n, const double2* G, int ldg, doubl
     if (!chol_inverse_block_fits(n) || ldg < n || !G || !Uinv || !info)
         throw Status(Q3B_ERR_INVALID, "block Cholesky: problem out of range");
     set_block_attributes();
-    chol_inverse_block<<<1, kBT, chol_smem(n), st>>>(n, G, ldg, Uinv, info);
+    launch_chained(chol_inverse_one, 1, kBT, chol_smem(n), st, n, G, ldg, Uinv, info);
     Q3B_LAUNCH_CHECK();
 }
 
 void hegv_block(cudaStream_t st, const BlockProblem& p) {
     if (!valid(p)) throw Status(Q3B_ERR_INVALID, "block eigensolver: problem out of range");
     set_block_attributes();
-    hegv_block_one<<<1, kBT, hegv_block_smem(p.n, p.nvec), st>>>(p);
+    launch_chained(hegv_block_one, 1, kBT, hegv_block_smem(p.n, p.nvec), st, p);
     Q3B_LAUNCH_CHECK();
 }
 

@@ -11,6 +11,7 @@ namespace q3b {
 template <typename T>
 __global__ void gamma_pack(int nhalf, int nvec, const T* __restrict__ psi, long ldpsi, T* __restrict__ phi,
                            long ldphi) {
+    chain_begin();
     const int npair = (nvec + 1) / 2;
     const long total = (long)nhalf * npair;
     for (long idx = blockIdx.x * (long)blockDim.x + threadIdx.x; idx < total;
@@ -43,6 +44,7 @@ __global__ void gamma_pack(int nhalf, int nvec, const T* __restrict__ psi, long 
 template <typename T>
 __global__ void gamma_unpack(int nhalf, int nvec, const T* __restrict__ F, long ldf, T* __restrict__ hpsi,
                              long ldh) {
+    chain_begin();
     using R = decltype(T{}.x);
     const int npair = (nvec + 1) / 2;
     const long total = (long)nhalf * npair;
@@ -73,6 +75,7 @@ __global__ void gamma_unpack(int nhalf, int nvec, const T* __restrict__ F, long 
 // origin coefficient
 template <typename T>
 __global__ void gamma_real_origin(int ncols, T* V, long ldv) {
+    chain_begin();
     for (int j = blockIdx.x * blockDim.x + threadIdx.x; j < ncols; j += gridDim.x * blockDim.x) V[(long)j * ldv].y = 0;
 }
 

@@ -64,6 +64,7 @@ constexpr int kSmallR = 10;
 template <typename R, int MAXR>
 __global__ void __launch_bounds__(kStickThreads)
 sticks_backward(LocalPlan<R> p, const cplx_t<R>* __restrict__ psi, long ldpsi, cplx_t<R>* X) {
+    chain_begin();
     using T = cplx_t<R>;
     extern __shared__ __align__(16) unsigned char smem[];
     T* tw = reinterpret_cast<T*>(smem);
@@ -115,6 +116,7 @@ template <typename R, int NT, int MAXR> constexpr int plane_min_blocks() {
 
 template <typename R, int NT, int MAXR>
 __global__ void __launch_bounds__(NT, (plane_min_blocks<R, NT, MAXR>())) planes(LocalPlan<R> p, cplx_t<R>* X) {
+    chain_begin();
     using T = cplx_t<R>;
     extern __shared__ __align__(16) unsigned char smem[];
     T* tw1 = reinterpret_cast<T*>(smem);
@@ -147,6 +149,7 @@ template <typename R, int MAXR>
 __global__ void __launch_bounds__(kStickThreads)
 sticks_forward(LocalPlan<R> p, const cplx_t<R>* __restrict__ X, const cplx_t<R>* __restrict__ psi,
                long ldpsi, cplx_t<R>* hpsi, long ldh) {
+    chain_begin();
     using T = cplx_t<R>;
     extern __shared__ __align__(16) unsigned char smem[];
     T* tw = reinterpret_cast<T*>(smem);
@@ -206,6 +209,7 @@ sticks_forward(LocalPlan<R> p, const cplx_t<R>* __restrict__ X, const cplx_t<R>*
 template <typename R>
 __global__ void kinetic_unmapped(LocalPlan<R> p, const cplx_t<R>* psi, long ldpsi, cplx_t<R>* hpsi,
                                  long ldh, int nvec) {
+    chain_begin();
     const long total = (long)p.nunmapped * nvec;
     for (long idx = blockIdx.x * (long)blockDim.x + threadIdx.x; idx < total;
          idx += (long)gridDim.x * blockDim.x) {
@@ -243,7 +247,7 @@ template <typename R> void set_smem_limits() {
 
 template <typename R, int NT, int MAXR>
 void launch_planes(dim3 grid, size_t smem, cudaStream_t st, const LocalPlan<R>& p, cplx_t<R>* X) {
-    planes<R, NT, MAXR><<<grid, NT, smem, st>>>(p, X);
+    launch_chained(planes<R, NT, MAXR>, grid, NT, smem, st, p, X);
 }
 
 // Charge density (accumulator.hpp:375-545, non-Gamma): the backward half of
@@ -257,6 +261,7 @@ constexpr int kAccBatch = 16;
 template <int MAXR>
 __global__ void __launch_bounds__(256, 2) planes_density(LocalPlan<double> p, const double2* X, int nb,
                                                       const double* w, double* partial, int groups) {
+    chain_begin();
     using T = double2;
     extern __shared__ __align__(16) unsigned char smem[];
     T* tw1 = reinterpret_cast<T*>(smem);
@@ -314,6 +319,7 @@ __global__ void __launch_bounds__(256, 2) planes_density(LocalPlan<double> p, co
 // the positions of (w1, w2, w3): digit-reversed, w1 only where w1_reversed
 __global__ void density_reduce(LocalPlan<double> p, int groups, const double* partial, double* rho,
                                int w1_reversed) {
+    chain_begin();
     const long n = (long)p.n1 * p.n2 * p.n3;
     const long nplane = (long)p.n1 * p.n2;
     for (long idx = blockIdx.x * (long)blockDim.x + threadIdx.x; idx < n; idx += (long)gridDim.x * blockDim.x) {
@@ -398,9 +404,9 @@ void run_sticks_backward(const LocalPlan<R>& p, const cplx_t<R>* psi, long ldpsi
     const dim3 grid(ceil_div(p.nsticks, p.sg), nb);
     if (sq_back(p, psi, ldpsi, X, nb, st)) {
     } else if (p.na3 <= kSmallR && p.nb3 <= kSmallR) {
-        sticks_backward<R, kSmallR><<<grid, kStickThreads, stick_smem_bytes(p), st>>>(p, psi, ldpsi, X);
+        launch_chained(sticks_backward<R, kSmallR>, grid, kStickThreads, stick_smem_bytes(p), st, p, psi, ldpsi, X);
     } else {
-        sticks_backward<R, 16><<<grid, kStickThreads, stick_smem_bytes(p), st>>>(p, psi, ldpsi, X);
+        launch_chained(sticks_backward<R, 16>, grid, kStickThreads, stick_smem_bytes(p), st, p, psi, ldpsi, X);
     }
     Q3B_LAUNCH_CHECK();
 }
@@ -411,9 +417,9 @@ void run_sticks_forward(const LocalPlan<R>& p, const cplx_t<R>* X, const cplx_t<
     const dim3 grid(ceil_div(p.nsticks, p.sg), nb);
     if (sq_fwd(p, X, psi, ldpsi, hpsi, ldh, nb, st)) {
     } else if (p.na3 <= kSmallR && p.nb3 <= kSmallR) {
-        sticks_forward<R, kSmallR><<<grid, kStickThreads, stick_smem_bytes(p), st>>>(p, X, psi, ldpsi, hpsi, ldh);
+        launch_chained(sticks_forward<R, kSmallR>, grid, kStickThreads, stick_smem_bytes(p), st, p, X, psi, ldpsi, hpsi, ldh);
     } else {
-        sticks_forward<R, 16><<<grid, kStickThreads, stick_smem_bytes(p), st>>>(p, X, psi, ldpsi, hpsi, ldh);
+        launch_chained(sticks_forward<R, 16>, grid, kStickThreads, stick_smem_bytes(p), st, p, X, psi, ldpsi, hpsi, ldh);
     }
     Q3B_LAUNCH_CHECK();
 }
@@ -462,7 +468,7 @@ void apply_local(cudaStream_t st, const LocalPlan<R>& p, const cplx_t<R>* psi, l
         const long total = (long)p.nunmapped * nvec;
         int blocks = ceil_div(total, 256);
         if (blocks > 1024) blocks = 1024;
-        kinetic_unmapped<R><<<blocks, 256, 0, st>>>(p, psi, ldpsi, hpsi, ldh, nvec);
+        launch_chained(kinetic_unmapped<R>, blocks, 256, 0, st, p, psi, ldpsi, hpsi, ldh, nvec);
         Q3B_LAUNCH_CHECK();
     }
 }
@@ -547,9 +553,9 @@ void accumulate_density(cudaStream_t st, const LocalPlan<double>& p, const doubl
         // groups leaves the remaining slabs as they are
         if (sq_density(p, X, nb, w + b0, partial, gb, st, nullptr)) {
         } else if (small12)
-            planes_density<kSmallR><<<dim3(p.n3, gb), 256, smem_p, st>>>(p, X, nb, w + b0, partial, gb);
+            launch_chained(planes_density<kSmallR>, dim3(p.n3, gb), 256, smem_p, st, p, X, nb, w + b0, partial, gb);
         else
-            planes_density<16><<<dim3(p.n3, gb), 256, smem_p, st>>>(p, X, nb, w + b0, partial, gb);
+            launch_chained(planes_density<16>, dim3(p.n3, gb), 256, smem_p, st, p, X, nb, w + b0, partial, gb);
         Q3B_LAUNCH_CHECK();
     }
     const long n = (long)p.n1 * p.n2 * p.n3;
@@ -557,7 +563,7 @@ void accumulate_density(cudaStream_t st, const LocalPlan<double>& p, const doubl
     if (blocks > 4096) blocks = 4096;
     int unused = 0;
     const int reversed = sq_density(p, nullptr, 0, nullptr, nullptr, 0, nullptr, &unused) ? 0 : 1;
-    density_reduce<<<blocks, 256, 0, st>>>(p, groups, partial, rho, reversed);
+    launch_chained(density_reduce, blocks, 256, 0, st, p, groups, partial, rho, reversed);
     Q3B_LAUNCH_CHECK();
 }
 

@@ -18,6 +18,7 @@ __global__ void apply_d_blocks(int P, int nvec, const int* __restrict__ pstart,
                                const int* __restrict__ psize, const int* __restrict__ poff,
                                const R* __restrict__ dpk, const cplx_t<R>* __restrict__ B,
                                cplx_t<R>* __restrict__ Bp) {
+    chain_begin();
     using T = cplx_t<R>;
     const long total = (long)P * nvec;
     for (long idx = blockIdx.x * (long)blockDim.x + threadIdx.x; idx < total;
@@ -39,6 +40,7 @@ __global__ void apply_d_blocks(int P, int nvec, const int* __restrict__ pstart,
 
 template <typename RI, typename RO>
 __global__ void convert_kernel(long n, const cplx_t<RI>* __restrict__ in, cplx_t<RO>* __restrict__ out) {
+    chain_begin();
     for (long i = blockIdx.x * (long)blockDim.x + threadIdx.x; i < n; i += (long)gridDim.x * blockDim.x) {
         const cplx_t<RI> v = in[i];
         out[i] = mk(static_cast<RO>(v.x), static_cast<RO>(v.y));
@@ -95,8 +97,7 @@ void apply_nonlocal(cudaStream_t st, const NonlocalData<R>& nl, int npw, int nve
     }
     if (tm) tm->end();
     if (tm) tm->begin(PhaseTimer::D_APPLY);
-    apply_d_blocks<R><<<grid_for((long)nl.nproj * nvec), 256, 0, st>>>(
-        nl.nproj, nvec, nl.pstart, nl.psize, nl.poff, nl.dpk, Bm, Bp);
+    launch_chained(apply_d_blocks<R>, grid_for((long)nl.nproj * nvec), 256, 0, st, nl.nproj, nvec, nl.pstart, nl.psize, nl.poff, nl.dpk, Bm, Bp);
     Q3B_LAUNCH_CHECK();
     if (tm) tm->end();
     if (tm) tm->begin(PhaseTimer::PROJ_ACCUM);
@@ -119,7 +120,7 @@ void apply_nonlocal(cudaStream_t st, const NonlocalData<R>& nl, int npw, int nve
 template <typename RI, typename RO>
 void convert(cudaStream_t st, long n, const cplx_t<RI>* in, cplx_t<RO>* out) {
     if (n <= 0) return;
-    convert_kernel<RI, RO><<<grid_for(n), 256, 0, st>>>(n, in, out);
+    launch_chained(convert_kernel<RI, RO>, grid_for(n), 256, 0, st, n, in, out);
     Q3B_LAUNCH_CHECK();
 }
 

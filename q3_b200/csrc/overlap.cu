@@ -15,6 +15,7 @@ namespace {
 // out = psi + (double) corr
 __global__ void add_widened(long n, const double2* __restrict__ psi, const float2* __restrict__ corr,
                             double2* __restrict__ out) {
+    chain_begin();
     for (long i = blockIdx.x * (long)blockDim.x + threadIdx.x; i < n; i += (long)gridDim.x * blockDim.x) {
         const double2 p = psi[i];
         const float2 c = corr[i];
@@ -55,7 +56,7 @@ void apply_s_device(Context& c, const double2* psi, double2* spsi, int nvec, int
                                      nonlocal_wanted_bytes<float>(c.overlap<float>(), npw, nvec));
         apply_nonlocal<float>(c.stream, c.overlap<float>(), npw, nvec, c.ws_conv_in.as<float2>(), npw,
                               c.ws_conv_out.as<float2>(), npw, c.ws_bm.as<float2>(), c.ws_bp.as<float2>(), ws);
-        add_widened<<<blocks_for((long)n), 256, 0, c.stream>>>((long)n, psi, c.ws_conv_out.as<float2>(), spsi);
+        launch_chained(add_widened, blocks_for((long)n), 256, 0, c.stream, (long)n, psi, c.ws_conv_out.as<float2>(), spsi);
         Q3B_LAUNCH_CHECK();
     } else {
         throw Status(Q3B_ERR_INVALID, "unknown precision");

@@ -204,6 +204,7 @@ __device__ __forceinline__ bool wait_phase0(uint64_t* bar, int* err) {
 template <typename R, int N, int L>
 __global__ void __launch_bounds__(reg_plane_threads<R, N, L>())
 planes_reg(LocalPlan<R> p, cplx_t<R>* X, int* err) {
+    chain_begin();
     using T = cplx_t<R>;
     constexpr int M = N / L;
     constexpr int PITCH = reg_plane_pitch<R, N>();
@@ -349,7 +350,7 @@ template <typename R, int N, int L> bool launch_one(const LocalPlan<R>& p, cplx_
         Q3B_CUDA(cudaFuncSetAttribute(planes_reg<R, N, L>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                       227 * 1024));
     });
-    planes_reg<R, N, L><<<dim3(p.n3, nb), reg_plane_threads<R, N, L>(), smem, st>>>(p, X, err);
+    launch_chained(planes_reg<R, N, L>, dim3(p.n3, nb), reg_plane_threads<R, N, L>(), smem, st, p, X, err);
     return true;
 }
 

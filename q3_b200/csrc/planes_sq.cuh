@@ -154,6 +154,7 @@ __device__ __forceinline__ void plane_in(const LocalPlan<R>& p, const PlaneSmem<
 
 template <typename R, int N, int NT, int MINB>
 __global__ void __launch_bounds__(NT, MINB) planes_sq(LocalPlan<R> p, cplx_t<R>* X) {
+    chain_begin();
     using T = cplx_t<R>;
     using G = Geometry<R, N>;
     constexpr int NA = G::NA, NB = G::NB, P = G::PITCH;
@@ -231,6 +232,7 @@ __global__ void __launch_bounds__(NT, MINB) planes_sq(LocalPlan<R> p, cplx_t<R>*
 template <int N, int NT, int MINB>
 __global__ void __launch_bounds__(NT, MINB)
 density_sq(LocalPlan<double> p, const double2* X, int nb, const double* __restrict__ wt, double* partial, int groups) {
+    chain_begin();
     using G = Geometry<double, N>;
     constexpr int NA = G::NA, NB = G::NB, P = G::PITCH;
     extern __shared__ __align__(16) unsigned char smem[];
@@ -283,6 +285,7 @@ template <typename R, int N> constexpr int stick_blocks() {
 template <typename R, int N>
 __global__ void __launch_bounds__(kStickNT, (stick_blocks<R, N>()))
 sticks_back(LocalPlan<R> p, const cplx_t<R>* __restrict__ psi, long ldpsi, cplx_t<R>* X) {
+    chain_begin();
     using T = cplx_t<R>;
     constexpr int NA = Geometry<R, N>::NA, NB = Geometry<R, N>::NB, P = StickSmem<R, N>::P, W = kStickNT / 32;
     extern __shared__ __align__(16) unsigned char smem[];
@@ -343,6 +346,7 @@ template <typename R, int N>
 __global__ void __launch_bounds__(kStickNT, (stick_blocks<R, N>()))
 sticks_fwd(LocalPlan<R> p, const cplx_t<R>* __restrict__ X, const cplx_t<R>* __restrict__ psi, long ldpsi,
            cplx_t<R>* hpsi, long ldh) {
+    chain_begin();
     using T = cplx_t<R>;
     constexpr int NA = Geometry<R, N>::NA, NB = Geometry<R, N>::NB, P = StickSmem<R, N>::P, W = kStickNT / 32;
     extern __shared__ __align__(16) unsigned char smem[];
@@ -426,7 +430,7 @@ template <typename R, int N, int NT> void launch(const LocalPlan<R>& p, cplx_t<R
         Q3B_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024));
         Q3B_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributePreferredSharedMemoryCarveout, 100));
     });
-    planes_sq<R, N, NT, MINB><<<dim3(p.n3, nb), NT, Geometry<R, N>::smem(p.nrows), st>>>(p, X);
+    launch_chained(planes_sq<R, N, NT, MINB>, dim3(p.n3, nb), NT, Geometry<R, N>::smem(p.nrows), st, p, X);
 }
 
 template <typename R, int N>
@@ -436,7 +440,7 @@ void launch_back(const LocalPlan<R>& p, const cplx_t<R>* psi, long ldpsi, cplx_t
     once.run([] {
         Q3B_CUDA(cudaFuncSetAttribute(sticks_back<R, N>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     });
-    sticks_back<R, N><<<dim3(ceil_div(p.nsticks, kGroup), nb), kStickNT, smem, st>>>(p, psi, ldpsi, X);
+    launch_chained(sticks_back<R, N>, dim3(ceil_div(p.nsticks, kGroup), nb), kStickNT, smem, st, p, psi, ldpsi, X);
 }
 template <typename R, int N>
 void launch_fwd(const LocalPlan<R>& p, const cplx_t<R>* X, const cplx_t<R>* psi, long ldpsi, cplx_t<R>* hpsi,
@@ -446,7 +450,7 @@ void launch_fwd(const LocalPlan<R>& p, const cplx_t<R>* X, const cplx_t<R>* psi,
     once.run([] {
         Q3B_CUDA(cudaFuncSetAttribute(sticks_fwd<R, N>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     });
-    sticks_fwd<R, N><<<dim3(ceil_div(p.nsticks, kGroup), nb), kStickNT, smem, st>>>(p, X, psi, ldpsi, hpsi, ldh);
+    launch_chained(sticks_fwd<R, N>, dim3(ceil_div(p.nsticks, kGroup), nb), kStickNT, smem, st, p, X, psi, ldpsi, hpsi, ldh);
 }
 
 // ------------------------------------------------------------------ dispatch
@@ -489,7 +493,7 @@ void density_of(const LocalPlan<double>& p, const double2* X, int nb, const doub
     density_limits<N>();
     const size_t smem = Geometry<double, N>::smem(p.nrows);
     if (nb > 0)
-        density_sq<N, B::NT, B::MINB><<<dim3(p.n3, groups), B::NT, smem, st>>>(p, X, nb, w, partial, groups);
+        launch_chained(density_sq<N, B::NT, B::MINB>, dim3(p.n3, groups), B::NT, smem, st, p, X, nb, w, partial, groups);
     else
         Q3B_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(per_sm, density_sq<N, B::NT, B::MINB>, B::NT, smem));
 }

@@ -148,6 +148,7 @@ __device__ __forceinline__ void take(double2 v, double& ss, double& mx) {
 // rows contiguous along K: one block a row
 __global__ void __launch_bounds__(256) exps_kmajor(int R, int K, const double2* __restrict__ X, long ld, double c,
                                                    int* exps) {
+    chain_begin();
     const int r = blockIdx.x;
     double ss = 0.0, mx = 0.0;
     if (r < R) {
@@ -182,6 +183,7 @@ __global__ void __launch_bounds__(256) exps_kmajor(int R, int K, const double2* 
 // rows along the contiguous index: 32 rows a block, K dealt to eight warps
 __global__ void __launch_bounds__(256) exps_mmajor(int R, int K, const double2* __restrict__ X, long ld, double c,
                                                    int* exps) {
+    chain_begin();
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     const int r = blockIdx.x * 32 + lane;
     double ss = 0.0, mx = 0.0;
@@ -228,6 +230,7 @@ enum PackAs { kPackA, kPackB, kPackBConj };
 template <bool KMAJOR, int ROWS, int AS>
 __global__ void __launch_bounds__(256) pack_rows(int R, int K, const double2* __restrict__ X, long ld,
                                                  const int* __restrict__ exps, int nkb, unsigned char* out) {
+    chain_begin();
     extern __shared__ __align__(16) unsigned char psm[];
     double2* s = reinterpret_cast<double2*>(psm);
     const int tid = threadIdx.x, kb = blockIdx.y, k0 = kb * BK, r0 = blockIdx.x * PACK_ROWS;
@@ -348,6 +351,7 @@ template <bool CONJ_A, int BC>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(THREADS, 1)
 zmod_gemm(Units un, int total, const unsigned char* __restrict__ A, const unsigned char* __restrict__ B,
           unsigned char* out, const __grid_constant__ ModTable tab, int* err) {
+    chain_begin();
     constexpr int B_TILE = Cols<BC>::b_tile, STAGE = A_TILE + B_TILE;
     extern __shared__ __align__(1024) unsigned char smem_raw[];
     __shared__ __align__(8) uint64_t full_bar[STAGES], peer_full[STAGES], empty_bar[STAGES], acc_full[2], acc_empty[2],
@@ -518,6 +522,7 @@ __global__ void __launch_bounds__(256)
 zmod_combine(int M, int N, int mt, int nt, int splits, const unsigned char* __restrict__ in,
              const int* __restrict__ ea, const int* __restrict__ eb, double product, double2 alpha, double2 beta,
              double2* C, long ldc) {
+    chain_begin();
     constexpr int GROUPS = BC / 4, OUT_TILE = Cols<BC>::out_tile;  // groups of eight columns a tile
     const int row = threadIdx.x >> 1, half = threadIdx.x & 1, cg = blockIdx.x % GROUPS, n = blockIdx.x / GROUPS;
     const int m = blockIdx.y, gm = m * BM + row, gn0 = n * 2 * BC + cg * 8 + half * 4;
@@ -682,10 +687,10 @@ template <bool KMAJOR, int ROWS, int AS>
 void pack_operand(cudaStream_t st, int R, int K, const double2* X, long ld, unsigned char* tiles, int* exps) {
     const int padded = ceil_div(R, 2 * ROWS) * 2 * ROWS, nkb = ceil_div(K, BK);
     if (nkb > 65535) throw std::runtime_error("complex GEMM: operand too large to pack");
-    if (KMAJOR) exps_kmajor<<<padded, 256, 0, st>>>(R, K, X, ld, scale_bits(), exps);
-    else exps_mmajor<<<padded / 32, 256, 0, st>>>(R, K, X, ld, scale_bits(), exps);
+    if (KMAJOR) launch_chained(exps_kmajor, padded, 256, 0, st, R, K, X, ld, scale_bits(), exps);
+    else launch_chained(exps_mmajor, padded / 32, 256, 0, st, R, K, X, ld, scale_bits(), exps);
     Q3B_LAUNCH_CHECK();
-    pack_rows<KMAJOR, ROWS, AS><<<dim3(padded / PACK_ROWS, nkb), 256, PACK_SMEM, st>>>(R, K, X, ld, exps, nkb, tiles);
+    launch_chained(pack_rows<KMAJOR, ROWS, AS>, dim3(padded / PACK_ROWS, nkb), 256, PACK_SMEM, st, R, K, X, ld, exps, nkb, tiles);
     Q3B_LAUNCH_CHECK();
 }
 void pack_rows_of_a(cudaStream_t st, int M, int K, const double2* A, long lda, bool kmajor, unsigned char* tiles,
@@ -703,14 +708,14 @@ void run_panel(cudaStream_t st, const Plan& p, int rows, int mt, int N, const un
     const Units un{p.nt, mt, p.splits, p.kb_per, p.nkb, !CONJ_A};
     const long pairs = device_sms() / 2 > 0 ? device_sms() / 2 : 1;
     const int grid = 2 * static_cast<int>(units < pairs ? units : pairs);
-    zmod_gemm<CONJ_A, BC><<<grid, THREADS, Cols<BC>::smem, st>>>(un, (int)units, a, b, out, tab, tc::error_word());
+    launch_chained(zmod_gemm<CONJ_A, BC>, grid, THREADS, Cols<BC>::smem, st, un, (int)units, a, b, out, tab, tc::error_word());
     Q3B_LAUNCH_CHECK();
     const dim3 cgrid(p.nt * (BC / 4), 2 * mt);
     if (p.splits > 1)
-        zmod_combine<true, BC><<<cgrid, 256, 0, st>>>(rows, N, 2 * mt, p.nt, p.splits, out, ea, eb, product, alpha,
+        launch_chained(zmod_combine<true, BC>, cgrid, 256, 0, st, rows, N, 2 * mt, p.nt, p.splits, out, ea, eb, product, alpha,
                                                       beta, C, ldc);
     else
-        zmod_combine<false, BC><<<cgrid, 256, 0, st>>>(rows, N, 2 * mt, p.nt, p.splits, out, ea, eb, product, alpha,
+        launch_chained(zmod_combine<false, BC>, cgrid, 256, 0, st, rows, N, 2 * mt, p.nt, p.splits, out, ea, eb, product, alpha,
                                                        beta, C, ldc);
     Q3B_LAUNCH_CHECK();
 }
