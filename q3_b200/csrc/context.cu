@@ -476,6 +476,8 @@ void Context::build_plan() {
     const int nent = start[S];
     constexpr int kStickGroup = 32;
     std::vector<int> eg(nent), ew3(nent), es(nent), ea(nent), fill(start.begin(), start.end() - 1);
+    std::vector<int> stick_map((size_t)S * n3, -1);
+    bool distinct = true;  // no two plane waves on one grid point
     for (int g = 0; g < k.npw; ++g) {
         if (gcol[g] < 0) continue;
         const int s = col_id[gcol[g]];
@@ -484,12 +486,16 @@ void Context::build_plan() {
         ew3[e] = gw3[g];
         es[e] = s;
         ea[e] = (s % kStickGroup) * p3 + gw3[g];
+        int& at = stick_map[(size_t)s * n3 + gw3[g]];
+        distinct = distinct && at < 0;
+        at = g;
     }
     upload(this, k.stick_start, start.data(), start.size());
     upload(this, k.entry_g, eg.data(), eg.size());
     upload(this, k.entry_w3, ew3.data(), ew3.size());
     upload(this, k.entry_stick, es.data(), es.size());
     upload(this, k.entry_at, ea.data(), ea.size());
+    upload(this, k.stick_map, stick_map.data(), stick_map.size());
     upload(this, k.stick_pos, stick_pos.data(), stick_pos.size());
     upload(this, k.row_base, rows.data(), rows.size());
     upload(this, k.row_map, row_map.data(), row_map.size());
@@ -532,6 +538,7 @@ void Context::build_plan() {
         lp.entry_w3 = k.entry_w3.as<int>();
         lp.entry_stick = k.entry_stick.as<int>();
         lp.entry_at = k.entry_at.as<int>();
+        lp.stick_map = distinct ? k.stick_map.as<int>() : nullptr;
         lp.stick_pos = k.stick_pos.as<int>();
         lp.row_base = k.row_base.as<int>();
         lp.row_map = k.row_map.as<short>();

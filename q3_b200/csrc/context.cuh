@@ -63,7 +63,7 @@ struct KPoint {
     bool has_q = false;             // ultrasoft overlap blocks set for this k-point
     DevBuf qpk64, qpk32;
     // sticks plan
-    DevBuf stick_start, entry_g, entry_w3, entry_stick, entry_at, stick_pos, row_map, row_base, unmapped;
+    DevBuf stick_start, entry_g, entry_w3, entry_stick, entry_at, stick_map, stick_pos, row_map, row_base, unmapped;
     DevBuf row_iv;  // int4 per stick row (LocalPlan::row_iv), when the sticks allow it
     DevBuf tw64[3], tw32[3];
     LocalPlan<double> lp64{};

@@ -33,6 +33,7 @@ template <typename R> struct LocalPlan {
     const int* entry_w3;
     const int* entry_stick;
     const int* entry_at;     // (stick % sg) * p3 + w3: its place in its block's lines
+    const int* stick_map;    // [stick][w3]: the G index there, or -1 (null when two share a grid point)
     const int* stick_pos;    // w1*p2 + w2
     const int* row_base;     // w1*p2 of each used row
     const short* row_map;    // [used row][w2]: the stick there, or -1 (grids up to 128 x 128)

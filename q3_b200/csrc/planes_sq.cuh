@@ -263,17 +263,24 @@ density_sq(LocalPlan<double> p, const double2* X, int nb, const double* __restri
 }
 
 // ------------------------------------------------------------------ sticks
-// Passes A and C (hpsi_local.cu) for a compile-time line length: 32 sticks a
-// block, one a lane, so that a warp's item is its number and no index is divided;
-// the place of a plane wave in the block's lines is read from the plan
-// (LocalPlan::entry_at) in one load.
+// Passes A and C (hpsi_local.cu) for a compile-time line length, 32 sticks a
+// block, one a lane where the stick buffer is read or written, so that no index
+// is divided there.  Bound: the latency of the gathers and of the buffer's L2
+// accesses.  Backward, the pass next to the sphere takes its values from psi
+// through the plan's map from (stick, w3) to plane waves (LocalPlan::stick_map),
+// its items running along q first so that neighbouring lanes meet neighbouring
+// entries, instead of clearing and filling the lines beforehand (the density of
+// the 64-atom cell 824 -> 816 us, FP32 backward 95 -> 90).  Forward, the values go
+// through the lines: handing them to H psi from that pass's registers took
+// 164 us instead of 98 (FP32, 256 bands of 80^3).  The general kernels took 130
+// and 176 us there.
 constexpr int kGroup = 32;      // sticks a block
 constexpr int kStickNT = 256;
 constexpr int kGathers = 4;     // global gathers a thread keeps in flight
 
 template <typename R, int N> struct StickSmem {
     static constexpr int P = N | 1;
-    static constexpr size_t bytes = (size_t)(2 * N + kGroup * P) * sizeof(cplx_t<R>);
+    static constexpr size_t bytes = (size_t)(N + kGroup * P) * sizeof(cplx_t<R>);
 };
 template <typename R, int N> constexpr int stick_blocks() {
     constexpr int regs = Geometry<R, N>::NA <= 10 ? (sizeof(R) == 8 ? 80 : 48) : (sizeof(R) == 8 ? 112 : 64);
@@ -290,44 +297,32 @@ sticks_back(LocalPlan<R> p, const cplx_t<R>* __restrict__ psi, long ldpsi, cplx_
     constexpr int NA = Geometry<R, N>::NA, NB = Geometry<R, N>::NB, P = StickSmem<R, N>::P, W = kStickNT / 32;
     extern __shared__ __align__(16) unsigned char smem[];
     T* twa = reinterpret_cast<T*>(smem);  // w^(q k) at [q < NB][k < NA]
-    T* lines = twa + 2 * N;
+    T* lines = twa + N;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int band = blockIdx.y, s0 = blockIdx.x * kGroup, ns = min(kGroup, p.nsticks - s0);
     for (int i = tid; i < N; i += kStickNT) twa[i] = p.tw3[(i / NA) * (i % NA)];
-    T* line = lines + lane * P;
-    for (int j = warp; j < N; j += W) line[j] = czero<T>();
     __syncthreads();
     const T* ps = psi + (long)band * ldpsi;
-    const int e1 = p.stick_start[s0 + ns];
-    for (int eb = p.stick_start[s0] + tid; eb < e1; eb += kGathers * kStickNT) {
-        T v[kGathers];
-        int at[kGathers];
-#pragma unroll
-        for (int u = 0; u < kGathers; ++u) {
-            const int e = eb + u * kStickNT;
-            at[u] = -1;
-            if (e < e1) {
-                at[u] = p.entry_at[e];
-                v[u] = ps[p.entry_g[e]];
-            }
-        }
-#pragma unroll
-        for (int u = 0; u < kGathers; ++u)
-            if (at[u] >= 0) lines[at[u]] = v[u];
-    }
-    __syncthreads();
 #pragma unroll 1
-    for (int q = warp; q < NB; q += W) {
+    for (int it = tid; it < ns * NB; it += kStickNT) {
+        const int l = it / NB, q = it % NB;
+        const int* at = p.stick_map + (long)(s0 + l) * N + q;
         const T* w = twa + q * NA;
+        int from[NA];
         T x[NA];
 #pragma unroll
-        for (int r = 0; r < NA; ++r) x[r] = line[q + NB * r];
-        fft::dft<NA, +1>(x, w, 0);
+        for (int r = 0; r < NA; ++r) from[r] = at[NB * r];
 #pragma unroll
-        for (int k = 0; k < NA; ++k) line[q + NB * k] = k ? cmulc(w[k], x[k]) : x[k];
+        for (int r = 0; r < NA; ++r) x[r] = from[r] >= 0 ? ps[from[r]] : czero<T>();
+        fft::dft<NA, +1>(x, w, 0);
+        T* b = lines + l * P + q;
+#pragma unroll
+        for (int k = 0; k < NA; ++k) b[NB * k] = k ? cmulc(w[k], x[k]) : x[k];
     }
     __syncthreads();
-    // the second pass leaves its values at positions NB q + k: straight to X
+    if (lane >= ns) return;
+    // the second pass leaves its values at positions NB q + k
+    const T* line = lines + lane * P;
     T* xb = X + (long)band * p.n3 * p.xpitch + s0 + lane;
 #pragma unroll 1
     for (int q = warp; q < NA; q += W) {
@@ -335,10 +330,8 @@ sticks_back(LocalPlan<R> p, const cplx_t<R>* __restrict__ psi, long ldpsi, cplx_
 #pragma unroll
         for (int r = 0; r < NB; ++r) x[r] = line[NB * q + r];
         fft::dft<NB, +1>(x, twa, 0);
-        if (lane < ns) {
 #pragma unroll
-            for (int k = 0; k < NB; ++k) xb[(long)(NB * q + k) * p.xpitch] = x[k];
-        }
+        for (int k = 0; k < NB; ++k) xb[(long)(NB * q + k) * p.xpitch] = x[k];
     }
 }
 
@@ -351,7 +344,7 @@ sticks_fwd(LocalPlan<R> p, const cplx_t<R>* __restrict__ X, const cplx_t<R>* __r
     constexpr int NA = Geometry<R, N>::NA, NB = Geometry<R, N>::NB, P = StickSmem<R, N>::P, W = kStickNT / 32;
     extern __shared__ __align__(16) unsigned char smem[];
     T* twb = reinterpret_cast<T*>(smem);  // w^(q k) at [q < NA][k < NB]
-    T* lines = twb + 2 * N;
+    T* lines = twb + N;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int band = blockIdx.y, s0 = blockIdx.x * kGroup, ns = min(kGroup, p.nsticks - s0);
     for (int i = tid; i < N; i += kStickNT) twb[i] = p.tw3[(i / NB) * (i % NB)];
@@ -530,6 +523,7 @@ void density_of(const LocalPlan<double>& p, const double2* X, int nb, const doub
     }                                                                                                          \
     bool NAME##_back(const LocalPlan<R>& p, const cplx_t<R>* psi, long ldpsi, cplx_t<R>* X, int nb,            \
                      cudaStream_t st) {                                                                        \
+        if (!p.stick_map) return false;                                                                        \
         switch (p.n3) {                                                                                        \
             SIZES(Q3B_SQ_BACK_##R)                                                                             \
             default: return false;                                                                             \
