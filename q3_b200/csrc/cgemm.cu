@@ -570,6 +570,43 @@ void cgemm(cudaStream_t st, bool conj_a, int M, int N, int K, cplx_t<R> alpha, c
     else run(std::false_type{});
 }
 
+namespace {
+size_t packed_once_bytes(int M, int K) {
+    return zmod::packed_a_bytes(M, K) + ((zmod::packed_a_exps(M) * sizeof(int) + 255) & ~size_t(255));
+}
+}  // namespace
+
+template <typename R> size_t cgemm_two_wanted_bytes(int M, int N, int K) {
+    if constexpr (std::is_same<R, double>::value) {
+        if (zmod::worth(true, M, N, K, false))
+            return packed_once_bytes(M, K) + zmod::workspace_bytes(true, M, N, K, true);
+    }
+    return 0;
+}
+
+template <typename R>
+void cgemm_two(cudaStream_t st, int M, int N, int K, const cplx_t<R>* A, long lda, const cplx_t<R>* B1,
+               const cplx_t<R>* B2, long ldb, cplx_t<R>* C1, cplx_t<R>* C2, long ldc, const GemmWorkspace& ws) {
+    const cplx_t<R> one = mk(R(1), R(0)), zero = mk(R(0), R(0));
+    if constexpr (std::is_same<R, double>::value) {
+        const size_t want = cgemm_two_wanted_bytes<R>(M, N, K);
+        if (want && ws.ptr && ws.bytes >= want && reinterpret_cast<uintptr_t>(A) % 16 == 0 &&
+            reinterpret_cast<uintptr_t>(B1) % 16 == 0 && reinterpret_cast<uintptr_t>(B2) % 16 == 0) {
+            unsigned char* tiles = static_cast<unsigned char*>(ws.ptr);
+            int* exps = reinterpret_cast<int*>(tiles + zmod::packed_a_bytes(M, K));
+            zmod::pack_a(st, M, K, A, lda, true, tiles, exps);
+            const zmod::PackedA pk{tiles, exps, M, K};
+            const size_t used = packed_once_bytes(M, K);
+            const GemmWorkspace rest{tiles + used, ws.bytes - used, ws.counters};
+            zmod::zgemm(st, true, M, N, K, one, nullptr, 0, &pk, B1, ldb, zero, C1, ldc, rest);
+            zmod::zgemm(st, true, M, N, K, one, nullptr, 0, &pk, B2, ldb, zero, C2, ldc, rest);
+            return;
+        }
+    }
+    cgemm<R>(st, true, M, N, K, one, A, lda, B1, ldb, zero, C1, ldc, ws);
+    cgemm<R>(st, true, M, N, K, one, A, lda, B2, ldb, zero, C2, ldc, ws);
+}
+
 double measure_dfma_tflops(cudaStream_t st) {
     int dev = 0, sms = 0;
     Q3B_CUDA(cudaGetDevice(&dev));
@@ -604,6 +641,9 @@ template void cgemm<float>(cudaStream_t, bool, int, int, int, float2, const floa
                            const float2*, long, float2, float2*, long, const GemmWorkspace&);
 template size_t cgemm_workspace_bytes<double>(int, int, int);
 template size_t cgemm_workspace_bytes<float>(int, int, int);
+template size_t cgemm_two_wanted_bytes<double>(int, int, int);
+template void cgemm_two<double>(cudaStream_t, int, int, int, const double2*, long, const double2*, const double2*,
+                                long, double2*, double2*, long, const GemmWorkspace&);
 template size_t cgemm_wanted_bytes<double>(bool, int, int, int);
 template size_t cgemm_wanted_bytes<float>(bool, int, int, int);
 

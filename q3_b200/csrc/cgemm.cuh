@@ -42,6 +42,13 @@ template <typename R> size_t cgemm_workspace_bytes(int M, int N, int K);
 // (zgemm_mod.cuh); with less it runs on the FP64 units
 template <typename R> size_t cgemm_wanted_bytes(bool conj_a, int M, int N, int K);
 
+// Two C,N products with the same A and shapes: C1 = A^H B1, C2 = A^H B2.  On the
+// integer tensor cores A is packed once for both.
+template <typename R>
+void cgemm_two(cudaStream_t st, int M, int N, int K, const cplx_t<R>* A, long lda, const cplx_t<R>* B1,
+               const cplx_t<R>* B2, long ldb, cplx_t<R>* C1, cplx_t<R>* C2, long ldc, const GemmWorkspace& ws);
+template <typename R> size_t cgemm_two_wanted_bytes(int M, int N, int K);
+
 // FP32 products of at least this many complex multiply-adds (M N K) run on
 // the tensor cores, smaller ones on the CUDA cores
 constexpr double kTensorCoreMinMacs = 67108864.0;  // 2^26

@@ -290,10 +290,12 @@ template <typename R> class Davidson {
     // half-sphere form
     void inner(int M, int N, const T* A, const T* B, T* C, long ldc) {
         gemm(true, M, N, npw_, one(), A, npw_, B, npw_, zero(), C, ldc);
-        if (gamma_) {
-            launch_chained(gamma_inner_fix<T>, grid_for((long)M * N), 256, 0, st_, M, N, A, npw_, B, npw_, C, ldc);
-            Q3B_LAUNCH_CHECK();
-        }
+        gamma_fix(M, N, A, B, C, ldc);
+    }
+    void gamma_fix(int M, int N, const T* A, const T* B, T* C, long ldc) {
+        if (!gamma_) return;
+        launch_chained(gamma_inner_fix<T>, grid_for((long)M * N), 256, 0, st_, M, N, A, npw_, B, npw_, C, ldc);
+        Q3B_LAUNCH_CHECK();
     }
     static T one() { return mk(R(1), R(0)); }
     static T zero() { return mk(R(0), R(0)); }
@@ -384,8 +386,13 @@ template <typename R> class Davidson {
         const T* Hn = HV_ + (size_t)start * npw_;
         const T* Sn = SV_ + (size_t)start * npw_;
         if constexpr (std::is_same<R, double>::value) {
-            inner(total, nnew, V_, Hn, Hs_ + (size_t)start * maxn_, maxn_);
-            inner(total, nnew, V_, Sn, Ss_ + (size_t)start * maxn_, maxn_);
+            double2 *h = Hs_ + (size_t)start * maxn_, *s = Ss_ + (size_t)start * maxn_;
+            GemmWorkspace ws = c_.gemm_ws(cgemm_workspace_bytes<R>(total, nnew, npw_),
+                                          std::max(cgemm_two_wanted_bytes<R>(total, nnew, npw_),
+                                                   cgemm_wanted_bytes<R>(true, total, nnew, npw_)));
+            cgemm_two<R>(st_, total, nnew, npw_, V_, npw_, Hn, Sn, npw_, h, s, maxn_, ws);
+            gamma_fix(total, nnew, V_, Hn, h, maxn_);
+            gamma_fix(total, nnew, V_, Sn, s, maxn_);
         } else {
             inner(total, nnew, V_, Hn, coef_, total);
             widen(total, nnew, coef_, total, Hs_ + (size_t)start * maxn_, maxn_);

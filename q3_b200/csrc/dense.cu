@@ -294,6 +294,12 @@ inline int grid_for(long n) { return stride_grid(n, 8); }
 // every pair has the value, with no fence and no separate flag to wait for (8-byte
 // halves of a vector access are single copies).  Steps count from 1; the buffers
 // are zeroed before the launch.
+// the sum of 16 values held twice across a warp, the same in every lane
+__device__ __forceinline__ double sum_over_half_warp(double v) {
+#pragma unroll
+    for (int o = 8; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+    return v;
+}
 struct Published {
     uint4 re, im;  // {low word, step, high word, step}
 };
@@ -412,14 +418,12 @@ hetrd_smem(int n, int cpb, int w_in_smem, const double2* A, double* d, double2* 
         __syncthreads();
         // the reflector, by every thread: v = x - alpha e_0 with alpha = -|x| x_0 / |x_0|,
         // tau = 2 / |v|^2 = 1 / (|x|^2 + |x| |x_0|)
-        double sigma = 0.0;
-#pragma unroll
-        for (int q = 0; q < WARPS; ++q) sigma += red[q];
+        const double sigma = sum_over_half_warp(red[lane & (WARPS - 1)]);
         const double2 x0 = sx[k + 1];
         double tk = 0.0;
         double2 alpha = x0;
         if (m > 1 && sigma > 0.0) {
-            const double a2 = x0.x * x0.x + x0.y * x0.y, n2 = sigma + a2, nrm = sqrt(n2);
+            const double a2 = x0.x * x0.x + x0.y * x0.y, n2 = sigma + a2, nrm = n2 * rsqrt(n2);
             // (below 1e-290 the square is no longer accurate, and x_0 counts for nothing)
             const double ra = a2 > 1e-290 ? rsqrt(a2) : 0.0, ax0 = a2 * ra;
             alpha = ra > 0.0 ? mk(-nrm * (x0.x * ra), -nrm * (x0.y * ra)) : mk(-nrm, 0.0);
@@ -495,9 +499,7 @@ hetrd_smem(int n, int cpb, int w_in_smem, const double2* A, double* d, double2* 
         double half = 0.0;
         double2 v0 = mk(0.0, 0.0), w0 = v0;
         if (tk != 0.0) {
-#pragma unroll
-            for (int q = 0; q < WARPS; ++q) half += redp[q];
-            half *= 0.5 * tk;
+            half = 0.5 * tk * sum_over_half_warp(redp[lane & (WARPS - 1)]);
             v0 = sv[0];
             w0 = mk(s_p0.x - half * v0.x, s_p0.y - half * v0.y);
         }
