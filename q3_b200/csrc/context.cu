@@ -190,11 +190,9 @@ GemmWorkspace Context::gemm_ws(size_t need, size_t want) {
 bool Context::release_optional() {
     // callers ask for the GEMM workspace after all their other buffers, so no
     // product that still has to be issued holds its address here
-    bool any = false;
-    for (DevBuf* b : {&kp.beta_zm_overlap, &kp.beta_zm_accum, &kp.beta_hs_overlap, &kp.beta_hs_accum}) {
-        any = any || b->ptr;
-        b->release();
-    }
+    bool any = kp.beta_packs.ptr != nullptr;
+    drop_packs();
+    kp.beta_packs.release();
     if (ws_gemm.bytes > ws_gemm_need_) {
         any = true;
         ws_gemm.release();
@@ -640,33 +638,45 @@ void Context::prepare_kpoint(int npw, const int32_t* g2g, const double* ke, cons
 // are.
 constexpr double kHalfMinMacs = 2e9;
 void Context::pack_projectors() {
-    for (DevBuf* b : {&kp.beta_zm_overlap, &kp.beta_zm_accum, &kp.beta_hs_overlap, &kp.beta_hs_accum}) b->release();
+    drop_packs();
     const int P = kp.nproj, npw = kp.npw;
     if (P <= 0) return;
-    auto pack = [&](auto convert_rows, DevBuf& buf, size_t tiles, size_t exps, const auto* beta, int M, int K, bool kmajor) {
-        if (!buf.try_reserve(this, tiles + exps * sizeof(int))) return;
-        unsigned char* t = buf.as<unsigned char>();
-        convert_rows(stream, M, K, beta, npw, kmajor, t, reinterpret_cast<int*>(t + tiles));
-    };
-    if (0.5 * P * P * npw >= kHalfMinMacs) {
-        pack(half2x::pack_a, kp.beta_hs_overlap, half2x::packed_a_bytes(P, npw), half2x::packed_a_exps(P),
-             kp.beta32.as<float2>(), P, npw, true);
-        pack(half2x::pack_a, kp.beta_hs_accum, half2x::packed_a_bytes(npw, P), half2x::packed_a_exps(npw),
-             kp.beta32.as<float2>(), npw, P, false);
-        kp.beta_pk_overlap.release();
-        kp.beta_pk_accum.release();
-    } else {
+    const bool half = 0.5 * P * P * npw >= kHalfMinMacs;
+    pk_valid_ = !half;  // the TF32 tiles are this k-point's
+    if (!half) {
         kp.beta_pk_overlap.reserve(this, tc::packed_a_bytes(P, npw));
         kp.beta_pk_accum.reserve(this, tc::packed_a_bytes(npw, P));
         tc::pack_a(stream, P, npw, kp.beta32.as<float2>(), npw, true, kp.beta_pk_overlap.as<unsigned char>());
         tc::pack_a(stream, npw, P, kp.beta32.as<float2>(), npw, false, kp.beta_pk_accum.as<unsigned char>());
     }
-    if (zmod::worth(true, P, P / 2, npw, true)) {
-        pack(zmod::pack_a, kp.beta_zm_overlap, zmod::packed_a_bytes(P, npw), zmod::packed_a_exps(P),
-             kp.beta64.as<double2>(), P, npw, true);
-        pack(zmod::pack_a, kp.beta_zm_accum, zmod::packed_a_bytes(npw, P), zmod::packed_a_exps(npw),
-             kp.beta64.as<double2>(), npw, P, false);
+    const bool residues = zmod::worth(true, P, P / 2, npw, true);
+    // tiles and exponents of the overlap and the accumulation form, one after another
+    auto span = [](size_t tiles, size_t exps) { return (tiles + exps * sizeof(int) + 255) & ~size_t(255); };
+    const size_t ho = half ? span(half2x::packed_a_bytes(P, npw), half2x::packed_a_exps(P)) : 0;
+    const size_t ha = half ? span(half2x::packed_a_bytes(npw, P), half2x::packed_a_exps(npw)) : 0;
+    const size_t zo = residues ? span(zmod::packed_a_bytes(P, npw), zmod::packed_a_exps(P)) : 0;
+    const size_t za = residues ? span(zmod::packed_a_bytes(npw, P), zmod::packed_a_exps(npw)) : 0;
+    if (ho + ha + zo + za == 0 || !kp.beta_packs.try_reserve(this, ho + ha + zo + za)) return;
+    unsigned char* at = kp.beta_packs.as<unsigned char>();
+    auto pack = [&](auto convert, auto& packed, size_t tiles, const auto* beta, int M, int K, bool kmajor, size_t bytes) {
+        int* exps = reinterpret_cast<int*>(at + tiles);
+        convert(stream, M, K, beta, npw, kmajor, at, exps);
+        packed = {at, exps, M, K};
+        at += bytes;
+    };
+    if (half) {
+        pack(half2x::pack_a, kp.hs_overlap, half2x::packed_a_bytes(P, npw), kp.beta32.as<float2>(), P, npw, true, ho);
+        pack(half2x::pack_a, kp.hs_accum, half2x::packed_a_bytes(npw, P), kp.beta32.as<float2>(), npw, P, false, ha);
     }
+    if (residues) {
+        pack(zmod::pack_a, kp.zm_overlap, zmod::packed_a_bytes(P, npw), kp.beta64.as<double2>(), P, npw, true, zo);
+        pack(zmod::pack_a, kp.zm_accum, zmod::packed_a_bytes(npw, P), kp.beta64.as<double2>(), npw, P, false, za);
+    }
+}
+
+void Context::drop_packs() {
+    kp.hs_overlap = kp.hs_accum = half2x::PackedA{};
+    kp.zm_overlap = kp.zm_accum = zmod::PackedA{};
 }
 
 template <> const LocalPlan<double>& Context::local_plan<double>() const { return kp.lp64; }
@@ -675,28 +685,19 @@ template <> const LocalPlan<float>& Context::local_plan<float>() const { return 
 template <> NonlocalData<double> Context::nonlocal<double>() const {
     NonlocalData<double> d{kp.nproj, kp.beta64.as<double2>(), kp.pstart.as<int>(),
                            kp.psize.as<int>(), kp.poff.as<int>(), kp.dpk64.as<double>()};
-    auto packed = [](const DevBuf& b, int M, int K) {
-        if (!b.ptr) return zmod::PackedA{};
-        const unsigned char* t = b.as<unsigned char>();
-        return zmod::PackedA{t, reinterpret_cast<const int*>(t + zmod::packed_a_bytes(M, K)), M, K};
-    };
-    d.zm_overlap = packed(kp.beta_zm_overlap, kp.nproj, kp.npw);
-    d.zm_accum = packed(kp.beta_zm_accum, kp.npw, kp.nproj);
+    d.zm_overlap = kp.zm_overlap;
+    d.zm_accum = kp.zm_accum;
     return d;
 }
 template <> NonlocalData<float> Context::nonlocal<float>() const {
     NonlocalData<float> d{kp.nproj, kp.beta32.as<float2>(), kp.pstart.as<int>(),
                           kp.psize.as<int>(), kp.poff.as<int>(), kp.dpk32.as<float>()};
-    if (kp.beta_pk_overlap.ptr)
+    if (kp.nproj > 0 && pk_valid_) {
         d.beta_overlap = tc::PackedA{kp.beta_pk_overlap.as<unsigned char>(), kp.nproj, kp.npw};
-    if (kp.beta_pk_accum.ptr) d.beta_accum = tc::PackedA{kp.beta_pk_accum.as<unsigned char>(), kp.npw, kp.nproj};
-    auto packed = [](const DevBuf& b, int M, int K) {
-        if (!b.ptr) return half2x::PackedA{};
-        const unsigned char* t = b.as<unsigned char>();
-        return half2x::PackedA{t, reinterpret_cast<const int*>(t + half2x::packed_a_bytes(M, K)), M, K};
-    };
-    d.hs_overlap = packed(kp.beta_hs_overlap, kp.nproj, kp.npw);
-    d.hs_accum = packed(kp.beta_hs_accum, kp.npw, kp.nproj);
+        d.beta_accum = tc::PackedA{kp.beta_pk_accum.as<unsigned char>(), kp.npw, kp.nproj};
+    }
+    d.hs_overlap = kp.hs_overlap;
+    d.hs_accum = kp.hs_accum;
     return d;
 }
 

@@ -52,12 +52,12 @@ struct KPoint {
     DevBuf ke64, ke32;
     DevBuf beta64, beta32;
     DevBuf beta_pk_overlap, beta_pk_accum;  // beta32 as TF32 tensor-core A tiles
-    // or, for large sets, as FP16 tiles, each followed by its rows' exponents
-    // (these, like the next, empty where memory is short)
-    DevBuf beta_hs_overlap, beta_hs_accum;
-    // beta64 as residue tiles for the FP64 products, each followed by its rows'
-    // exponents; empty for small sets and where memory is short
-    DevBuf beta_zm_overlap, beta_zm_accum;
+    // or, for large sets, as FP16 tiles; beta64 as residue tiles for the FP64
+    // products; one buffer for all, kept from one k-point to the next, empty
+    // where memory is short
+    DevBuf beta_packs;
+    half2x::PackedA hs_overlap{}, hs_accum{};  // in beta_packs, or no tiles
+    zmod::PackedA zm_overlap{}, zm_accum{};
     DevBuf pstart, psize, poff, dpk64, dpk32;
     size_t dpk_len = 0;             // packed block entries (D, and Q when set)
     bool has_q = false;             // ultrasoft overlap blocks set for this k-point
@@ -159,7 +159,9 @@ class Context {
     size_t ws_gemm_need_ = 0;     // largest `need` of gemm_ws
     size_t ws_gemm_refused_ = 0;  // smallest `want` the device had no room for (0: none)
     void build_plan();
+    bool pk_valid_ = false;       // kp.beta_pk_* hold the prepared k-point's projectors
     void pack_projectors();
+    void drop_packs();
 };
 
 // convert an exception into a status code and message
