@@ -289,41 +289,43 @@ __global__ void copy_matrix(int n, const double2* src, int lds, double2* dst, in
 inline int grid_for(long n) { return stride_grid(n, 8); }
 
 // ------------------------------------------------------------ exchange between blocks
-// A published complex value is 32 bytes: each of its four 32-bit words beside a
-// word that holds the step it belongs to, so a reader that sees the step in
-// every pair has the value, with no fence and no separate flag to wait for (8-byte
-// halves of a vector access are single copies).  Steps count from 1; the buffers
-// are zeroed before the launch.
+// A published complex value is four 64-bit words: each 32-bit half of a part
+// beside the step it belongs to, so a reader that sees the step in every word
+// has the value, with no fence and no separate flag to wait for.  The accesses
+// are vectors of two 64-bit elements: an element is read or written whole, while
+// nothing is promised about the elements of one access among each other.
+// Steps count from 1; the buffers are zeroed before the launch.
 // the sum of 16 values held twice across a warp, the same in every lane
 __device__ __forceinline__ double sum_over_half_warp(double v) {
 #pragma unroll
     for (int o = 8; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
     return v;
 }
-struct Published {
-    uint4 re, im;  // {low word, step, high word, step}
+struct __align__(16) Published {
+    unsigned long long re_lo, re_hi, im_lo, im_hi;  // (step << 32) | half of a part
 };
-__device__ __forceinline__ void publish(Published* at, double2 v, unsigned step) {
-    const unsigned r0 = __double2loint(v.x), r1 = __double2hiint(v.x), i0 = __double2loint(v.y),
-                   i1 = __double2hiint(v.y);
-    asm volatile("st.volatile.global.v4.u32 [%0], {%1, %2, %3, %2};" ::"l"(&at->re), "r"(r0), "r"(step), "r"(r1)
-                 : "memory");
-    asm volatile("st.volatile.global.v4.u32 [%0], {%1, %2, %3, %2};" ::"l"(&at->im), "r"(i0), "r"(step), "r"(i1)
-                 : "memory");
+__device__ __forceinline__ unsigned long long tagged(int half, unsigned step) {
+    return (static_cast<unsigned long long>(step) << 32) | static_cast<unsigned>(half);
 }
-__device__ __forceinline__ uint4 load_pairs(const uint4* at) {
-    uint4 v;
-    asm volatile("ld.volatile.global.v4.u32 {%0, %1, %2, %3}, [%4];"
-                 : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w)
-                 : "l"(at)
-                 : "memory");
+__device__ __forceinline__ void store_two(unsigned long long* at, unsigned long long a, unsigned long long b) {
+    asm volatile("st.volatile.global.v2.b64 [%0], {%1, %2};" ::"l"(at), "l"(a), "l"(b) : "memory");
+}
+__device__ __forceinline__ void publish(Published* at, double2 v, unsigned step) {
+    store_two(&at->re_lo, tagged(__double2loint(v.x), step), tagged(__double2hiint(v.x), step));
+    store_two(&at->im_lo, tagged(__double2loint(v.y), step), tagged(__double2hiint(v.y), step));
+}
+__device__ __forceinline__ ulonglong2 load_two(const unsigned long long* at) {
+    ulonglong2 v;
+    asm volatile("ld.volatile.global.v2.b64 {%0, %1}, [%2];" : "=l"(v.x), "=l"(v.y) : "l"(at) : "memory");
     return v;
 }
+__device__ __forceinline__ unsigned step_of(unsigned long long w) { return static_cast<unsigned>(w >> 32); }
 // one look: true with the value once it is there
 __device__ __forceinline__ bool look(const Published* at, unsigned step, double2& v) {
-    const uint4 a = load_pairs(&at->re), b = load_pairs(&at->im);
-    v = mk(__hiloint2double(a.z, a.x), __hiloint2double(b.z, b.x));
-    return a.y == step && a.w == step && b.y == step && b.w == step;
+    const ulonglong2 a = load_two(&at->re_lo), b = load_two(&at->im_lo);
+    v = mk(__hiloint2double(static_cast<int>(a.y), static_cast<int>(a.x)),
+           __hiloint2double(static_cast<int>(b.y), static_cast<int>(b.x)));
+    return step_of(a.x) == step && step_of(a.y) == step && step_of(b.x) == step && step_of(b.y) == step;
 }
 // Every wait is bounded (about 2 s of clock), after which the kernel records an
 // error and all blocks leave.
