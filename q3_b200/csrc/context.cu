@@ -621,8 +621,10 @@ void Context::prepare_kpoint(int npw, const int32_t* g2g, const double* ke, cons
         upload(this, kp.dpk32, d32.data(), d32.size());
         kp.dpk_len = d64.size();
     }
-    build_plan();
+    // packed first: the plan's host work hides the packing, and the wait at its end
+    // covers it, so that the caller may go on on another stream
     pack_projectors();
+    build_plan();
     kp.valid = true;
 }
 
