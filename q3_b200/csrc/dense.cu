@@ -367,6 +367,10 @@ struct Patience {
 // reads, which cost a fence, an atomic and a second L2 read, and W after it.
 constexpr int kHetrdThreads = 512;
 constexpr int kHetrdEntries = 3;  // of a vector a thread holds: orders up to 1536
+// |x|^2 between these is formed from x as it is: x_0 has a share in |x| only where
+// |x_0|^2 > 1e-282, and no square, sum of squares or product of two of them
+// leaves the range
+constexpr double kSquaresLow = 1e-250, kSquaresHigh = 1e250;
 __global__ void __launch_bounds__(kHetrdThreads, 1)
 hetrd_smem(int n, int cpb, int w_in_smem, const double2* A, double* d, double2* e, double2* W,
            Published* xpre2, Published* pbuf2, unsigned* seen, int* err) {
@@ -420,18 +424,48 @@ hetrd_smem(int n, int cpb, int w_in_smem, const double2* A, double* d, double2* 
         __syncthreads();
         // the reflector, by every thread: v = x - alpha e_0 with alpha = -|x| x_0 / |x_0|,
         // tau = 2 / |v|^2 = 1 / (|x|^2 + |x| |x_0|)
-        const double sigma = sum_over_half_warp(red[lane & (WARPS - 1)]);
-        const double2 x0 = sx[k + 1];
+        double sigma = sum_over_half_warp(red[lane & (WARPS - 1)]);
+        double2 x0 = sx[k + 1];
+        double a2 = x0.x * x0.x + x0.y * x0.y, unit = 1.0;
+        if (m > 1 && (sigma + a2 < kSquaresLow || sigma + a2 > kSquaresHigh)) {
+            // squares near the ends of the range (every block comes to the same): the
+            // same reflector from x over a power of two near its largest part
+            double mx = 0.0;
+            for (int j = tid; j < m; j += kHetrdThreads) {
+                const double2 x = sx[k + 1 + j];
+                mx = fmax(mx, fmax(fabs(x.x), fabs(x.y)));
+            }
+            for (int o = 16; o > 0; o >>= 1) mx = fmax(mx, __shfl_xor_sync(0xffffffffu, mx, o));
+            if (lane == 0) redp[warp] = mx;
+            __syncthreads();  // and `red` has been read
+            for (int q = 0; q < WARPS; ++q) mx = fmax(mx, redp[q]);
+            const int ex = mx > 0.0 && mx < INFINITY ? max(-1000, min(1000, ilogb(mx))) : 0;
+            const double by = __hiloint2double((1023 - ex) << 20, 0);
+            unit = __hiloint2double((1023 + ex) << 20, 0);
+            part = 0.0;
+            for (int j = tid; j < m; j += kHetrdThreads) {
+                const double2 x = by * sx[k + 1 + j];
+                sv[j] = x;
+                if (j > 0) part += x.x * x.x + x.y * x.y;
+            }
+            part = warp_sum(part);
+            if (lane == 0) red[warp] = part;
+            __syncthreads();
+            sigma = sum_over_half_warp(red[lane & (WARPS - 1)]);
+            x0 = by * x0;
+            a2 = x0.x * x0.x + x0.y * x0.y;
+        }
         double tk = 0.0;
         double2 alpha = x0;
         if (m > 1 && sigma > 0.0) {
-            const double a2 = x0.x * x0.x + x0.y * x0.y, n2 = sigma + a2, nrm = n2 * rsqrt(n2);
-            // (below 1e-290 the square is no longer accurate, and x_0 counts for nothing)
+            const double n2 = sigma + a2, nrm = n2 * rsqrt(n2);
+            // where the square of |x_0| is no longer accurate, it counts for nothing beside |x|
             const double ra = a2 > 1e-290 ? rsqrt(a2) : 0.0, ax0 = a2 * ra;
             alpha = ra > 0.0 ? mk(-nrm * (x0.x * ra), -nrm * (x0.y * ra)) : mk(-nrm, 0.0);
             tk = 1.0 / fma(nrm, ax0, n2);
             if (tid == 0) sv[0] = x0 - alpha;
         }
+        alpha = unit * alpha;
         if (b == 0 && tid == 0) {
             d[k] = sx[k].x;
             e[k] = alpha;

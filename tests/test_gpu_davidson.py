@@ -83,6 +83,33 @@ def test_hegv_degenerate(cuda_device, ctx_app):
     assert np.max(np.abs(z.conj().T @ z - np.eye(n))) < 1e-11
 
 
+@pytest.mark.parametrize("scale", [1e-153, 1e-150, 1e-146, 1e-143, 1e-125, 1e125, 1e148])
+@pytest.mark.parametrize("n", [97, 130])
+def test_hegv_columns_whose_squares_leave_the_range(cuda_device, ctx_app, n, scale):
+    """One plane wave coupled to the others by entries whose squares are denormal, zero or
+    infinite: the reflector of that column has to stay unitary.  Compared with the problem in which
+    the coupling is exactly zero (small scales: it moves an eigenvalue by scale^2 at most) or, for
+    the large scales, in which all entries are divided by the scale."""
+    from q3_b200.davidson import hegv
+    rng = np.random.default_rng(n)
+    x = rng.standard_normal((n, n)) + 1j * rng.standard_normal((n, n))
+    h = (x + x.conj().T) / 2
+    if scale < 1.0:
+        h[0, 1:] *= scale
+        h[1:, 0] *= scale
+        ref = h.copy()
+        ref[0, 1:] = ref[1:, 0] = 0.0
+        unit = 1.0
+    else:
+        h = h * scale
+        ref, unit = h / scale, scale
+    w, z = hegv(ctx_app, h, np.eye(n))
+    we = np.linalg.eigvalsh(ref)
+    assert np.max(np.abs(z.conj().T @ z - np.eye(n))) < 1e-11
+    assert np.max(np.abs(w / unit - we)) < 1e-12 * np.max(np.abs(we)) * n / 16
+    assert np.max(np.abs(ref @ z - z * (w / unit)[None, :])) < 1e-11 * n / 16
+
+
 def test_hegv_not_positive_definite(cuda_device, ctx_app):
     from q3_b200.davidson import hegv
     with pytest.raises(Q3BError):
