@@ -122,7 +122,9 @@ template <int BC> struct Cols {
                                       (static_cast<uint32_t>((2 * BM) >> 4) << 24);
 };
 constexpr int kMaxK = 16384;          // of one partial sum: 2 * 255^2 * 16384 < 2^31
-constexpr int kMaxSplits = 64;
+constexpr int kMaxSplits = 64;        // K ranges taken for the sake of a better share of work
+constexpr int kMaxRanges = 257;       // K ranges at all: their bytes are added up in 16 bits
+static_assert(255 * kMaxRanges <= 0xffff, "zmod_combine adds the ranges' bytes in 16 bits");
 
 // --------------------------------------------------------- row scales
 // exponent s with |row| 2^s <= 2^c from the row's sum of squares and largest
@@ -751,7 +753,7 @@ void pack_a(cudaStream_t st, int M, int K, const double2* A, long lda, bool kmaj
 // (the projectors), beta Q beta^H psi of 90 bands of the 64-atom cell takes 0.39 ms
 // against 1.14.
 bool worth(bool conj_a, int M, int N, int K, bool packed) {
-    if (M < 64 || N < 16 || K < 64) return false;
+    if (M < 64 || N < 16 || K < 64 || K > kMaxRanges * kMaxK) return false;
     const double tiles = (double)ceil_div(M, 2 * BM) * (narrow(N) ? 2 : 4 * ceil_div(N, 128)) * ceil_div(K, BK);
     const double entries = (double)K * N + (packed ? 0.0 : (double)M * K);
     const double here = 40e-6 + 19e-12 * entries + 60e-9 * tiles + 10e-12 * (double)M * N;

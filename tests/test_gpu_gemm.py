@@ -83,3 +83,13 @@ def test_gemm_rejects_unsupported(ctx):
     rc = lib.q3b_gemm(h, b"T", b"N", 4, 4, 4, Cplx128(1, 0), None, 4, None, 4, Cplx128(0, 0), None, 4)
     with pytest.raises(Q3BError):
         check(h, rc)
+
+
+def test_residue_products_end_where_their_byte_sums_do(ctx):
+    """257 K ranges of 16384 are the most whose bytes add up in 16 bits."""
+    worth = ctx.lib["_ZN3q3b4zmod5worthEbiiib"]  # bool q3b::zmod::worth(bool, int, int, int, bool)
+    worth.restype, worth.argtypes = C.c_bool, [C.c_bool, C.c_int, C.c_int, C.c_int, C.c_bool]
+    for packed in (False, True):
+        assert worth(True, 2048, 1024, 257 * 16384, packed)
+        assert not worth(True, 2048, 1024, 257 * 16384 + 1, packed)
+        assert not worth(False, 2048, 1024, 257 * 16384 + 1, packed)
