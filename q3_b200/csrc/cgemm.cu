@@ -352,11 +352,13 @@ inline double busiest(long blocks, int k, int start, int bm, int bn, double rate
 }
 
 // The tile and the K ranges of a product on the pipelined tiles.
-//   tile: 64 x 64 or 32 x 32, whichever takes fewer clocks; 32 x 16 where 32
-//     columns would leave a quarter or more of them empty;
+//   tile: 64 x 64 or 32 x 32, whichever takes fewer clocks (64 x 64 where a grid has
+//     no room for the tiles of 32 rows); 32 x 16 where 32 columns would leave a
+//     quarter or more of them empty;
 //   ranges (C,N only): the count with the least clocks, each costing two steps of K
 //     for its share of the sum.  At most 64, of at least 32 steps, and as many tiles
 //     as there are counters.
+constexpr int kMaxGridRows = 65535;
 struct PipePlan {
     int tm, tn, splits, kchunk;
     size_t part;   // complex values of the partial sums
@@ -379,7 +381,7 @@ PipePlan pipe_plan(bool conj_a, int M, int N, int K) {
             }
         }
     };
-    consider(2, ceil_div(N, 16) * 16 * 4 <= ceil_div(N, 32) * 32 * 3 ? 1 : 2);
+    if (ceil_div(M, 32) <= kMaxGridRows) consider(2, ceil_div(N, 16) * 16 * 4 <= ceil_div(N, 32) * 32 * 3 ? 1 : 2);
     consider(4, 4);
     return best;
 }
@@ -554,7 +556,7 @@ void cgemm(cudaStream_t st, bool conj_a, int M, int N, int K, cplx_t<R> alpha, c
         p.splits = 1;
         p.kchunk = K;
     }
-    if (ceil_div(M, 16 * p.tm) > 65535) throw std::runtime_error("complex GEMM: M too large");
+    if (ceil_div(M, 16 * p.tm) > kMaxGridRows) throw std::runtime_error("complex GEMM: M too large");
     const dim3 grid(ceil_div(N, 16 * p.tn), ceil_div(M, 16 * p.tm), p.splits);
     T* part = p.splits > 1 ? static_cast<T*>(ws.ptr) : nullptr;
     auto run = [&](auto conj) {

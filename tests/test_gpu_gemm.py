@@ -85,6 +85,24 @@ def test_gemm_rejects_unsupported(ctx):
         check(h, rc)
 
 
+def test_gemm_long_operands(ctx):
+    """What the FP64 units took stays accepted: more rows than a grid of 32-row tiles has."""
+    import torch
+    m, n, k = 2_097_153, 8, 8
+    g = torch.Generator(device="cuda")
+    g.manual_seed(1)
+    a, b = (torch.randn(k, r, dtype=torch.complex128, device="cuda", generator=g) for r in (m, n))
+    b = b.T.contiguous()  # column-major k x n
+    c = torch.empty(n, m, dtype=torch.complex128, device="cuda")
+    torch.cuda.synchronize()
+    check(ctx.handle, ctx.lib.q3b_gemm(ctx.handle, b"N", b"N", m, n, k, Cplx128(1, 0), a.data_ptr(), m,
+                                       b.data_ptr(), k, Cplx128(0, 0), c.data_ptr(), m))
+    ctx.synchronize()
+    # 8 k rounded FMAs a part
+    err = float(((c - b @ a).abs() / (b.abs() @ a.abs())).max())
+    assert err < 32 * k * 2.0 ** -53, err
+
+
 def test_residue_products_end_where_their_byte_sums_do(ctx):
     """257 K ranges of 16384 are the most whose bytes add up in 16 bits."""
     worth = ctx.lib["_ZN3q3b4zmod5worthEbiiib"]  # bool q3b::zmod::worth(bool, int, int, int, bool)
