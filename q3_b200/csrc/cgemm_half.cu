@@ -41,6 +41,7 @@ using namespace umma;
 
 constexpr int BM = 128;              // complex rows a CTA holds of a pair's 256
 constexpr int BK = 64;               // K per stage: one 128-byte row of FP16
+static_assert(kLongestK == 65535 * BK, "a grid row per stage");
 constexpr int ROW = 128;             // bytes
 constexpr int A_TILE = 4 * BM * ROW;  // re hi, re lo, im hi, im lo
 constexpr int STAGES = 2;
@@ -465,7 +466,7 @@ void set_limits() {
 template <bool KMAJOR, int ROWS, int AS>
 void pack_operand(cudaStream_t st, int R, int K, const float2* X, long ld, unsigned char* tiles, int* exps) {
     const int padded = ceil_div(R, 2 * ROWS) * 2 * ROWS, nkb = ceil_div(K, BK);
-    if (nkb > 65535) throw std::runtime_error("tensor-core GEMM: operand too large to pack");
+    if (K > kLongestK) throw std::runtime_error("tensor-core GEMM: operand too large to pack");
     if (KMAJOR) launch_chained(exps_kmajor, padded, 256, 0, st, R, K, X, ld, exps);
     else launch_chained(exps_mmajor, padded / 32, 256, 0, st, R, K, X, ld, exps);
     Q3B_LAUNCH_CHECK();

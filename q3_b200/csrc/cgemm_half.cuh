@@ -14,6 +14,7 @@ struct PackedA {
     const int* exps = nullptr;  // power of two each row was scaled by
     int M = 0, K = 0;
 };
+constexpr int kLongestK = 65535 * 64;  // of a packed operand: one grid row per 64 of K
 size_t packed_a_bytes(int M, int K);
 size_t packed_a_exps(int M);  // ints
 // kmajor: element (m, k) at A[m * lda + k] (the "C,N" operand); else at A[m + k * lda]

@@ -643,7 +643,7 @@ void Context::pack_projectors() {
     drop_packs();
     const int P = kp.nproj, npw = kp.npw;
     if (P <= 0) return;
-    const bool half = 0.5 * P * P * npw >= kHalfMinMacs;
+    const bool half = 0.5 * P * P * npw >= kHalfMinMacs && npw <= half2x::kLongestK && P <= half2x::kLongestK;
     pk_valid_ = !half;  // the TF32 tiles are this k-point's
     if (!half) {
         kp.beta_pk_overlap.reserve(this, tc::packed_a_bytes(P, npw));
