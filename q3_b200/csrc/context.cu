@@ -632,10 +632,11 @@ void Context::prepare_kpoint(int npw, const int32_t* g2g, const double* ke, cons
 // them, in both precisions.  FP32: FP16 tiles from kHalfMinMacs complex
 // multiply-adds of a block of usual size (half the projectors, as four bands an
 // atom make), TF32 tiles below.  The FP16 form packs the bands as well (two
-// launches) and works in 256 rows: both products of a block took 204 us against 300
-// at 64 atoms (3.1e9), 155 against 142 at 48 (1.3e9), 77 against 42 at 19 (8e7);
-// with half the 64-atom cell's bands 157 against 167, with a quarter 122 against
-// 122.  FP64: residue tiles where the products of such a block run on them.
+// launches) and works in 256 rows: both products of a block took 198 us against 300
+// at 64 atoms (3.1e9), 155 against 142 at 48 (1.3e9), 77 against 42 at 19 (8e7).
+// Blocks of few bands, as the last iterations of a solve have them, are no slower
+// either: 64 atoms, 64 bands 111 us against 122, 32 bands 108 against 112, 8 bands 100
+// against 103; 56 atoms, 32 bands 98 against 101; 97 atoms, 32 bands 172 against 192.  FP64: residue tiles where the products of such a block run on them.
 // Without room for FP16 or residue tiles the products take the projectors as they
 // are.
 constexpr double kHalfMinMacs = 2e9;
