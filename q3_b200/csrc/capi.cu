@@ -353,8 +353,7 @@ int q3b_hegv_lowest(q3b_context* ctx, int n, const q3b_cplx128* h, const q3b_cpl
         if (n == 0) return;
         c.ws_dense.reserve(&c, q3b::dense::hegv_scratch_bytes(n));
         q3b::dense::Scratch ws{c.ws_dense.as<char>(), c.ws_dense.bytes, 0};
-        q3b::GemmWorkspace g = c.gemm_ws(q3b::cgemm_workspace_bytes<double>(n, n, n),
-                                         q3b::cgemm_wanted_bytes<double>(true, n, n, n));
+        const q3b::GemmWorkspace g = q3b::dense::hegv_workspace(c, n, nvec);
         const int info = q3b::dense::hegv(c.stream, n, reinterpret_cast<const double2*>(h),
                                           reinterpret_cast<const double2*>(s), ld, w,
                                           reinterpret_cast<double2*>(evec), nvec, ws, g, &c.hegv_graphs);
@@ -417,8 +416,7 @@ int q3b_hegv(q3b_context* ctx, int n, const q3b_cplx128* h, const q3b_cplx128* s
         if (n == 0) return;
         c.ws_dense.reserve(&c, q3b::dense::hegv_scratch_bytes(n));
         q3b::dense::Scratch ws{c.ws_dense.as<char>(), c.ws_dense.bytes, 0};
-        q3b::GemmWorkspace g = c.gemm_ws(q3b::cgemm_workspace_bytes<double>(n, n, n),
-                                         q3b::cgemm_wanted_bytes<double>(true, n, n, n));
+        const q3b::GemmWorkspace g = q3b::dense::hegv_workspace(c, n, n);
         const int info = q3b::dense::hegv(c.stream, n, reinterpret_cast<const double2*>(h),
                                           reinterpret_cast<const double2*>(s), ld, w,
                                           reinterpret_cast<double2*>(evec), n, ws, g, &c.hegv_graphs);

@@ -539,7 +539,7 @@ void cgemm(cudaStream_t st, bool conj_a, int M, int N, int K, cplx_t<R> alpha, c
         return;
     }
     if constexpr (std::is_same<R, double>::value) {
-        if (zmod::worth(conj_a, M, N, K, false) && ws.ptr &&
+        if (ws.wanted && zmod::worth(conj_a, M, N, K, false) &&
             ws.bytes >= zmod::workspace_bytes(conj_a, M, N, K, false) && reinterpret_cast<uintptr_t>(A) % 16 == 0 &&
             reinterpret_cast<uintptr_t>(B) % 16 == 0) {
             zmod::zgemm(st, conj_a, M, N, K, alpha, A, lda, nullptr, B, ldb, beta, C, ldc, ws);
@@ -592,14 +592,14 @@ void cgemm_two(cudaStream_t st, int M, int N, int K, const cplx_t<R>* A, long ld
     const cplx_t<R> one = mk(R(1), R(0)), zero = mk(R(0), R(0));
     if constexpr (std::is_same<R, double>::value) {
         const size_t want = cgemm_two_wanted_bytes<R>(M, N, K);
-        if (want && ws.ptr && ws.bytes >= want && reinterpret_cast<uintptr_t>(A) % 16 == 0 &&
+        if (want && ws.wanted && ws.bytes >= want && reinterpret_cast<uintptr_t>(A) % 16 == 0 &&
             reinterpret_cast<uintptr_t>(B1) % 16 == 0 && reinterpret_cast<uintptr_t>(B2) % 16 == 0) {
             unsigned char* tiles = static_cast<unsigned char*>(ws.ptr);
             int* exps = reinterpret_cast<int*>(tiles + zmod::packed_a_bytes(M, K));
             zmod::pack_a(st, M, K, A, lda, true, tiles, exps);
             const zmod::PackedA pk{tiles, exps, M, K};
             const size_t used = packed_once_bytes(M, K);
-            const GemmWorkspace rest{tiles + used, ws.bytes - used, ws.counters};
+            const GemmWorkspace rest{tiles + used, ws.bytes - used, ws.counters, true};
             zmod::zgemm(st, true, M, N, K, one, nullptr, 0, &pk, B1, ldb, zero, C1, ldc, rest);
             zmod::zgemm(st, true, M, N, K, one, nullptr, 0, &pk, B2, ldb, zero, C2, ldc, rest);
             return;

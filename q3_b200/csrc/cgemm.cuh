@@ -15,6 +15,9 @@
 
 namespace q3b {
 
+// A product's workspace: the bytes that were asked for with it, not those of the
+// buffer behind it, so that the kernels a product takes and the order of its sums
+// follow from its own shape and not from what the context has run before.
 struct GemmWorkspace {
     void* ptr = nullptr;
     size_t bytes = 0;
@@ -22,6 +25,9 @@ struct GemmWorkspace {
     // and leaves zeroed (none: products run unsplit)
     static constexpr int kCounters = 1024;
     unsigned* counters = nullptr;
+    // the bytes wanted for the faster kernels (cgemm_wanted_bytes and the like) were
+    // asked for and are there
+    bool wanted = false;
 };
 
 template <typename R>

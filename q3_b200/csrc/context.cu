@@ -184,7 +184,8 @@ GemmWorkspace Context::gemm_ws(size_t need, size_t want) {
         if (!ws_gemm.try_reserve(this, want) && in_budget) ws_gemm_refused_ = want;
     }
     ws_gemm.reserve(this, need);
-    return GemmWorkspace{ws_gemm.ptr, ws_gemm.bytes, gemm_counters.as<unsigned>()};
+    const bool wanted = want > 0 && ws_gemm.bytes >= want;
+    return GemmWorkspace{ws_gemm.ptr, wanted ? std::max(need, want) : need, gemm_counters.as<unsigned>(), wanted};
 }
 
 bool Context::release_optional() {

@@ -387,9 +387,9 @@ template <typename R> class Davidson {
         const T* Sn = SV_ + (size_t)start * npw_;
         if constexpr (std::is_same<R, double>::value) {
             double2 *h = Hs_ + (size_t)start * maxn_, *s = Ss_ + (size_t)start * maxn_;
-            GemmWorkspace ws = c_.gemm_ws(cgemm_workspace_bytes<R>(total, nnew, npw_),
-                                          std::max(cgemm_two_wanted_bytes<R>(total, nnew, npw_),
-                                                   cgemm_wanted_bytes<R>(true, total, nnew, npw_)));
+            const size_t need = cgemm_workspace_bytes<R>(total, nnew, npw_);
+            GemmWorkspace ws = c_.gemm_ws(need, cgemm_two_wanted_bytes<R>(total, nnew, npw_));
+            if (!ws.wanted) ws = c_.gemm_ws(need, cgemm_wanted_bytes<R>(true, total, nnew, npw_));
             cgemm_two<R>(st_, total, nnew, npw_, V_, npw_, Hn, Sn, npw_, h, s, maxn_, ws);
             gamma_fix(total, nnew, V_, Hn, h, maxn_);
             gamma_fix(total, nnew, V_, Sn, s, maxn_);
@@ -419,7 +419,7 @@ template <typename R> class Davidson {
             if (st == 0 && publish) whost_.assign(wread_.begin(), wread_.begin() + nvec);
             return st;
         }
-        GemmWorkspace gws = c_.gemm_ws(cgemm_workspace_bytes<double>(n, n, n), cgemm_wanted_bytes<double>(true, n, n, n));
+        const GemmWorkspace gws = dense::hegv_workspace(c_, n, nvec);
         // the lowest nvec eigenvalues come back in the solve's own status read
         wread_.assign(n, 0.0);
         const int info = dense::hegv(st_, n, H, S, ld, w_, evec_, nvec, dscratch_, gws, &c_.hegv_graphs,

@@ -1208,6 +1208,16 @@ std::atomic<int> g_block_max_order{kBlockOrderDefault};
 void set_block_max_order(int n) { g_block_max_order.store(n < 0 ? 0 : n); }
 int block_max_order() { return g_block_max_order.load(); }
 
+GemmWorkspace hegv_workspace(Context& c, int n, int nvec) {
+    const int nv = nvec > 0 ? nvec : n;
+    // H U^-1 and U^-H (H U^-1) (n x n x n), W^H (D Y) and U^-1 Z (n x nvec x n)
+    const size_t need = std::max(cgemm_workspace_bytes<double>(n, n, n), cgemm_workspace_bytes<double>(n, nv, n));
+    const size_t want = std::max(
+        std::max(cgemm_wanted_bytes<double>(true, n, n, n), cgemm_wanted_bytes<double>(false, n, n, n)),
+        std::max(cgemm_wanted_bytes<double>(true, n, nv, n), cgemm_wanted_bytes<double>(false, n, nv, n)));
+    return c.gemm_ws(need, want);
+}
+
 int hegv(cudaStream_t st, int n, const double2* H, const double2* S, int ld, double* w, double2* Z,
          int nvec, Scratch& ws, const GemmWorkspace& gws, HegvGraphs* graphs, double* w_host) {
     if (n <= 0) return 0;

@@ -116,6 +116,10 @@ template <typename F> cudaGraphExec_t HegvGraphs::get(const Key& k, F&& issue) {
     return e;
 }
 
+// the context's GEMM workspace with the bytes of all products hegv issues for
+// order n and nvec vectors (0: as n)
+GemmWorkspace hegv_workspace(Context& c, int n, int nvec);
+
 // Generalized Hermitian eigenproblem H c = w S c (itype 1; upper triangles of
 // H and S, ld ld).  The lowest nvec eigenvalues ascending in w (device; all n
 // when nvec is 0), their S-orthonormal eigenvectors in Z (n x nvec, ld n).  Returns 0, or n + j

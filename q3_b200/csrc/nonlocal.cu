@@ -68,7 +68,7 @@ template <typename R> size_t nonlocal_wanted_bytes(const NonlocalData<R>& nl, in
 // whether an FP32 projector product runs on the FP16 tiles (beta^H psi
 // with `overlap`, else beta B')
 static bool on_half_tiles(const NonlocalData<float>& nl, bool overlap, int npw, int nvec, const GemmWorkspace& ws) {
-    if (!use_tensor_cores(nl.nproj, nvec, npw) || !ws.ptr) return false;
+    if (!use_tensor_cores(nl.nproj, nvec, npw) || !ws.wanted) return false;
     return overlap ? nl.hs_overlap.tiles && ws.bytes >= half2x::workspace_bytes(true, nl.nproj, nvec, npw)
                    : nl.hs_accum.tiles && ws.bytes >= half2x::workspace_bytes(false, npw, nvec, nl.nproj);
 }
@@ -88,7 +88,7 @@ void apply_nonlocal(cudaStream_t st, const NonlocalData<R>& nl, int npw, int nve
             tc::cgemm_packed(st, true, nl.nproj, nvec, npw, one, nl.beta_overlap, psi, ldpsi, zero, Bm, nl.nproj, ws);
         else
             cgemm<R>(st, true, nl.nproj, nvec, npw, one, nl.beta, npw, psi, ldpsi, zero, Bm, nl.nproj, ws);
-    } else if (nl.zm_overlap.tiles && zmod::worth(true, nl.nproj, nvec, npw, true) && ws.ptr &&
+    } else if (nl.zm_overlap.tiles && zmod::worth(true, nl.nproj, nvec, npw, true) && ws.wanted &&
                ws.bytes >= zmod::workspace_bytes(true, nl.nproj, nvec, npw, true) &&
                reinterpret_cast<uintptr_t>(psi) % 16 == 0) {
         zmod::zgemm(st, true, nl.nproj, nvec, npw, one, nullptr, 0, &nl.zm_overlap, psi, ldpsi, zero, Bm, nl.nproj, ws);
@@ -108,7 +108,7 @@ void apply_nonlocal(cudaStream_t st, const NonlocalData<R>& nl, int npw, int nve
             tc::cgemm_packed(st, false, npw, nvec, nl.nproj, one, nl.beta_accum, Bp, nl.nproj, one, hpsi, ldh, ws);
         else
             cgemm<R>(st, false, npw, nvec, nl.nproj, one, nl.beta, npw, Bp, nl.nproj, one, hpsi, ldh, ws);
-    } else if (nl.zm_accum.tiles && zmod::worth(false, npw, nvec, nl.nproj, true) && ws.ptr &&
+    } else if (nl.zm_accum.tiles && zmod::worth(false, npw, nvec, nl.nproj, true) && ws.wanted &&
                ws.bytes >= zmod::workspace_bytes(false, npw, nvec, nl.nproj, true)) {
         zmod::zgemm(st, false, npw, nvec, nl.nproj, one, nullptr, 0, &nl.zm_accum, Bp, nl.nproj, one, hpsi, ldh, ws);
     } else {

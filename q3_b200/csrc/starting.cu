@@ -119,8 +119,7 @@ int q3b_starting_subspace(q3b_context* ctx, const q3b_cplx128* chi_host, int nch
         start_project_dev(c, H, S);
         c.ws_dense.reserve(&c, q3b::dense::hegv_scratch_bytes(n));
         q3b::dense::Scratch ws{c.ws_dense.as<char>(), c.ws_dense.bytes, 0};
-        q3b::GemmWorkspace g = c.gemm_ws(q3b::cgemm_workspace_bytes<double>(n, n, n),
-                                         q3b::cgemm_wanted_bytes<double>(true, n, n, n));
+        const q3b::GemmWorkspace g = q3b::dense::hegv_workspace(c, n, nb);
         const int info = q3b::dense::hegv(c.stream, n, H, S, n, w, Z, nb, ws, g, &c.hegv_graphs);
         if (info != 0)
             throw q3b::Status(Q3B_ERR_LINALG, "overlap of the starting vectors is not positive definite (info " +

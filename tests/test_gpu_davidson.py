@@ -110,6 +110,30 @@ def test_hegv_columns_whose_squares_leave_the_range(cuda_device, ctx_app, n, sca
     assert np.max(np.abs(ref @ z - z * (w / unit)[None, :])) < 1e-11 * n / 16
 
 
+@pytest.mark.parametrize("n,nvec", [(320, 160), (384, 192), (440, 220)])
+def test_hegv_does_not_depend_on_what_the_context_ran_before(cuda_device, n, nvec):
+    """The products' kernels, and with them the last bits, follow from the problem alone: the same
+    bytes from a fresh context and from one whose workspace a larger product has grown."""
+    import torch
+    from q3_b200._lib import Cplx128, check
+    from q3_b200.applicator import PlanewaveHamiltonianApplicator
+    from q3_b200.davidson import hegv_lowest
+    rng = np.random.default_rng(n)
+    x, y = (rng.standard_normal((n, n)) + 1j * rng.standard_normal((n, n)) for _ in range(2))
+    h, s = (x + x.conj().T) / 2, np.eye(n) + 1e-2 * (y @ y.conj().T) / n
+    ap = PlanewaveHamiltonianApplicator()
+    fresh = hegv_lowest(ap, h, s, nvec)
+    m, k = 512, 24000
+    a = torch.randn(m, k, dtype=torch.complex128, device="cuda")
+    c = torch.empty(m, m, dtype=torch.complex128, device="cuda")
+    torch.cuda.synchronize()
+    check(ap.h, ap.lib.q3b_gemm(ap.h, b"C", b"N", m, m, k, Cplx128(1, 0), a.data_ptr(), k, a.data_ptr(), k,
+                                Cplx128(0, 0), c.data_ptr(), m))
+    ap.ctx.synchronize()
+    later = hegv_lowest(ap, h, s, nvec)
+    assert np.array_equal(fresh[0], later[0]) and np.array_equal(fresh[1], later[1])
+
+
 def test_hegv_not_positive_definite(cuda_device, ctx_app):
     from q3_b200.davidson import hegv
     with pytest.raises(Q3BError):
