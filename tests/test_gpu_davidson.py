@@ -134,6 +134,21 @@ def test_hegv_does_not_depend_on_what_the_context_ran_before(cuda_device, n, nve
     assert np.array_equal(fresh[0], later[0]) and np.array_equal(fresh[1], later[1])
 
 
+@pytest.mark.parametrize("n", [130, 640])
+def test_hegv_with_basis_vectors_of_unequal_norms(cuda_device, ctx_app, n):
+    """A basis scaled by powers of two, D H D and D S D: Cholesky factor, its inverse and the
+    reduced matrix are those of H and S up to exact scalings, so the eigenvalues are too."""
+    from q3_b200.davidson import hegv
+    rng = np.random.default_rng(n)
+    x, y = (rng.standard_normal((n, n)) + 1j * rng.standard_normal((n, n)) for _ in range(2))
+    h, s = (x + x.conj().T) / 2, np.eye(n) + 1e-2 * (y @ y.conj().T) / n
+    d = 2.0 ** rng.integers(-20, 21, n)
+    w0, z0 = hegv(ctx_app, h, s)
+    w, z = hegv(ctx_app, d[:, None] * h * d[None, :], d[:, None] * s * d[None, :])
+    assert np.array_equal(w, w0)
+    assert np.array_equal(d[:, None] * z, z0)
+
+
 def test_hegv_not_positive_definite(cuda_device, ctx_app):
     from q3_b200.davidson import hegv
     with pytest.raises(Q3BError):
