@@ -424,12 +424,23 @@ hetrd_smem(int n, int cpb, int w_in_smem, const double2* A, double* d, double2* 
         __syncthreads();
         // the reflector, by every thread: v = x - alpha e_0 with alpha = -|x| x_0 / |x_0|,
         // tau = 2 / |v|^2 = 1 / (|x|^2 + |x| |x_0|)
-        double sigma = sum_over_half_warp(red[lane & (WARPS - 1)]);
-        double2 x0 = sx[k + 1];
-        double a2 = x0.x * x0.x + x0.y * x0.y, unit = 1.0;
-        if (m > 1 && (sigma + a2 < kSquaresLow || sigma + a2 > kSquaresHigh)) {
+        double2 x0 = sx[k + 1], alpha = x0;
+        double tk = 0.0, n2 = 0.0;
+        auto reflector = [&](double sigma) {
+            const double a2 = x0.x * x0.x + x0.y * x0.y;
+            n2 = sigma + a2;
+            if (m > 1 && sigma > 0.0) {
+                const double nrm = n2 * rsqrt(n2);
+                // where the square of |x_0| is no longer accurate, it counts for nothing beside |x|
+                const double ra = a2 > 1e-290 ? rsqrt(a2) : 0.0, ax0 = a2 * ra;
+                alpha = ra > 0.0 ? mk(-nrm * (x0.x * ra), -nrm * (x0.y * ra)) : mk(-nrm, 0.0);
+                tk = 1.0 / fma(nrm, ax0, n2);
+            }
+        };
+        reflector(sum_over_half_warp(red[lane & (WARPS - 1)]));
+        if (m > 1 && (n2 < kSquaresLow || n2 > kSquaresHigh)) {
             // squares near the ends of the range (every block comes to the same): the
-            // same reflector from x over a power of two near its largest part
+            // reflector of x over a power of two near its largest part instead
             double mx = 0.0;
             for (int j = tid; j < m; j += kHetrdThreads) {
                 const double2 x = sx[k + 1 + j];
@@ -441,7 +452,6 @@ hetrd_smem(int n, int cpb, int w_in_smem, const double2* A, double* d, double2* 
             for (int q = 0; q < WARPS; ++q) mx = fmax(mx, redp[q]);
             const int ex = mx > 0.0 && mx < INFINITY ? max(-1000, min(1000, ilogb(mx))) : 0;
             const double by = __hiloint2double((1023 - ex) << 20, 0);
-            unit = __hiloint2double((1023 + ex) << 20, 0);
             part = 0.0;
             for (int j = tid; j < m; j += kHetrdThreads) {
                 const double2 x = by * sx[k + 1 + j];
@@ -451,21 +461,15 @@ hetrd_smem(int n, int cpb, int w_in_smem, const double2* A, double* d, double2* 
             part = warp_sum(part);
             if (lane == 0) red[warp] = part;
             __syncthreads();
-            sigma = sum_over_half_warp(red[lane & (WARPS - 1)]);
             x0 = by * x0;
-            a2 = x0.x * x0.x + x0.y * x0.y;
+            alpha = x0;
+            tk = 0.0;
+            reflector(sum_over_half_warp(red[lane & (WARPS - 1)]));
+            if (tk != 0.0 && tid == 0) sv[0] = x0 - alpha;
+            alpha = __hiloint2double((1023 + ex) << 20, 0) * alpha;
+        } else if (tk != 0.0 && tid == 0) {
+            sv[0] = x0 - alpha;
         }
-        double tk = 0.0;
-        double2 alpha = x0;
-        if (m > 1 && sigma > 0.0) {
-            const double n2 = sigma + a2, nrm = n2 * rsqrt(n2);
-            // where the square of |x_0| is no longer accurate, it counts for nothing beside |x|
-            const double ra = a2 > 1e-290 ? rsqrt(a2) : 0.0, ax0 = a2 * ra;
-            alpha = ra > 0.0 ? mk(-nrm * (x0.x * ra), -nrm * (x0.y * ra)) : mk(-nrm, 0.0);
-            tk = 1.0 / fma(nrm, ax0, n2);
-            if (tid == 0) sv[0] = x0 - alpha;
-        }
-        alpha = unit * alpha;
         if (b == 0 && tid == 0) {
             d[k] = sx[k].x;
             e[k] = alpha;
@@ -1211,8 +1215,9 @@ int block_max_order() { return g_block_max_order.load(); }
 // The products run on the FP64 units at every order.  The residue products round a
 // row of one operand and a column of the other against their norms, and in H U^-1
 // basis vectors of unequal norms d stand as d in the one and as 1/d in the other:
-// norms over 2^40 cost 1e-6 of the eigenvalues at order 640, where FMAs give the
-// bits of the problem with equal norms.
+// norms over 2^40 cost 5e-8 of the eigenvalues at order 640, where FMAs give the
+// bits of the problem with equal norms.  Order 512 takes 4.32 ms on them against
+// 4.27, 1024 14.3 against 13.4.
 GemmWorkspace hegv_workspace(Context& c, int n, int nvec) {
     const int nv = nvec > 0 ? nvec : n;
     // U^-H (H U^-1) (n x n x n) and W^H (D Y) (n x nvec x n)
