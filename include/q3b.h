@@ -148,13 +148,26 @@ int q3b_apply_h_noalloc(q3b_context* ctx, const q3b_cplx128* psi_dev, q3b_cplx12
  * path uses them: C = alpha op(A) B + beta C, column-major, device pointers,
  * transpose_a 'N' or 'C', transpose_b 'N'.  q3b_gemm runs in FP64 on the CUDA
  * cores; q3b_gemm_single runs on the tensor cores (TF32 split into hi + lo,
- * three products, FP32 accumulation: FP32 accuracy).  Queued on the stream. */
+ * three products, FP32 accumulation: FP32 accuracy).  Queued on the stream.
+ *
+ * q3b_gemm_residue is q3b_gemm on the integer tensor cores, as the large FP64
+ * products inside q3b_apply_h, q3b_apply_s, the Davidson solver and the starting
+ * subspace run: exact integer products of operands rounded against the 2-norms of
+ * the rows of op(A) and the columns of B.  An output is within about
+ * 2e-18 |row| |column| of the exact product, closer than rounded FMAs, unless the
+ * row's large entries meet the column's small ones: entries below 2^-59 of their
+ * row's or column's norm count for nothing.  An infinity or a NaN makes all outputs
+ * of its row or column NaN.  Matrices start on 16 bytes, 0 < k <= 4210688;
+ * Q3B_ERR_MEMORY where its workspace does not fit. */
 int q3b_gemm(q3b_context* ctx, char transpose_a, char transpose_b, int m, int n, int k,
              q3b_cplx128 alpha, const q3b_cplx128* a_dev, int lda, const q3b_cplx128* b_dev, int ldb,
              q3b_cplx128 beta, q3b_cplx128* c_dev, int ldc);
 int q3b_gemm_single(q3b_context* ctx, char transpose_a, char transpose_b, int m, int n, int k,
                     q3b_cplx64 alpha, const q3b_cplx64* a_dev, int lda, const q3b_cplx64* b_dev, int ldb,
                     q3b_cplx64 beta, q3b_cplx64* c_dev, int ldc);
+int q3b_gemm_residue(q3b_context* ctx, char transpose_a, char transpose_b, int m, int n, int k,
+                     q3b_cplx128 alpha, const q3b_cplx128* a_dev, int lda, const q3b_cplx128* b_dev, int ldb,
+                     q3b_cplx128 beta, q3b_cplx128* c_dev, int ldc);
 
 /* ---- diagnostics ---------------------------------------------------------- */
 

@@ -104,6 +104,7 @@ SIGNATURES = {
     "q3b_gemm": (_i, [_vp, C.c_char, C.c_char, _i, _i, _i, Cplx128, _vp, _i, _vp, _i, Cplx128, _vp, _i]),
     "q3b_gemm_single": (_i, [_vp, C.c_char, C.c_char, _i, _i, _i, Cplx64, _vp, _i, _vp, _i, Cplx64, _vp,
                              _i]),
+    "q3b_gemm_residue": (_i, [_vp, C.c_char, C.c_char, _i, _i, _i, Cplx128, _vp, _i, _vp, _i, Cplx128, _vp, _i]),
     "q3b_davidson_default_opts": (None, [C.POINTER(DavidsonOpts)]),
     "q3b_davidson_solve": (_i, [_vp, _vp, _vp, _i, C.POINTER(DavidsonOpts), C.POINTER(DavidsonStats)]),
     "q3b_davidson_solve_dev": (_i, [_vp, _vp, _vp, _i, C.POINTER(DavidsonOpts),

@@ -23,20 +23,30 @@ template <typename F> int guarded(q3b_context* c, F&& f) {
     }
 }
 
-template <typename R, typename CT>
-void gemm_entry(Context& c, char ta, char tb, int m, int n, int k, CT alpha, const CT* a, int lda,
-                       const CT* b, int ldb, CT beta, CT* cc, int ldc) {
-    using T = q3b::cplx_t<R>;
+// true for "C"; throws where a gemm's arguments are not taken
+template <typename CT>
+bool gemm_conj(char ta, char tb, int m, int n, int k, const CT* a, int lda, const CT* b, int ldb, const CT* cc,
+               int ldc) {
     const bool conj = (ta == 'C' || ta == 'c');
     if (!(conj || ta == 'N' || ta == 'n') || !(tb == 'N' || tb == 'n'))
         throw q3b::Status(Q3B_ERR_INVALID, "gemm: transpose_a must be N or C and transpose_b N");
     if (m < 0 || n < 0 || k < 0) throw q3b::Status(Q3B_ERR_INVALID, "gemm: negative size");
-    if (m == 0 || n == 0) return;
+    if (m == 0 || n == 0) return conj;
     if ((k > 0 && (!a || !b)) || !cc) throw q3b::Status(Q3B_ERR_INVALID, "gemm: null matrix");
     if (lda < (conj ? k : m) || ldb < k || ldc < m || lda < 1 || ldb < 1)
         throw q3b::Status(Q3B_ERR_INVALID, "gemm: leading dimension too small");
-    q3b::GemmWorkspace ws = c.gemm_ws(conj ? q3b::cgemm_workspace_bytes<R>(m, n, k) : 0,
-                                      q3b::cgemm_wanted_bytes<R>(conj, m, n, k));
+    return conj;
+}
+
+template <typename R, typename CT>
+void gemm_entry(Context& c, char ta, char tb, int m, int n, int k, CT alpha, const CT* a, int lda,
+                       const CT* b, int ldb, CT beta, CT* cc, int ldc) {
+    using T = q3b::cplx_t<R>;
+    const bool conj = gemm_conj(ta, tb, m, n, k, a, lda, b, ldb, cc, ldc);
+    if (m == 0 || n == 0) return;
+    // no bytes for the residue tiles: a product of any operands keeps each entry's 53
+    // bits (q3b_gemm_residue does not)
+    q3b::GemmWorkspace ws = c.gemm_ws(conj ? q3b::cgemm_workspace_bytes<R>(m, n, k) : 0);
     if constexpr (std::is_same<R, float>::value) {
         // the single-precision entry point always runs on the tensor cores
         // (the library's own products route small ones to the CUDA cores)
@@ -297,6 +307,22 @@ int q3b_gemm(q3b_context* ctx, char ta, char tb, int m, int n, int k, q3b_cplx12
 int q3b_gemm_single(q3b_context* ctx, char ta, char tb, int m, int n, int k, q3b_cplx64 alpha, const q3b_cplx64* a,
                     int lda, const q3b_cplx64* b, int ldb, q3b_cplx64 beta, q3b_cplx64* cc, int ldc) {
     return guarded(ctx, [&](Context& c) { gemm_entry<float>(c, ta, tb, m, n, k, alpha, a, lda, b, ldb, beta, cc, ldc); });
+}
+
+int q3b_gemm_residue(q3b_context* ctx, char ta, char tb, int m, int n, int k, q3b_cplx128 alpha, const q3b_cplx128* a,
+                     int lda, const q3b_cplx128* b, int ldb, q3b_cplx128 beta, q3b_cplx128* cc, int ldc) {
+    return guarded(ctx, [&](Context& c) {
+        const bool conj = gemm_conj(ta, tb, m, n, k, a, lda, b, ldb, cc, ldc);
+        if (m == 0 || n == 0) return;
+        if (k < 1 || k > q3b::zmod::kLongestK) throw q3b::Status(Q3B_ERR_INVALID, "gemm_residue: k out of range");
+        if ((reinterpret_cast<uintptr_t>(a) | reinterpret_cast<uintptr_t>(b) | reinterpret_cast<uintptr_t>(cc)) % 16)
+            throw q3b::Status(Q3B_ERR_INVALID, "gemm_residue: matrices must start on 16 bytes");
+        const q3b::GemmWorkspace ws = c.gemm_ws(0, q3b::zmod::workspace_bytes(conj, m, n, k, false));
+        if (!ws.wanted) throw q3b::Status(Q3B_ERR_MEMORY, "gemm_residue: no room for the workspace");
+        q3b::zmod::zgemm(c.stream, conj, m, n, k, double2{alpha.re, alpha.im}, reinterpret_cast<const double2*>(a), lda,
+                         nullptr, reinterpret_cast<const double2*>(b), ldb, double2{beta.re, beta.im},
+                         reinterpret_cast<double2*>(cc), ldc, ws);
+    });
 }
 
 }  // extern "C"

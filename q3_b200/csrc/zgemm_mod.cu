@@ -124,6 +124,7 @@ template <int BC> struct Cols {
 constexpr int kMaxK = 16384;          // of one partial sum: 2 * 255^2 * 16384 < 2^31
 constexpr int kMaxSplits = 64;        // K ranges taken for the sake of a better share of work
 constexpr int kMaxRanges = 257;       // K ranges at all: their bytes are added up in 16 bits
+static_assert(kLongestK == kMaxRanges * kMaxK, "the longest product");
 static_assert(255 * kMaxRanges <= 0xffff, "zmod_combine adds the ranges' bytes in 16 bits");
 
 // --------------------------------------------------------- row scales
@@ -753,7 +754,7 @@ void pack_a(cudaStream_t st, int M, int K, const double2* A, long lda, bool kmaj
 // (the projectors), beta Q beta^H psi of 90 bands of the 64-atom cell takes 0.39 ms
 // against 1.14.
 bool worth(bool conj_a, int M, int N, int K, bool packed) {
-    if (M < 64 || N < 16 || K < 64 || K > kMaxRanges * kMaxK) return false;
+    if (M < 64 || N < 16 || K < 64 || K > kLongestK) return false;
     const double tiles = (double)ceil_div(M, 2 * BM) * (narrow(N) ? 2 : 4 * ceil_div(N, 128)) * ceil_div(K, BK);
     const double entries = (double)K * N + (packed ? 0.0 : (double)M * K);
     const double here = 40e-6 + 19e-12 * entries + 60e-9 * tiles + 10e-12 * (double)M * N;

@@ -6,6 +6,8 @@
 namespace q3b {
 namespace zmod {
 
+constexpr int kLongestK = 257 * 16384;  // of a product (zmod_combine adds the bytes of 257 ranges)
+
 // An operand scaled to integers and reduced modulo each modulus, as the tiles
 // of 128 rows x 128 K the kernel copies, for operands used many times (a
 // k-point's projectors).  Rows are M of the product, K its reduction index.

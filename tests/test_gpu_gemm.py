@@ -103,6 +103,29 @@ def test_gemm_long_operands(ctx):
     assert err < 32 * k * 2.0 ** -53, err
 
 
+@pytest.mark.parametrize("ta,m,n,k", [("C", 512, 256, 24000), ("N", 24000, 256, 512)])
+def test_gemm_keeps_small_entries(ctx, ta, m, n, k):
+    """q3b_gemm's bar is per entry, also where a row's large entries meet a column's tiny ones."""
+    import torch
+    g = torch.Generator(device="cuda")
+    g.manual_seed(m)
+
+    def rand(*shape):
+        return torch.randn(*shape, dtype=torch.complex128, device="cuda", generator=g)
+
+    front = (torch.arange(k, device="cuda") < k // 2).double()
+    a = rand(m, k) * (front + 1e-25 * (1 - front))   # op(A)
+    b = rand(k, n) * (1e-25 * front + 1 - front)[:, None]
+    A = (a.conj() if ta == "C" else a.T).resolve_conj().contiguous()  # column-major K x M, or M x K
+    B, c = b.T.contiguous(), torch.empty(n, m, dtype=torch.complex128, device="cuda")
+    torch.cuda.synchronize()
+    check(ctx.handle, ctx.lib.q3b_gemm(ctx.handle, ta.encode(), b"N", m, n, k, Cplx128(1, 0), A.data_ptr(),
+                                       k if ta == "C" else m, B.data_ptr(), k, Cplx128(0, 0), c.data_ptr(), m))
+    ctx.synchronize()
+    err = (c.T - a @ b).abs() / (a.abs() @ b.abs())
+    assert float(err.max()) < 1e-13
+
+
 def test_residue_products_end_where_their_byte_sums_do(ctx):
     """257 K ranges of 16384 are the most whose bytes add up in 16 bits."""
     worth = ctx.lib["_ZN3q3b4zmod5worthEbiiib"]  # bool q3b::zmod::worth(bool, int, int, int, bool)

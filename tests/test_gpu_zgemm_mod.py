@@ -1,5 +1,5 @@
-"""The FP64 complex products that run on the integer tensor cores (q3b_gemm at the sizes
-that take them), entry by entry against exactly rounded sums.
+"""The FP64 complex products on the integer tensor cores (q3b_gemm_residue, and the library's own
+large products), entry by entry against exactly rounded sums.
 
 Bound: both operands are rounded to integers of row norm at least 2^(c-1), c = 58.39, with an
 error of at most 1/2 in each real number, so an entry is off by at most
@@ -19,6 +19,7 @@ pytestmark = pytest.mark.gpu
 SHAPES = [
     ("C", 257, 257, 16384), ("C", 300, 193, 16385), ("C", 260, 130, 40007), ("C", 513, 257, 1023),
     ("N", 6200, 256, 384), ("N", 4097, 321, 257), ("N", 130, 65, 16500), ("N", 512, 512, 512),
+    ("C", 1, 1, 1), ("N", 3, 2, 5),
 ]
 
 
@@ -39,9 +40,9 @@ def _gemm(ctx, ta, a, b, c, alpha, beta, pad=1):
     (A, lda), (B, ldb), (C, ldc) = dev(a, pad), dev(b, 2 * pad), dev(c, pad)
     m, n, k = c.shape[0], c.shape[1], b.shape[0]
     before = ctx.lib.q3b_kernel_launches()
-    check(ctx.handle, ctx.lib.q3b_gemm(ctx.handle, ta.encode(), b"N", m, n, k, Cplx128(alpha.real, alpha.imag),
-                                       A.data_ptr(), lda, B.data_ptr(), ldb, Cplx128(beta.real, beta.imag),
-                                       C.data_ptr(), ldc))
+    check(ctx.handle, ctx.lib.q3b_gemm_residue(ctx.handle, ta.encode(), b"N", m, n, k,
+                                               Cplx128(alpha.real, alpha.imag), A.data_ptr(), lda, B.data_ptr(), ldb,
+                                               Cplx128(beta.real, beta.imag), C.data_ptr(), ldc))
     ctx.synchronize()
     # two kernels pack each operand, two make the product (the FP64 units' path has two at most)
     assert ctx.lib.q3b_kernel_launches() - before >= 6
