@@ -596,7 +596,7 @@ void cgemm_two(cudaStream_t st, int M, int N, int K, const cplx_t<R>* A, long ld
             reinterpret_cast<uintptr_t>(B1) % 16 == 0 && reinterpret_cast<uintptr_t>(B2) % 16 == 0) {
             unsigned char* tiles = static_cast<unsigned char*>(ws.ptr);
             int* exps = reinterpret_cast<int*>(tiles + zmod::packed_a_bytes(M, K));
-            zmod::pack_a(st, M, K, A, lda, true, tiles, exps);
+            zmod::pack_a(st, M, K, A, lda, true, nullptr, tiles, exps);
             const zmod::PackedA pk{tiles, exps, M, K};
             const size_t used = packed_once_bytes(M, K);
             const GemmWorkspace rest{tiles + used, ws.bytes - used, ws.counters, true};

@@ -8,7 +8,9 @@
 // largest part lies in [2^13, 2^14), and every part is split into two FP16
 // numbers, x = hi + lo with hi = rn(x), lo = rn(x - hi): 22 bits, what a split
 // into two TF32 numbers keeps, for parts down to 2^-18 of the row's largest (lo
-// stays normal), and an absolute 2^-39 of it below.  A real product is
+// stays normal), and an absolute 2^-39 of it below.  So that the large parts of the
+// one operand do not meet the small ones of the other, beta and the bands are first
+// balanced along K by powers of two (PackedA::balance).  A real product is
 // hi*hi + hi*lo + lo*hi, accumulated in FP32 in TMEM, as in the TF32 kernel
 // (cgemm_tc.cu) at twice the tensor rate and half the operand bytes.
 //
@@ -66,8 +68,29 @@ __device__ __forceinline__ int exponent_for(float mx) {
     return kTop - e;
 }
 __device__ __forceinline__ float larger(float mx, float2 v) { return fmaxf(mx, fmaxf(fabsf(v.x), fabsf(v.y))); }
+__device__ __forceinline__ float pow2f(int e) { return __int_as_float((127 + e) << 23); }
 
-__global__ void __launch_bounds__(256) exps_kmajor(int R, int K, const float2* __restrict__ X, long ld, int* exps) {
+// The operands along K (PackedA::balance): A and B times 2^(sign balance[k]), with opposite
+// signs.  Lines of A more than 2^60 below the largest are left 2^60 below it.
+struct Balance {
+    const int* exps;
+    int sign;
+    __device__ __forceinline__ int at(int k) const { return exps ? sign * max(exps[k], -60) : 0; }
+    // of eight places from a multiple of eight on (the array is padded with zeros)
+    __device__ __forceinline__ void get8(int k, int* e) const {
+#pragma unroll
+        for (int q = 0; q < 2; ++q) {
+            const int4 v = exps ? *reinterpret_cast<const int4*>(exps + k + 4 * q) : make_int4(0, 0, 0, 0);
+            e[4 * q] = sign * max(v.x, -60);
+            e[4 * q + 1] = sign * max(v.y, -60);
+            e[4 * q + 2] = sign * max(v.z, -60);
+            e[4 * q + 3] = sign * max(v.w, -60);
+        }
+    }
+};
+
+__global__ void __launch_bounds__(256) exps_kmajor(int R, int K, const float2* __restrict__ X, long ld, Balance bal,
+                                                   int* exps) {
     chain_begin();
     const int r = blockIdx.x;
     float mx = 0.f;
@@ -75,10 +98,15 @@ __global__ void __launch_bounds__(256) exps_kmajor(int R, int K, const float2* _
         const float2* x = X + (long)r * ld;
         for (int k = threadIdx.x; k < K; k += 8 * 256) {
             float2 v[8];
+            float f[8];
 #pragma unroll
-            for (int u = 0; u < 8; ++u) v[u] = k + 256 * u < K ? x[k + 256 * u] : make_float2(0.f, 0.f);
+            for (int u = 0; u < 8; ++u) {
+                const bool ok = k + 256 * u < K;
+                v[u] = ok ? x[k + 256 * u] : make_float2(0.f, 0.f);
+                f[u] = pow2f(ok ? bal.at(k + 256 * u) : 0);
+            }
 #pragma unroll
-            for (int u = 0; u < 8; ++u) mx = larger(mx, v[u]);
+            for (int u = 0; u < 8; ++u) mx = larger(mx, f[u] * v[u]);
         }
     }
     __shared__ float s[8];
@@ -91,17 +119,23 @@ __global__ void __launch_bounds__(256) exps_kmajor(int R, int K, const float2* _
     }
 }
 
-__global__ void __launch_bounds__(256) exps_mmajor(int R, int K, const float2* __restrict__ X, long ld, int* exps) {
+__global__ void __launch_bounds__(256) exps_mmajor(int R, int K, const float2* __restrict__ X, long ld, Balance bal,
+                                                   int* exps) {
     chain_begin();
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, r = blockIdx.x * 32 + lane;
     float mx = 0.f;
     if (r < R) {
         for (int k = w; k < K; k += 8 * 8) {
             float2 v[8];
+            float f[8];
 #pragma unroll
-            for (int u = 0; u < 8; ++u) v[u] = k + 8 * u < K ? X[r + (long)(k + 8 * u) * ld] : make_float2(0.f, 0.f);
+            for (int u = 0; u < 8; ++u) {
+                const bool ok = k + 8 * u < K;
+                v[u] = ok ? X[r + (long)(k + 8 * u) * ld] : make_float2(0.f, 0.f);
+                f[u] = pow2f(ok ? bal.at(k + 8 * u) : 0);
+            }
 #pragma unroll
-            for (int u = 0; u < 8; ++u) mx = larger(mx, v[u]);
+            for (int u = 0; u < 8; ++u) mx = larger(mx, f[u] * v[u]);
         }
     }
     __shared__ float s[8][32];
@@ -113,9 +147,8 @@ __global__ void __launch_bounds__(256) exps_mmajor(int R, int K, const float2* _
     }
 }
 
-// x 2^e without leaving the range on the way (|e| up to 163)
+// x 2^e without leaving the range on the way (|e| up to 163, and 60 along K)
 __device__ __forceinline__ float scaled(float x, float f1, float f2) { return x * f1 * f2; }
-__device__ __forceinline__ float pow2f(int e) { return __int_as_float((127 + e) << 23); }
 
 // ------------------------------------------------------------------ packing
 // 32 rows x 64 K a block; a thread takes eight consecutive K of one row and writes
@@ -128,7 +161,8 @@ constexpr int PACK_PITCH = 8 * 9 + 1;  // float2 per row: chunks of 8 + 1, odd i
 
 template <bool KMAJOR, int ROWS, int AS>
 __global__ void __launch_bounds__(256) pack_rows(int R, int K, const float2* __restrict__ X, long ld,
-                                                 const int* __restrict__ exps, int nkb, unsigned char* out) {
+                                                 Balance bal, const int* __restrict__ exps, int nkb,
+                                                 unsigned char* out) {
     chain_begin();
     __shared__ float2 s[PACK_ROWS * PACK_PITCH];
     const int tid = threadIdx.x, kb = blockIdx.y, k0 = kb * BK, r0 = blockIdx.x * PACK_ROWS;
@@ -148,14 +182,17 @@ __global__ void __launch_bounds__(256) pack_rows(int R, int K, const float2* __r
     }
     __syncthreads();
     const int row = tid >> 3, ch = tid & 7, gr = r0 + row, e = exps[gr];
-    const float f1 = pow2f(e / 2), f2 = pow2f(e - e / 2);
+    const float f1 = pow2f(e / 2);
+    int along[8];
+    bal.get8(k0 + 8 * ch, along);
     unsigned hi[2][4], lo[2][4];
 #pragma unroll
     for (int j = 0; j < 4; ++j) {
         const float2 a = s[row * PACK_PITCH + ch * 9 + 2 * j], b = s[row * PACK_PITCH + ch * 9 + 2 * j + 1];
+        const float f2 = pow2f(e - e / 2 + along[2 * j]), g2 = pow2f(e - e / 2 + along[2 * j + 1]);
 #pragma unroll
         for (int p = 0; p < 2; ++p) {
-            const float x = scaled(p ? a.y : a.x, f1, f2), y = scaled(p ? b.y : b.x, f1, f2);
+            const float x = scaled(p ? a.y : a.x, f1, f2), y = scaled(p ? b.y : b.x, f1, g2);
             const __half2 h = __floats2half2_rn(x, y);
             const float2 hf = __half22float2(h);
             const __half2 l = __floats2half2_rn(x - hf.x, y - hf.y);
@@ -464,20 +501,22 @@ void set_limits() {
 
 // scales and tiles of R rows, padded to whole pair tiles (2 ROWS)
 template <bool KMAJOR, int ROWS, int AS>
-void pack_operand(cudaStream_t st, int R, int K, const float2* X, long ld, unsigned char* tiles, int* exps) {
+void pack_operand(cudaStream_t st, int R, int K, const float2* X, long ld, const int* balance, unsigned char* tiles,
+                  int* exps) {
+    const Balance bal{balance, AS == kPackA ? -1 : 1};
     const int padded = ceil_div(R, 2 * ROWS) * 2 * ROWS, nkb = ceil_div(K, BK);
     if (K > kLongestK) throw std::runtime_error("tensor-core GEMM: operand too large to pack");
-    if (KMAJOR) launch_chained(exps_kmajor, padded, 256, 0, st, R, K, X, ld, exps);
-    else launch_chained(exps_mmajor, padded / 32, 256, 0, st, R, K, X, ld, exps);
+    if (KMAJOR) launch_chained(exps_kmajor, padded, 256, 0, st, R, K, X, ld, bal, exps);
+    else launch_chained(exps_mmajor, padded / 32, 256, 0, st, R, K, X, ld, bal, exps);
     Q3B_LAUNCH_CHECK();
-    launch_chained(pack_rows<KMAJOR, ROWS, AS>, dim3(padded / PACK_ROWS, nkb), 256, 0, st, R, K, X, ld, exps, nkb, tiles);
+    launch_chained(pack_rows<KMAJOR, ROWS, AS>, dim3(padded / PACK_ROWS, nkb), 256, 0, st, R, K, X, ld, bal, exps, nkb, tiles);
     Q3B_LAUNCH_CHECK();
 }
 
 template <bool CONJ_A, int BC>
 void run(cudaStream_t st, const Plan& p, int M, int N, int K, float2 alpha, const PackedA& A, const float2* B, long ldb,
          float2 beta, float2* C, long ldc, unsigned char* bt, float2* part, int* eb) {
-    pack_operand<true, BC, CONJ_A ? kPackBConj : kPackB>(st, N, K, B, ldb, bt, eb);
+    pack_operand<true, BC, CONJ_A ? kPackBConj : kPackB>(st, N, K, B, ldb, A.balance, bt, eb);
     const long units = (long)p.mt * p.nt * p.splits, pairs = device_sms() / 2 > 0 ? device_sms() / 2 : 1;
     if (units > 0x7fffffffL) throw std::runtime_error("tensor-core GEMM: too large");
     const int grid = 2 * static_cast<int>(units < pairs ? units : pairs);
@@ -496,10 +535,11 @@ void run(cudaStream_t st, const Plan& p, int M, int N, int K, float2 alpha, cons
 size_t packed_a_bytes(int M, int K) { return (size_t)ceil_div(M, 2 * BM) * 2 * ceil_div(K, BK) * A_TILE; }
 size_t packed_a_exps(int M) { return (size_t)ceil_div(M, 2 * BM) * 2 * BM; }
 
-void pack_a(cudaStream_t st, int M, int K, const float2* A, long lda, bool kmajor, unsigned char* tiles, int* exps) {
+void pack_a(cudaStream_t st, int M, int K, const float2* A, long lda, bool kmajor, const int* balance,
+            unsigned char* tiles, int* exps) {
     if (M <= 0 || K <= 0) return;
-    if (kmajor) pack_operand<true, BM, kPackA>(st, M, K, A, lda, tiles, exps);
-    else pack_operand<false, BM, kPackA>(st, M, K, A, lda, tiles, exps);
+    if (kmajor) pack_operand<true, BM, kPackA>(st, M, K, A, lda, balance, tiles, exps);
+    else pack_operand<false, BM, kPackA>(st, M, K, A, lda, balance, tiles, exps);
 }
 
 size_t workspace_bytes(bool conj_a, int M, int N, int K) { return plan_of(conj_a, M, N, K).total; }

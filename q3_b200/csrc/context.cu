@@ -660,12 +660,18 @@ void Context::pack_projectors() {
     const size_t ha = half ? span(half2x::packed_a_bytes(npw, P), half2x::packed_a_exps(npw)) : 0;
     const size_t zo = residues ? span(zmod::packed_a_bytes(P, npw), zmod::packed_a_exps(P)) : 0;
     const size_t za = residues ? span(zmod::packed_a_bytes(npw, P), zmod::packed_a_exps(npw)) : 0;
-    if (ho + ha + zo + za == 0 || !kp.beta_packs.try_reserve(this, ho + ha + zo + za)) return;
+    // and the balance along the plane waves (overlap) and along the projectors (accumulation)
+    const size_t bo = span(0, zmod::balance_ints(npw)), ba = span(0, zmod::balance_ints(P));
+    if (ho + ha + zo + za == 0 || !kp.beta_packs.try_reserve(this, bo + ba + ho + ha + zo + za)) return;
     unsigned char* at = kp.beta_packs.as<unsigned char>();
+    int *along_pw = reinterpret_cast<int*>(at), *along_proj = reinterpret_cast<int*>(at + bo);
+    zmod::balance_projectors(stream, npw, P, kp.beta64.as<double2>(), along_proj, along_pw);
+    at += bo + ba;
     auto pack = [&](auto convert, auto& packed, size_t tiles, const auto* beta, int M, int K, bool kmajor, size_t bytes) {
         int* exps = reinterpret_cast<int*>(at + tiles);
-        convert(stream, M, K, beta, npw, kmajor, at, exps);
-        packed = {at, exps, M, K};
+        const int* balance = kmajor ? along_pw : along_proj;
+        convert(stream, M, K, beta, npw, kmajor, balance, at, exps);
+        packed = {at, exps, M, K, balance};
         at += bytes;
     };
     if (half) {

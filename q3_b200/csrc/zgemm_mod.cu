@@ -26,6 +26,21 @@
 // 0.6 2^-58.4 |a| |b| = 1.6e-18 |a| |b| (|a|, |b| the norms of its row and
 // column), where K rounded DFMAs leave about 4e-17 |a| |b|.
 //
+// Balance.  DFMAs leave 1e-16 sum |a_k b_k| at the worst, whatever the scales along K;
+// the norms count a_k and b_k by themselves.  Where the large entries of the one
+// operand meet small ones of the other (projectors of unequal norms, whose D
+// makes up for it; U^-1 of a basis of unequal norms), |a| |b| is far above the sum,
+// so op(A) and B are first multiplied along K by 2^t_k and 2^-t_k, exactly:
+//   N,N: t_k from the norms of B's rows;
+//   projectors: from the norms of beta's columns for beta B', and of its rows, with
+//     the columns balanced, for beta^H psi, once per k-point (balance_projectors).
+// beta D beta^H psi of the 64-atom cell, relative 2-norm from the exact value, without
+// the balance, with it, and on DFMAs: projector norms spread over 1e6, 1.7e-12, 1.6e-15
+// and 3.7e-15; bands of high plane waves only, 1.9e-13, 3.4e-16 and 2.7e-15; as the cell
+// has them, 1.7e-16, 2.0e-16 and 3.3e-15.  It costs 17 us of the 1.8 ms of H|psi>.
+// Other C,N products are inner products of vectors, which need no more than
+// 1.6e-18 of their norms.
+//
 // Rows or columns that hold an infinity or a NaN give NaN in all their outputs.
 #include <cmath>
 #include <cstdint>
@@ -44,6 +59,8 @@ using namespace umma;
 constexpr int NMOD = 15;
 constexpr int kMod[NMOD] = {256, 255, 253, 251, 247, 241, 239, 233, 229, 227, 223, 217, 211, 199, 197};
 constexpr int kNotFinite = -(1 << 30);  // exponent of a row that holds an infinity or a NaN
+constexpr int kZeroLine = 1 << 29;      // of a line of zeros, where lines are balanced
+constexpr int kBalanceSpan = 100;       // lines are balanced to within 2^100 of the largest
 
 // ------------------------------------------------------------ modulus constants
 constexpr unsigned pow256(int j, int m) {
@@ -131,13 +148,13 @@ static_assert(255 * kMaxRanges <= 0xffff, "zmod_combine adds the ranges' bytes i
 // exponent s with |row| 2^s <= 2^c from the row's sum of squares and largest
 // magnitude; the sum of squares of very large or very small values leaves
 // the range of doubles, and the bound |row| <= max sqrt(2 K) takes its place
-__device__ __forceinline__ int row_exponent(double ss, double mx, int K, double c) {
+__device__ __forceinline__ int row_exponent(double ss, double mx, int K, double c, int zero) {
     if (!(mx < INFINITY) || ss != ss) return kNotFinite;
-    if (mx == 0.0) return 0;
+    if (mx == 0.0) return zero;
     if (ss > 1e-280 && ss < 1e300) return static_cast<int>(floor(c - 0.5 * log2(ss)));
     int e;
-    frexp(mx, &e);  // mx < 2^e
-    return static_cast<int>(floor(c - e - 0.5 * log2(2.0 * K)));
+    frexp(mx, &e);  // mx < 2^e; a denormal may have been rounded down to half
+    return static_cast<int>(floor(c - e - 0.5 * log2(2.0 * K))) - (mx < 1e-300 ? 1 : 0);
 }
 
 __device__ __forceinline__ void take(double2 v, double& ss, double& mx) {
@@ -148,9 +165,30 @@ __device__ __forceinline__ void take(double2 v, double& ss, double& mx) {
     if (b > mx) mx = b;
 }
 
+__device__ __forceinline__ double pow2(int e) { return __hiloint2double((1023 + e) << 20, 0); }
+
+// The operands along K (`balance`, may be null): op(A) and B times 2^(sign balance[k]),
+// with opposite signs, which leaves the product as it is.
+struct Balance {
+    const int* exps;
+    int sign;
+    __device__ __forceinline__ int at(int k) const { return exps ? sign * exps[k] : 0; }
+    // of 16 places from a multiple of 16 on (the array is padded with zeros to whole K blocks)
+    __device__ __forceinline__ void get16(int k, int* e) const {
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+            const int4 v = exps ? *reinterpret_cast<const int4*>(exps + k + 4 * q) : make_int4(0, 0, 0, 0);
+            e[4 * q] = sign * v.x;
+            e[4 * q + 1] = sign * v.y;
+            e[4 * q + 2] = sign * v.z;
+            e[4 * q + 3] = sign * v.w;
+        }
+    }
+};
+
 // rows contiguous along K: one block a row
 __global__ void __launch_bounds__(256) exps_kmajor(int R, int K, const double2* __restrict__ X, long ld, double c,
-                                                   int* exps) {
+                                                   Balance bal, int zero, int* exps) {
     chain_begin();
     const int r = blockIdx.x;
     double ss = 0.0, mx = 0.0;
@@ -158,10 +196,15 @@ __global__ void __launch_bounds__(256) exps_kmajor(int R, int K, const double2* 
         const double2* x = X + (long)r * ld;
         for (int k = threadIdx.x; k < K; k += 4 * 256) {
             double2 v[4];
+            double f[4];
 #pragma unroll
-            for (int u = 0; u < 4; ++u) v[u] = k + 256 * u < K ? x[k + 256 * u] : make_double2(0.0, 0.0);
+            for (int u = 0; u < 4; ++u) {
+                const bool ok = k + 256 * u < K;
+                v[u] = ok ? x[k + 256 * u] : make_double2(0.0, 0.0);
+                f[u] = pow2(ok ? bal.at(k + 256 * u) : 0);
+            }
 #pragma unroll
-            for (int u = 0; u < 4; ++u) take(v[u], ss, mx);
+            for (int u = 0; u < 4; ++u) take(f[u] * v[u], ss, mx);
         }
     }
     __shared__ double s_ss[8], s_mx[8];
@@ -179,40 +222,65 @@ __global__ void __launch_bounds__(256) exps_kmajor(int R, int K, const double2* 
             ss += s_ss[w];
             mx = fmax(mx, s_mx[w]);
         }
-        exps[r] = r < R ? row_exponent(ss, mx, K, c) : 0;
+        exps[r] = r < R ? row_exponent(ss, mx, K, c, zero) : 0;
     }
 }
 
-// rows along the contiguous index: 32 rows a block, K dealt to eight warps
-__global__ void __launch_bounds__(256) exps_mmajor(int R, int K, const double2* __restrict__ X, long ld, double c,
-                                                   int* exps) {
+// rows along the contiguous index: 32 rows a block, K dealt to W warps
+template <int W>
+__global__ void __launch_bounds__(32 * W) exps_mmajor(int R, int K, const double2* __restrict__ X, long ld, double c,
+                                                   Balance bal, int zero, int* exps) {
     chain_begin();
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     const int r = blockIdx.x * 32 + lane;
     double ss = 0.0, mx = 0.0;
     if (r < R) {
-        for (int k = w; k < K; k += 4 * 8) {
+        for (int k = w; k < K; k += 4 * W) {
             double2 v[4];
+            double f[4];
 #pragma unroll
-            for (int u = 0; u < 4; ++u) v[u] = k + 8 * u < K ? X[r + (long)(k + 8 * u) * ld] : make_double2(0.0, 0.0);
+            for (int u = 0; u < 4; ++u) {
+                const bool ok = k + W * u < K;
+                v[u] = ok ? X[r + (long)(k + W * u) * ld] : make_double2(0.0, 0.0);
+                f[u] = pow2(ok ? bal.at(k + W * u) : 0);
+            }
 #pragma unroll
-            for (int u = 0; u < 4; ++u) take(v[u], ss, mx);
+            for (int u = 0; u < 4; ++u) take(f[u] * v[u], ss, mx);
         }
     }
-    __shared__ double s_ss[8][32], s_mx[8][32];
+    __shared__ double s_ss[W][32], s_mx[W][32];
     s_ss[w][lane] = ss;
     s_mx[w][lane] = mx;
     __syncthreads();
     if (w == 0) {
-        for (int j = 1; j < 8; ++j) {
+        for (int j = 1; j < W; ++j) {
             ss += s_ss[j][lane];
             mx = fmax(mx, s_mx[j][lane]);
         }
-        exps[r] = r < R ? row_exponent(ss, mx, K, c) : 0;
+        exps[r] = r < R ? row_exponent(ss, mx, K, c, zero) : 0;
     }
 }
 
-__device__ __forceinline__ double pow2(int e) { return __hiloint2double((1023 + e) << 20, 0); }
+// Exponents of lines (each with its norm's distance below 2^c) to those that bring
+// the shorter lines up to the longest, times `sign`, with zeros up to `padded`.  One
+// block.
+__global__ void __launch_bounds__(1024) balance_lines(int n, int padded, int sign, int* exps) {
+    chain_begin();
+    __shared__ int s_least[32];
+    int least = kZeroLine;
+    for (int i = threadIdx.x; i < n; i += 1024) {
+        const int e = exps[i];
+        if (e != kNotFinite) least = min(least, e);
+    }
+    least = __reduce_min_sync(0xffffffffu, least);
+    if ((threadIdx.x & 31) == 0) s_least[threadIdx.x >> 5] = least;
+    __syncthreads();
+    for (int w = 0; w < 32; ++w) least = min(least, s_least[w]);
+    for (int i = threadIdx.x; i < padded; i += 1024) {
+        const int e = i < n ? exps[i] : kNotFinite;
+        exps[i] = e == kNotFinite ? 0 : sign * (e == kZeroLine ? kBalanceSpan : min(e - least, kBalanceSpan));
+    }
+}
 
 // ------------------------------------------------------------------ packing
 // 32 rows x 128 K a block; a thread takes 16 consecutive K of one row and
@@ -232,7 +300,8 @@ constexpr int PACK_SMEM = PACK_ROWS * PACK_PITCH * 16;
 enum PackAs { kPackA, kPackB, kPackBConj };
 template <bool KMAJOR, int ROWS, int AS>
 __global__ void __launch_bounds__(256) pack_rows(int R, int K, const double2* __restrict__ X, long ld,
-                                                 const int* __restrict__ exps, int nkb, unsigned char* out) {
+                                                 Balance bal, const int* __restrict__ exps, int nkb,
+                                                 unsigned char* out) {
     chain_begin();
     extern __shared__ __align__(16) unsigned char psm[];
     double2* s = reinterpret_cast<double2*>(psm);
@@ -252,11 +321,15 @@ __global__ void __launch_bounds__(256) pack_rows(int R, int K, const double2* __
     const int gr = r0 + row;
     const int e = exps[gr];
     const int e1 = e == kNotFinite ? 0 : e / 2, e2 = e == kNotFinite ? 0 : e - e / 2;
-    const double f1 = pow2(e1), f2 = pow2(e2);
+    // in two steps, so that only the scaled value has to be in range
+    const double f1 = pow2(e1);
+    int along[16];
+    bal.get16(k0 + 16 * ch, along);
     unsigned lo[2][16], hi[2][16];
 #pragma unroll
     for (int j = 0; j < 16; ++j) {
         const double2 v = s[row * PACK_PITCH + ch * 17 + j];
+        const double f2 = pow2(e2 + along[j]);
         // + 2^63 as an unsigned number; each modulus takes it back
         const unsigned long long a = static_cast<unsigned long long>(__double2ll_rn(v.x * f1 * f2)) ^ (1ull << 63);
         const unsigned long long b = static_cast<unsigned long long>(__double2ll_rn(v.y * f1 * f2)) ^ (1ull << 63);
@@ -637,7 +710,7 @@ bool narrow(int N) { return N <= 64; }
 
 struct Plan {
     int bc, mt, nt, nkb, splits, kb_per, panel;  // panel: pair tiles along M that a launch takes
-    size_t b_bytes, a_bytes, out_bytes, exp_bytes, total;
+    size_t b_bytes, a_bytes, out_bytes, exp_bytes, balance_bytes, total;
 };
 
 // the packed rows of A and the output bytes of one panel stay below this
@@ -662,7 +735,8 @@ Plan plan_of(bool conj_a, int M, int N, int K, bool packed) {
     p.a_bytes = packed ? 0 : (size_t)p.panel * 2 * p.nkb * NMOD * A_TILE;
     p.out_bytes = (size_t)p.panel * 2 * p.nt * NMOD * out_tile * p.splits;
     p.exp_bytes = align256(((size_t)p.panel * 2 * BM + (size_t)p.nt * 2 * p.bc) * sizeof(int));
-    p.total = p.b_bytes + p.a_bytes + p.out_bytes + p.exp_bytes;
+    p.balance_bytes = !conj_a && !packed ? align256(balance_ints(K) * sizeof(int)) : 0;
+    p.total = p.b_bytes + p.a_bytes + p.out_bytes + p.exp_bytes + p.balance_bytes;
     return p;
 }
 
@@ -687,19 +761,21 @@ void set_limits() {
 
 // scales and residue tiles of R rows, padded to whole pair tiles (2 ROWS)
 template <bool KMAJOR, int ROWS, int AS>
-void pack_operand(cudaStream_t st, int R, int K, const double2* X, long ld, unsigned char* tiles, int* exps) {
+void pack_operand(cudaStream_t st, int R, int K, const double2* X, long ld, const int* balance, unsigned char* tiles,
+                  int* exps) {
+    const Balance bal{balance, AS == kPackA ? -1 : 1};
     const int padded = ceil_div(R, 2 * ROWS) * 2 * ROWS, nkb = ceil_div(K, BK);
     if (nkb > 65535) throw std::runtime_error("complex GEMM: operand too large to pack");
-    if (KMAJOR) launch_chained(exps_kmajor, padded, 256, 0, st, R, K, X, ld, scale_bits(), exps);
-    else launch_chained(exps_mmajor, padded / 32, 256, 0, st, R, K, X, ld, scale_bits(), exps);
+    if (KMAJOR) launch_chained(exps_kmajor, padded, 256, 0, st, R, K, X, ld, scale_bits(), bal, 0, exps);
+    else launch_chained(exps_mmajor<8>, padded / 32, 256, 0, st, R, K, X, ld, scale_bits(), bal, 0, exps);
     Q3B_LAUNCH_CHECK();
-    launch_chained(pack_rows<KMAJOR, ROWS, AS>, dim3(padded / PACK_ROWS, nkb), 256, PACK_SMEM, st, R, K, X, ld, exps, nkb, tiles);
+    launch_chained(pack_rows<KMAJOR, ROWS, AS>, dim3(padded / PACK_ROWS, nkb), 256, PACK_SMEM, st, R, K, X, ld, bal, exps, nkb, tiles);
     Q3B_LAUNCH_CHECK();
 }
-void pack_rows_of_a(cudaStream_t st, int M, int K, const double2* A, long lda, bool kmajor, unsigned char* tiles,
-                    int* exps) {
-    if (kmajor) pack_operand<true, BM, kPackA>(st, M, K, A, lda, tiles, exps);
-    else pack_operand<false, BM, kPackA>(st, M, K, A, lda, tiles, exps);
+void pack_rows_of_a(cudaStream_t st, int M, int K, const double2* A, long lda, bool kmajor, const int* balance,
+                    unsigned char* tiles, int* exps) {
+    if (kmajor) pack_operand<true, BM, kPackA>(st, M, K, A, lda, balance, tiles, exps);
+    else pack_operand<false, BM, kPackA>(st, M, K, A, lda, balance, tiles, exps);
 }
 
 template <bool CONJ_A, int BC>
@@ -738,10 +814,27 @@ ModTable mod_table() {
 size_t packed_a_bytes(int M, int K) { return (size_t)ceil_div(M, 2 * BM) * 2 * ceil_div(K, BK) * NMOD * A_TILE; }
 size_t packed_a_exps(int M) { return (size_t)ceil_div(M, 2 * BM) * 2 * BM; }
 
-void pack_a(cudaStream_t st, int M, int K, const double2* A, long lda, bool kmajor, unsigned char* tiles, int* exps) {
+void pack_a(cudaStream_t st, int M, int K, const double2* A, long lda, bool kmajor, const int* balance,
+            unsigned char* tiles, int* exps) {
     if (M <= 0 || K <= 0) return;
     set_limits();
-    pack_rows_of_a(st, M, K, A, lda, kmajor, tiles, exps);
+    pack_rows_of_a(st, M, K, A, lda, kmajor, balance, tiles, exps);
+}
+
+size_t balance_ints(int lines) { return (size_t)ceil_div(lines, BK) * BK; }
+
+void balance_projectors(cudaStream_t st, int npw, int nproj, const double2* beta, int* along_proj, int* along_pw) {
+    if (npw <= 0 || nproj <= 0) return;
+    launch_chained(exps_kmajor, nproj, 256, 0, st, nproj, npw, beta, npw, scale_bits(), Balance{nullptr, 0}, kZeroLine,
+                   along_proj);
+    Q3B_LAUNCH_CHECK();
+    launch_chained(balance_lines, 1, 1024, 0, st, nproj, (int)balance_ints(nproj), -1, along_proj);
+    Q3B_LAUNCH_CHECK();
+    launch_chained(exps_mmajor<8>, ceil_div(npw, 32), 256, 0, st, npw, nproj, beta, npw, scale_bits(),
+                   Balance{along_proj, -1}, kZeroLine, along_pw);
+    Q3B_LAUNCH_CHECK();
+    launch_chained(balance_lines, 1, 1024, 0, st, npw, (int)balance_ints(npw), -1, along_pw);
+    Q3B_LAUNCH_CHECK();
 }
 
 // Estimated times of both paths, from runs of q3b_gemm on shapes of the 8- to
@@ -783,12 +876,22 @@ void zgemm(cudaStream_t st, bool conj_a, int M, int N, int K, double2 alpha, con
     long double prod = std::ldexp(1.0L, -80);
     for (int m : kMod) prod *= m;
     const double product = static_cast<double>(prod);
+    const int* balance = pk ? pk->balance : nullptr;
+    if (p.balance_bytes) {
+        int* rows_of_b = reinterpret_cast<int*>(out + p.out_bytes + p.exp_bytes);
+        launch_chained(exps_mmajor<32>, ceil_div(K, 32), 1024, 0, st, K, N, B, ldb, scale_bits(),
+                       Balance{nullptr, 0}, kZeroLine, rows_of_b);
+        Q3B_LAUNCH_CHECK();
+        launch_chained(balance_lines, 1, 1024, 0, st, K, (int)balance_ints(K), 1, rows_of_b);
+        Q3B_LAUNCH_CHECK();
+        balance = rows_of_b;
+    }
     if (p.bc == 64) {
-        if (conj_a) pack_operand<true, 64, kPackBConj>(st, N, K, B, ldb, bt, eb);
-        else pack_operand<true, 64, kPackB>(st, N, K, B, ldb, bt, eb);
+        if (conj_a) pack_operand<true, 64, kPackBConj>(st, N, K, B, ldb, balance, bt, eb);
+        else pack_operand<true, 64, kPackB>(st, N, K, B, ldb, balance, bt, eb);
     } else {
-        if (conj_a) pack_operand<true, 32, kPackBConj>(st, N, K, B, ldb, bt, eb);
-        else pack_operand<true, 32, kPackB>(st, N, K, B, ldb, bt, eb);
+        if (conj_a) pack_operand<true, 32, kPackBConj>(st, N, K, B, ldb, balance, bt, eb);
+        else pack_operand<true, 32, kPackB>(st, N, K, B, ldb, balance, bt, eb);
     }
     const ModTable tab = mod_table();
     for (int m0 = 0; m0 < p.mt; m0 += p.panel) {
@@ -797,7 +900,7 @@ void zgemm(cudaStream_t st, bool conj_a, int M, int N, int K, double2 alpha, con
         const int rows = static_cast<int>(M - r0 < (long)mt * 2 * BM ? M - r0 : (long)mt * 2 * BM);
         const unsigned char* a = pk ? pk->tiles + (size_t)m0 * 2 * p.nkb * NMOD * A_TILE : at;
         const int* ea = pk ? pk->exps + r0 : ea_ws;
-        if (!pk) pack_rows_of_a(st, rows, K, conj_a ? A + r0 * lda : A + r0, lda, conj_a, at, ea_ws);
+        if (!pk) pack_rows_of_a(st, rows, K, conj_a ? A + r0 * lda : A + r0, lda, conj_a, balance, at, ea_ws);
         auto run = [&](auto conj) {
             constexpr bool CA = decltype(conj)::value;
             if (p.bc == 64)

@@ -102,6 +102,22 @@ def test_entries_against_exact_sums(ctx, ta, m, n, k, kind):
             assert abs(got[i, j] - want) <= slack, (i, j, abs(got[i, j] - want), slack)
 
 
+def test_scales_along_k_do_not_count(ctx):
+    """N,N: the scales of A's columns and B's rows against each other, as in a basis of unequal
+    norms times the inverse of its Cholesky factor, leave every bit as it is without them."""
+    rng = np.random.default_rng(11)
+    m, n, k = 1000, 130, 257
+    a, b = _operand(rng, "normal", m, k), _operand(rng, "normal", k, n)
+    scale = 2.0 ** rng.integers(-40, 41, k)
+    zero = np.zeros((m, n), complex)
+    want = _gemm(ctx, "N", a, b, zero, 1 + 0j, 0j)
+    got = _gemm(ctx, "N", a * scale[None, :], b / scale[:, None], zero, 1 + 0j, 0j)
+    assert np.array_equal(got, want)
+    far = 2.0 ** rng.integers(-400, 401, k)  # beyond what is balanced: the bits are those of the largest
+    got = _gemm(ctx, "N", a * far[None, :], b / far[:, None], zero, 1 + 0j, 0j)
+    assert np.isfinite(got).all()
+
+
 @pytest.mark.parametrize("ta", ["C", "N"])
 def test_scales_zeros_and_non_finite(ctx, ta):
     """Rows far out of the usual range (their squares leave it), zero rows, and rows with an
