@@ -98,6 +98,10 @@ struct ErrorScope {
 };
 // read (and clear) it; throws CudaError when it was set.  Synchronises st.
 void check_error(cudaStream_t st);
+// read and clear `word` on an error path, where nothing may be thrown; false also
+// where it cannot be read
+bool take_error(cudaStream_t st, int* word) noexcept;
+extern const char* const kTimedOut;
 }  // namespace tc
 
 }  // namespace q3b

@@ -586,6 +586,9 @@ int* error_word() {
     return cached;
 }
 
+const char* const kTimedOut =
+    "a bounded device wait timed out (tensor-core GEMM pipeline or plane-kernel stick copy)";
+
 void check_error(cudaStream_t st) {
     int* w = error_word();
     int* hb = static_cast<int*>(host_readback(sizeof(int)));
@@ -593,8 +596,22 @@ void check_error(cudaStream_t st) {
     Q3B_CUDA(cudaStreamSynchronize(st));
     if (hb[0]) {
         Q3B_CUDA(cudaMemsetAsync(w, 0, sizeof(int), st));
-        throw CudaError("a bounded device wait timed out (tensor-core GEMM pipeline or plane-kernel stick copy)");
+        throw CudaError(kTimedOut);
     }
+}
+
+bool take_error(cudaStream_t st, int* word) noexcept {
+    try {
+        if (!word) return false;
+        int* hb = static_cast<int*>(host_readback(sizeof(int)));
+        hb[0] = 0;
+        if (cudaMemcpyAsync(hb, word, sizeof(int), cudaMemcpyDeviceToHost, st) == cudaSuccess &&
+            cudaStreamSynchronize(st) == cudaSuccess && hb[0])
+            return cudaMemsetAsync(word, 0, sizeof(int), st) == cudaSuccess;
+    } catch (const std::exception&) {
+    }
+    cudaGetLastError();
+    return false;
 }
 
 size_t workspace_bytes(int M, int N, int K) {

@@ -918,7 +918,16 @@ int fail(q3b_context* c, const std::exception& e) {
     int code = Q3B_ERR_INTERNAL;
     if (auto s = dynamic_cast<const Status*>(&e)) code = s->code;
     else if (dynamic_cast<const CudaError*>(&e)) code = Q3B_ERR_CUDA;
-    if (c) c->impl.err = e.what();
+    if (!c) return code;
+    c->impl.err = e.what();
+    // An error of the device work's results may come from a product that a bounded wait
+    // cut short: that is reported, and the word cleared, so that the next call's waits
+    // do not heed it.  Errors of the arguments leave the word to the calls it belongs to.
+    if ((code == Q3B_ERR_LINALG || code == Q3B_ERR_CUDA || code == Q3B_ERR_INTERNAL) &&
+        tc::take_error(c->impl.stream, c->impl.err_word.as<int>())) {
+        code = Q3B_ERR_CUDA;
+        c->impl.err = std::string(tc::kTimedOut) + "; " + c->impl.err;
+    }
     return code;
 }
 

@@ -224,7 +224,7 @@ class Server {
             j.status = Q3B_OK;
         } catch (const std::exception& e) {
             j.status = fail(ctx, e);
-            j.err = e.what();
+            j.err = ctx->impl.err;
         }
     }
 

@@ -87,6 +87,7 @@ int q3b_start_project(q3b_context* ctx, q3b_cplx128* h_host, q3b_cplx128* s_host
         Q3B_CUDA(cudaMemcpyAsync(h_host, H, nn * sizeof(double2), cudaMemcpyDeviceToHost, c.stream));
         Q3B_CUDA(cudaMemcpyAsync(s_host, S, nn * sizeof(double2), cudaMemcpyDeviceToHost, c.stream));
         Q3B_CUDA(cudaStreamSynchronize(c.stream));
+        q3b::tc::check_error(c.stream);
     });
 }
 
@@ -100,6 +101,7 @@ int q3b_start_rotate(q3b_context* ctx, const q3b_cplx128* coefficients_host, int
         Q3B_CUDA(cudaMemcpyAsync(C, coefficients_host, nc * sizeof(double2), cudaMemcpyHostToDevice, c.stream));
         start_rotate_dev(c, C, c.start_n, nb, reinterpret_cast<double2*>(bands_dev));
         Q3B_CUDA(cudaStreamSynchronize(c.stream));
+        q3b::tc::check_error(c.stream);
     });
 }
 
