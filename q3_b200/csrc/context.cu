@@ -191,9 +191,9 @@ GemmWorkspace Context::gemm_ws(size_t need, size_t want) {
 bool Context::release_optional() {
     // callers ask for the GEMM workspace after all their other buffers, so no
     // product that still has to be issued holds its address here
-    bool any = kp.beta_packs.ptr != nullptr;
-    drop_packs();
-    kp.beta_packs.release();
+    bool any = kp.beta_residues.ptr != nullptr;
+    drop_residues();
+    kp.beta_residues.release();
     if (ws_gemm.bytes > ws_gemm_need_) {
         any = true;
         ws_gemm.release();
@@ -637,12 +637,13 @@ void Context::prepare_kpoint(int npw, const int32_t* g2g, const double* ke, cons
 // at 64 atoms (3.1e9), 155 against 142 at 48 (1.3e9), 77 against 42 at 19 (8e7).
 // Blocks of few bands, as the last iterations of a solve have them, are no slower
 // either: 64 atoms, 64 bands 111 us against 122, 32 bands 108 against 112, 8 bands 100
-// against 103; 56 atoms, 32 bands 98 against 101; 97 atoms, 32 bands 172 against 192.  FP64: residue tiles where the products of such a block run on them.
-// Without room for FP16 or residue tiles the products take the projectors as they
-// are.
+// against 103; 56 atoms, 32 bands 98 against 101; 97 atoms, 32 bands 172 against 192.
+// FP64: residue tiles where the products of such a block run on them;
+// without room for these the FP64 products take the projectors as they are.
 constexpr double kHalfMinMacs = 2e9;
 void Context::pack_projectors() {
-    drop_packs();
+    drop_residues();
+    kp.hs_overlap = kp.hs_accum = half2x::PackedA{};
     const int P = kp.nproj, npw = kp.npw;
     if (P <= 0) return;
     const bool half = 0.5 * P * P * npw >= kHalfMinMacs && npw <= half2x::kLongestK && P <= half2x::kLongestK;
@@ -654,40 +655,40 @@ void Context::pack_projectors() {
         tc::pack_a(stream, npw, P, kp.beta32.as<float2>(), npw, false, kp.beta_pk_accum.as<unsigned char>());
     }
     const bool residues = zmod::worth(true, P, P / 2, npw, true);
-    // tiles and exponents of the overlap and the accumulation form, one after another
+    if (!half && !residues) return;
     auto span = [](size_t tiles, size_t exps) { return (tiles + exps * sizeof(int) + 255) & ~size_t(255); };
-    const size_t ho = half ? span(half2x::packed_a_bytes(P, npw), half2x::packed_a_exps(P)) : 0;
-    const size_t ha = half ? span(half2x::packed_a_bytes(npw, P), half2x::packed_a_exps(npw)) : 0;
-    const size_t zo = residues ? span(zmod::packed_a_bytes(P, npw), zmod::packed_a_exps(P)) : 0;
-    const size_t za = residues ? span(zmod::packed_a_bytes(npw, P), zmod::packed_a_exps(npw)) : 0;
-    // and the balance along the plane waves (overlap) and along the projectors (accumulation)
-    const size_t bo = span(0, zmod::balance_ints(npw)), ba = span(0, zmod::balance_ints(P));
-    if (ho + ha + zo + za == 0 || !kp.beta_packs.try_reserve(this, bo + ba + ho + ha + zo + za)) return;
-    unsigned char* at = kp.beta_packs.as<unsigned char>();
-    int *along_pw = reinterpret_cast<int*>(at), *along_proj = reinterpret_cast<int*>(at + bo);
+    const size_t along_pw_bytes = span(0, zmod::balance_ints(npw));
+    kp.beta_balance.reserve(this, along_pw_bytes + span(0, zmod::balance_ints(P)));
+    int* along_pw = kp.beta_balance.as<int>();
+    int* along_proj = reinterpret_cast<int*>(kp.beta_balance.as<char>() + along_pw_bytes);
     zmod::balance_projectors(stream, npw, P, kp.beta64.as<double2>(), along_proj, along_pw);
-    at += bo + ba;
-    auto pack = [&](auto convert, auto& packed, size_t tiles, const auto* beta, int M, int K, bool kmajor, size_t bytes) {
+    // tiles and exponents of the overlap form, after them those of the accumulation form
+    auto pack = [&](auto convert, unsigned char* at, auto& packed, size_t tiles, const auto* beta, bool overlap) {
         int* exps = reinterpret_cast<int*>(at + tiles);
-        const int* balance = kmajor ? along_pw : along_proj;
-        convert(stream, M, K, beta, npw, kmajor, balance, at, exps);
+        const int M = overlap ? P : npw, K = overlap ? npw : P;
+        const int* balance = overlap ? along_pw : along_proj;
+        convert(stream, M, K, beta, npw, overlap, balance, at, exps);
         packed = {at, exps, M, K, balance};
-        at += bytes;
     };
     if (half) {
-        pack(half2x::pack_a, kp.hs_overlap, half2x::packed_a_bytes(P, npw), kp.beta32.as<float2>(), P, npw, true, ho);
-        pack(half2x::pack_a, kp.hs_accum, half2x::packed_a_bytes(npw, P), kp.beta32.as<float2>(), npw, P, false, ha);
+        const size_t to = half2x::packed_a_bytes(P, npw), ta = half2x::packed_a_bytes(npw, P);
+        const size_t first = span(to, half2x::packed_a_exps(P));
+        kp.beta_half.reserve(this, first + span(ta, half2x::packed_a_exps(npw)));
+        unsigned char* at = kp.beta_half.as<unsigned char>();
+        pack(half2x::pack_a, at, kp.hs_overlap, to, kp.beta32.as<float2>(), true);
+        pack(half2x::pack_a, at + first, kp.hs_accum, ta, kp.beta32.as<float2>(), false);
     }
     if (residues) {
-        pack(zmod::pack_a, kp.zm_overlap, zmod::packed_a_bytes(P, npw), kp.beta64.as<double2>(), P, npw, true, zo);
-        pack(zmod::pack_a, kp.zm_accum, zmod::packed_a_bytes(npw, P), kp.beta64.as<double2>(), npw, P, false, za);
+        const size_t to = zmod::packed_a_bytes(P, npw), ta = zmod::packed_a_bytes(npw, P);
+        const size_t first = span(to, zmod::packed_a_exps(P));
+        if (!kp.beta_residues.try_reserve(this, first + span(ta, zmod::packed_a_exps(npw)))) return;
+        unsigned char* at = kp.beta_residues.as<unsigned char>();
+        pack(zmod::pack_a, at, kp.zm_overlap, to, kp.beta64.as<double2>(), true);
+        pack(zmod::pack_a, at + first, kp.zm_accum, ta, kp.beta64.as<double2>(), false);
     }
 }
 
-void Context::drop_packs() {
-    kp.hs_overlap = kp.hs_accum = half2x::PackedA{};
-    kp.zm_overlap = kp.zm_accum = zmod::PackedA{};
-}
+void Context::drop_residues() { kp.zm_overlap = kp.zm_accum = zmod::PackedA{}; }
 
 template <> const LocalPlan<double>& Context::local_plan<double>() const { return kp.lp64; }
 template <> const LocalPlan<float>& Context::local_plan<float>() const { return kp.lp32; }
@@ -881,7 +882,7 @@ void Context::apply_h(const cplx_t<R>* psi, long ldpsi, cplx_t<R>* hpsi, long ld
         const size_t pb = (size_t)kp.nproj * nvec * sizeof(T);
         ws_bm.reserve(this, pb);
         ws_bp.reserve(this, pb);
-        GemmWorkspace ws = gemm_ws(cgemm_workspace_bytes<R>(kp.nproj, nvec, kp.npw),
+        GemmWorkspace ws = gemm_ws(nonlocal_workspace_bytes<R>(nonlocal<R>(), kp.npw, nvec),
                                    nonlocal_wanted_bytes<R>(nonlocal<R>(), kp.npw, nvec));
         apply_nonlocal<R>(stream, nonlocal<R>(), kp.npw, nvec, psi, ldpsi, hpsi, ldh,
                           ws_bm.as<T>(), ws_bp.as<T>(), ws, tm);

@@ -51,13 +51,14 @@ struct KPoint {
     std::vector<double> ke_host;
     DevBuf ke64, ke32;
     DevBuf beta64, beta32;
-    DevBuf beta_pk_overlap, beta_pk_accum;  // beta32 as TF32 tensor-core A tiles
-    // or, for large sets, as FP16 tiles; beta64 as residue tiles for the FP64
-    // products; one buffer for all, kept from one k-point to the next, empty
-    // where memory is short
-    DevBuf beta_packs;
-    half2x::PackedA hs_overlap{}, hs_accum{};  // in beta_packs, or no tiles
-    zmod::PackedA zm_overlap{}, zm_accum{};
+    // beta32 as TF32 tensor-core A tiles or, for large sets, as FP16 tiles (half their bytes)
+    DevBuf beta_pk_overlap, beta_pk_accum, beta_half;
+    DevBuf beta_balance;                       // along the plane waves and the projectors
+    half2x::PackedA hs_overlap{}, hs_accum{};  // in beta_half, or no tiles
+    // beta64 as residue tiles for the FP64 products, kept from one k-point to the
+    // next, empty where memory is short
+    DevBuf beta_residues;
+    zmod::PackedA zm_overlap{}, zm_accum{};    // in beta_residues, or no tiles
     DevBuf pstart, psize, poff, dpk64, dpk32;
     size_t dpk_len = 0;             // packed block entries (D, and Q when set)
     bool has_q = false;             // ultrasoft overlap blocks set for this k-point
@@ -161,7 +162,7 @@ class Context {
     void build_plan();
     bool pk_valid_ = false;       // kp.beta_pk_* hold the prepared k-point's projectors
     void pack_projectors();
-    void drop_packs();
+    void drop_residues();
 };
 
 // convert an exception into a status code and message

@@ -545,7 +545,7 @@ template <typename R> class Davidson {
         const size_t pb = (size_t)P * nv * sizeof(T);
         c_.ws_bm.reserve(&c_, pb);
         c_.ws_bp.reserve(&c_, pb);
-        GemmWorkspace ws = c_.gemm_ws(cgemm_workspace_bytes<R>(P, nv, len),
+        GemmWorkspace ws = c_.gemm_ws(nonlocal_workspace_bytes<R>(c_.overlap<R>(), len, nv),
                                       nonlocal_wanted_bytes<R>(c_.overlap<R>(), len, nv));
         apply_nonlocal<R>(st_, c_.overlap<R>(), len, nv, in, len, out, len, c_.ws_bm.as<T>(), c_.ws_bp.as<T>(), ws);
         if (gamma_) {

@@ -58,9 +58,17 @@ template <typename R> size_t nonlocal_wanted_bytes(const NonlocalData<R>& nl, in
             b = zmod::workspace_bytes(true, nl.nproj, nvec, npw, true);
         if (nl.zm_accum.tiles && zmod::worth(false, npw, nvec, nl.nproj, true))
             b = std::max(b, zmod::workspace_bytes(false, npw, nvec, nl.nproj, true));
-    } else if (use_tensor_cores(nl.nproj, nvec, npw)) {
-        if (nl.hs_overlap.tiles) b = half2x::workspace_bytes(true, nl.nproj, nvec, npw);
-        if (nl.hs_accum.tiles) b = std::max(b, half2x::workspace_bytes(false, npw, nvec, nl.nproj));
+    }
+    return b;
+}
+
+template <typename R> size_t nonlocal_workspace_bytes(const NonlocalData<R>& nl, int npw, int nvec) {
+    size_t b = cgemm_workspace_bytes<R>(nl.nproj, nvec, npw);
+    if constexpr (std::is_same<R, float>::value) {
+        if (use_tensor_cores(nl.nproj, nvec, npw)) {
+            if (nl.hs_overlap.tiles) b = std::max(b, half2x::workspace_bytes(true, nl.nproj, nvec, npw));
+            if (nl.hs_accum.tiles) b = std::max(b, half2x::workspace_bytes(false, npw, nvec, nl.nproj));
+        }
     }
     return b;
 }
@@ -68,7 +76,7 @@ template <typename R> size_t nonlocal_wanted_bytes(const NonlocalData<R>& nl, in
 // whether an FP32 projector product runs on the FP16 tiles (beta^H psi
 // with `overlap`, else beta B')
 static bool on_half_tiles(const NonlocalData<float>& nl, bool overlap, int npw, int nvec, const GemmWorkspace& ws) {
-    if (!use_tensor_cores(nl.nproj, nvec, npw) || !ws.wanted) return false;
+    if (!use_tensor_cores(nl.nproj, nvec, npw) || !ws.ptr) return false;
     return overlap ? nl.hs_overlap.tiles && ws.bytes >= half2x::workspace_bytes(true, nl.nproj, nvec, npw)
                    : nl.hs_accum.tiles && ws.bytes >= half2x::workspace_bytes(false, npw, nvec, nl.nproj);
 }
@@ -130,6 +138,8 @@ template void apply_nonlocal<double>(cudaStream_t, const NonlocalData<double>&, 
 template void apply_nonlocal<float>(cudaStream_t, const NonlocalData<float>&, int, int,
                                     const float2*, long, float2*, long, float2*, float2*,
                                     const GemmWorkspace&, PhaseTimer*);
+template size_t nonlocal_workspace_bytes<double>(const NonlocalData<double>&, int, int);
+template size_t nonlocal_workspace_bytes<float>(const NonlocalData<float>&, int, int);
 template size_t nonlocal_wanted_bytes<double>(const NonlocalData<double>&, int, int);
 template size_t nonlocal_wanted_bytes<float>(const NonlocalData<float>&, int, int);
 template void convert<double, float>(cudaStream_t, long, const double2*, float2*);

@@ -25,6 +25,9 @@ template <typename R> struct NonlocalData {
     zmod::PackedA zm_overlap{}, zm_accum{};
 };
 
+// workspace that the projector products of nvec bands need (FP32 on FP16 tiles: the
+// packed bands)
+template <typename R> size_t nonlocal_workspace_bytes(const NonlocalData<R>& nl, int npw, int nvec);
 // workspace with which both projector products of nvec bands run on the
 // residue tiles (0: they do not, at this size or for these projectors)
 template <typename R> size_t nonlocal_wanted_bytes(const NonlocalData<R>& nl, int npw, int nvec);

@@ -39,7 +39,7 @@ void apply_s_device(Context& c, const double2* psi, double2* spsi, int nvec, int
         const size_t pb = (size_t)P * nvec * sizeof(double2);
         c.ws_bm.reserve(&c, pb);
         c.ws_bp.reserve(&c, pb);
-        GemmWorkspace ws = c.gemm_ws(cgemm_workspace_bytes<double>(P, nvec, npw),
+        GemmWorkspace ws = c.gemm_ws(nonlocal_workspace_bytes<double>(c.overlap<double>(), npw, nvec),
                                      nonlocal_wanted_bytes<double>(c.overlap<double>(), npw, nvec));
         apply_nonlocal<double>(c.stream, c.overlap<double>(), npw, nvec, psi, npw, spsi, npw,
                                c.ws_bm.as<double2>(), c.ws_bp.as<double2>(), ws);
@@ -52,7 +52,7 @@ void apply_s_device(Context& c, const double2* psi, double2* spsi, int nvec, int
         const size_t pb = (size_t)P * nvec * sizeof(float2);
         c.ws_bm.reserve(&c, pb);
         c.ws_bp.reserve(&c, pb);
-        GemmWorkspace ws = c.gemm_ws(cgemm_workspace_bytes<float>(P, nvec, npw),
+        GemmWorkspace ws = c.gemm_ws(nonlocal_workspace_bytes<float>(c.overlap<float>(), npw, nvec),
                                      nonlocal_wanted_bytes<float>(c.overlap<float>(), npw, nvec));
         apply_nonlocal<float>(c.stream, c.overlap<float>(), npw, nvec, c.ws_conv_in.as<float2>(), npw,
                               c.ws_conv_out.as<float2>(), npw, c.ws_bm.as<float2>(), c.ws_bp.as<float2>(), ws);
