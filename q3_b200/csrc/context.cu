@@ -118,7 +118,13 @@ void DevBuf::reserve(Context* c, size_t need) {
 
 bool DevBuf::try_reserve(Context* c, size_t need) {
     if (need <= bytes && ptr) return true;
-    if (c->budget && c->held - bytes + need > c->budget) return false;
+    if (c->budget) {
+        if (c->held - bytes + need > c->budget) return false;
+    } else {
+        size_t free = 0, total = 0;
+        Q3B_CUDA(cudaMemGetInfo(&free, &total));
+        if (free + bytes < need + total / 8) return false;
+    }
     release();
     ctx = c;
     if (need == 0) return true;
@@ -572,6 +578,7 @@ void Context::prepare_kpoint(int npw, const int32_t* g2g, const double* ke, cons
     if (nproj < 0 || (nproj > 0 && (!beta || natoms <= 0 || !offs || !dblk)))
         throw Status(Q3B_ERR_INVALID, "bad projector set");
     kp.valid = false;
+    ws_gemm_refused_ = 0;  // what was short may be there again
     gamma_half = 0;
     kp.has_q = false;
     kp.dpk_len = 0;

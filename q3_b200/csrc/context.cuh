@@ -36,8 +36,10 @@ struct DevBuf {
     void release();
     // grow to at least `need` bytes (contents are not kept)
     void reserve(Context* c, size_t need);
-    // the same, but false (and the buffer as it was, or empty) where the budget
-    // or the device does not have the bytes
+    // the same for bytes that only speed things up: false (and the buffer as it was, or
+    // empty) where the budget does not have them or, without a budget, where they would
+    // leave less than an eighth of the device to the caller and to other contexts,
+    // which cannot make this one give them back
     bool try_reserve(Context* c, size_t need);
     template <typename T> T* as() const { return static_cast<T*>(ptr); }
 };
@@ -158,7 +160,7 @@ class Context {
 
   private:
     size_t ws_gemm_need_ = 0;     // largest `need` of gemm_ws
-    size_t ws_gemm_refused_ = 0;  // smallest `want` the device had no room for (0: none)
+    size_t ws_gemm_refused_ = 0;  // smallest `want` refused for this k-point (0: none)
     void build_plan();
     bool pk_valid_ = false;       // kp.beta_pk_* hold the prepared k-point's projectors
     void pack_projectors();

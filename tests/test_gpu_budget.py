@@ -55,3 +55,39 @@ def test_large_fp32_sets_keep_their_tiles(cuda_device):
     got_held, got, got_launches = _held_and_result(held - residues // 2, MIXED, npw, nproj, nvec)
     assert got_held <= held - residues // 2
     assert got_launches == launches and np.array_equal(got, want)
+
+
+def test_optional_buffers_leave_room_on_the_device_and_come_back(cuda_device):
+    """Without a budget, an eighth of the device is left to others; once there is room again, the next
+    k-point has its fast products, residues and workspace, as if there had always been."""
+    import torch
+    from q3_b200.applicator import PlanewaveHamiltonianApplicator
+    rng = np.random.default_rng(5)
+    beta = rng.standard_normal((NPW, NPROJ)) + 1j * rng.standard_normal((NPW, NPROJ))
+    x = torch.from_numpy(rng.standard_normal((NVEC, NPW)) + 1j * rng.standard_normal((NVEC, NPW))).cuda()
+
+    def apply(ap):
+        ap.prepare_kpoint(0, NPW, np.full(NPW, -1, np.int32), np.zeros(NPW), beta,
+                          np.arange(0, NPROJ + 1, 8, dtype=np.int32), np.ones(8 * NPROJ))
+        y = torch.empty_like(x)
+        ap.apply_batch(x, y, NVEC, FP64)
+        torch.cuda.synchronize()
+        return ap.ctx.device_bytes(), y
+
+    def fresh():
+        ap = PlanewaveHamiltonianApplicator()
+        ap.update_potential(np.zeros(16 ** 3), (16, 16, 16))
+        return ap
+
+    roomy, want = apply(fresh())
+    free, total = torch.cuda.mem_get_info()
+    assert free > total // 4
+    ap = fresh()
+    other = torch.empty(free - total // 10, dtype=torch.uint8, device="cuda")  # leaves a tenth
+    tight, got = apply(ap)
+    assert tight < roomy - 60 * NPW * NPROJ  # no residues
+    assert float((got - want).norm() / want.norm()) < 1e-13
+    del other
+    torch.cuda.empty_cache()
+    again, got = apply(ap)
+    assert again == roomy and torch.equal(got, want)
