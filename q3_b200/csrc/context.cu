@@ -793,13 +793,13 @@ template <typename R> void Context::tune_local() {
     LocalPlan<R>& lp = const_cast<LocalPlan<R>&>(local_plan<R>());
     if (lp.nsticks == 0) return;
     const auto key = std::make_tuple(lp.n1, lp.n2, lp.n3, (int)sizeof(R), lp.row_iv ? 1 : 0);
-    {
-        std::lock_guard<std::mutex> lk(g_tune_mu);
-        auto it = g_tuned.find(key);
-        if (it != g_tuned.end()) {
-            set_choice(lp, it->second);
-            return;
-        }
+    // held while the candidates run: contexts that meet a grid at the same time would
+    // time them beside each other, choose differently and round differently
+    std::lock_guard<std::mutex> lk(g_tune_mu);
+    auto it = g_tuned.find(key);
+    if (it != g_tuned.end()) {
+        set_choice(lp, it->second);
+        return;
     }
     // enough bands for a few planes per SM, as in a real application
     const int nb = 64;
@@ -838,10 +838,7 @@ template <typename R> void Context::tune_local() {
         }
     }
     set_choice(lp, best_choice);
-    {
-        std::lock_guard<std::mutex> lk(g_tune_mu);
-        g_tuned[key] = best_choice;
-    }
+    g_tuned[key] = best_choice;
     cudaEventDestroy(e0);
     cudaEventDestroy(e1);
     ws_tune.release();

@@ -54,3 +54,28 @@ def test_kernels_match_the_oracle(cuda_device, grid):
     torch.cuda.synchronize()
     want = odens.accumulate(psi, kp.g_to_grid, sy.cell.grid, w)
     assert np.max(np.abs(rho.cpu().numpy() - want)) / np.max(np.abs(want)) < 1e-12
+
+
+def test_contexts_that_meet_a_grid_at_once_choose_one_kernel(cuda_device):
+    """The tuner's choice is one for all contexts of a process, also when several tune at the same time
+    (a server's workers on the first requests): another kernel rounds otherwise."""
+    import threading
+    from q3_b200.applicator import PlanewaveHamiltonianApplicator
+    for n in (30, 36, 45, 48, 54):
+        sy = _system((n, n, n), 3)
+        aps = [PlanewaveHamiltonianApplicator() for _ in range(8)]
+        for ap in aps:
+            ap.update_potential(sy.v_r, sy.cell.grid)
+            ap.prepare_system_kpoint(sy)
+        start, chosen = threading.Barrier(len(aps)), [None] * len(aps)
+
+        def tune(i):
+            start.wait()
+            chosen[i] = [aps[i].local_kernel(precision) for precision in (FP64, MIXED)]
+
+        threads = [threading.Thread(target=tune, args=(i,)) for i in range(len(aps))]
+        for t in threads:
+            t.start()
+        for t in threads:
+            t.join()
+        assert all(c == chosen[0] for c in chosen), (n, chosen)
