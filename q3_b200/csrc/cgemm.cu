@@ -573,6 +573,9 @@ void cgemm(cudaStream_t st, bool conj_a, int M, int N, int K, cplx_t<R> alpha, c
 }
 
 namespace {
+// an A packed whole for two products takes at most this; a larger one is packed a panel
+// at a time for each of them (zgemm_mod.cu)
+constexpr size_t kPackedOnceBytes = 4ull << 30;
 size_t packed_once_bytes(int M, int K) {
     return zmod::packed_a_bytes(M, K) + ((zmod::packed_a_exps(M) * sizeof(int) + 255) & ~size_t(255));
 }
@@ -580,7 +583,7 @@ size_t packed_once_bytes(int M, int K) {
 
 template <typename R> size_t cgemm_two_wanted_bytes(int M, int N, int K) {
     if constexpr (std::is_same<R, double>::value) {
-        if (zmod::worth(true, M, N, K, false))
+        if (zmod::worth(true, M, N, K, false) && packed_once_bytes(M, K) <= kPackedOnceBytes)
             return packed_once_bytes(M, K) + zmod::workspace_bytes(true, M, N, K, true);
     }
     return 0;

@@ -11,6 +11,7 @@
 // every reduction in it has a fixed order, so a result does not depend on what
 // else runs beside it.  Worker contexts keep their buffers between requests
 // (no cudaFree, which would stall the other streams).
+#include <algorithm>
 #include <chrono>
 #include <condition_variable>
 #include <deque>
@@ -73,12 +74,21 @@ size_t estimate_bytes(const Job& j) {
     b += std::min<size_t>(48ull << 20, (size_t)j.nb * j.n3 * (size_t)j.n1 * j.n2 / 4 * sizeof(double2));
     // projectors: FP64, FP32 and the two packed tensor-core copies (16 B each at most)
     b += (size_t)j.npw * j.nproj * (sizeof(double2) + sizeof(float2) + 32);
-    // the projectors' residue tiles and the workspace of the largest FP64 products
+    // the projectors' residue tiles and the workspace of the largest products: both
+    // subspace rows with the basis packed once, rotations, and the projectors' own
     const int P = j.nproj, nb = (int)maxn64 / 2;
-    if (P > 0 && zmod::worth(true, P, P / 2, j.npw, true))
+    size_t ws = std::max({cgemm_two_wanted_bytes<double>((int)maxn64, nb, j.npw),
+                          cgemm_wanted_bytes<double>(true, (int)maxn64, nb, j.npw),
+                          cgemm_wanted_bytes<double>(false, j.npw, nb, (int)maxn64)});
+    if (P > 0 && zmod::worth(true, P, P / 2, j.npw, true)) {
         b += zmod::packed_a_bytes(P, j.npw) + zmod::packed_a_bytes(j.npw, P);
-    b += std::max(cgemm_wanted_bytes<double>(true, (int)maxn64, nb, j.npw),
-                  cgemm_wanted_bytes<double>(false, j.npw, nb, (int)maxn64));
+        ws = std::max({ws, zmod::workspace_bytes(true, P, nb, j.npw, true),
+                       zmod::workspace_bytes(false, j.npw, nb, P, true)});
+    }
+    if (P > 0 && mixed)
+        ws = std::max({ws, half2x::workspace_bytes(true, P, (int)nbi, j.npw),
+                       half2x::workspace_bytes(false, j.npw, (int)nbi, P)});
+    b += ws;
     b += 2 * N * (sizeof(double) + sizeof(float));  // V/N in two layouts
     b += 2 * (size_t)j.nproj * j.nb * sizeof(double2) + (16ull << 20);
     return b + b / 5;

@@ -713,7 +713,7 @@ struct Plan {
     size_t b_bytes, a_bytes, out_bytes, exp_bytes, balance_bytes, total;
 };
 
-// the packed rows of A and the output bytes of one panel stay below this
+// the output bytes of one panel and the rows of A that are packed with it stay below this
 constexpr size_t kPanelBytes = 640ull << 20;
 
 Plan plan_of(bool conj_a, int M, int N, int K, bool packed) {

@@ -91,3 +91,17 @@ def test_optional_buffers_leave_room_on_the_device_and_come_back(cuda_device):
     torch.cuda.empty_cache()
     again, got = apply(ap)
     assert again == roomy and torch.equal(got, want)
+
+
+def test_a_basis_packed_for_two_products_stays_within_bounds(cuda_device):
+    """The workspace in which the Davidson's basis is packed whole, once for both subspace rows, ends
+    at 4 GB of packed basis (30 bytes an entry, rows padded to 256): above, each product packs it a
+    panel at a time, and its workspace is that of one product."""
+    import ctypes as C
+    from q3_b200 import _lib
+    lib = _lib.load()
+    two = lib["_ZN3q3b22cgemm_two_wanted_bytesIdEEmiii"]  # size_t q3b::cgemm_two_wanted_bytes<double>(int, int, int)
+    two.restype, two.argtypes = C.c_size_t, [C.c_int] * 3
+    below, above = 128 * (4 * 2 ** 30 // (128 * 30 * 1024)), 160000
+    assert two(1024, 512, below) >= 30 * 1024 * below
+    assert two(1024, 512, above) == 0
