@@ -89,32 +89,35 @@ struct Balance {
     }
 };
 
-__global__ void __launch_bounds__(256) exps_kmajor(int R, int K, const float2* __restrict__ X, long ld, Balance bal,
+// one block of NT threads a row, 1024 from kLongRow of K on
+constexpr int kLongRow = 4096;
+template <int NT>
+__global__ void __launch_bounds__(NT) exps_kmajor(int R, int K, const float2* __restrict__ X, long ld, Balance bal,
                                                    int* exps) {
     chain_begin();
     const int r = blockIdx.x;
     float mx = 0.f;
     if (r < R) {
         const float2* x = X + (long)r * ld;
-        for (int k = threadIdx.x; k < K; k += 8 * 256) {
+        for (int k = threadIdx.x; k < K; k += 8 * NT) {
             float2 v[8];
             float f[8];
 #pragma unroll
             for (int u = 0; u < 8; ++u) {
-                const bool ok = k + 256 * u < K;
-                v[u] = ok ? x[k + 256 * u] : make_float2(0.f, 0.f);
-                f[u] = pow2f(ok ? bal.at(k + 256 * u) : 0);
+                const bool ok = k + NT * u < K;
+                v[u] = ok ? x[k + NT * u] : make_float2(0.f, 0.f);
+                f[u] = pow2f(ok ? bal.at(k + NT * u) : 0);
             }
 #pragma unroll
             for (int u = 0; u < 8; ++u) mx = larger(mx, f[u] * v[u]);
         }
     }
-    __shared__ float s[8];
+    __shared__ float s[NT / 32];
     for (int o = 16; o > 0; o >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
     if ((threadIdx.x & 31) == 0) s[threadIdx.x >> 5] = mx;
     __syncthreads();
     if (threadIdx.x == 0) {
-        for (int w = 1; w < 8; ++w) mx = fmaxf(mx, s[w]);
+        for (int w = 1; w < NT / 32; ++w) mx = fmaxf(mx, s[w]);
         exps[r] = exponent_for(mx);
     }
 }
@@ -506,7 +509,8 @@ void pack_operand(cudaStream_t st, int R, int K, const float2* X, long ld, const
     const Balance bal{balance, AS == kPackA ? -1 : 1};
     const int padded = ceil_div(R, 2 * ROWS) * 2 * ROWS, nkb = ceil_div(K, BK);
     if (K > kLongestK) throw std::runtime_error("tensor-core GEMM: operand too large to pack");
-    if (KMAJOR) launch_chained(exps_kmajor, padded, 256, 0, st, R, K, X, ld, bal, exps);
+    if (KMAJOR && K >= kLongRow) launch_chained(exps_kmajor<1024>, padded, 1024, 0, st, R, K, X, ld, bal, exps);
+    else if (KMAJOR) launch_chained(exps_kmajor<256>, padded, 256, 0, st, R, K, X, ld, bal, exps);
     else launch_chained(exps_mmajor, padded / 32, 256, 0, st, R, K, X, ld, bal, exps);
     Q3B_LAUNCH_CHECK();
     launch_chained(pack_rows<KMAJOR, ROWS, AS>, dim3(padded / PACK_ROWS, nkb), 256, 0, st, R, K, X, ld, bal, exps, nkb, tiles);

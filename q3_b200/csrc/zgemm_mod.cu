@@ -37,7 +37,8 @@
 // beta D beta^H psi of the 64-atom cell, relative 2-norm from the exact value, without
 // the balance, with it, and on DFMAs: projector norms spread over 1e6, 1.7e-12, 1.6e-15
 // and 3.7e-15; bands of high plane waves only, 1.9e-13, 3.4e-16 and 2.7e-15; as the cell
-// has them, 1.7e-16, 2.0e-16 and 3.3e-15.  It costs 17 us of the 1.8 ms of H|psi>.
+// has them, 1.7e-16, 2.0e-16 and 3.3e-15.  It cost 17 us of the 1.8 ms of H|psi> while the
+// norms of a long row were formed by 256 threads, and nothing with 1024.
 // Other C,N products are inner products of vectors, which need no more than
 // 1.6e-18 of their norms.
 //
@@ -186,28 +187,31 @@ struct Balance {
     }
 };
 
-// rows contiguous along K: one block a row
-__global__ void __launch_bounds__(256) exps_kmajor(int R, int K, const double2* __restrict__ X, long ld, double c,
+// rows contiguous along K: one block of NT threads a row (kLongRow and above 1024, which takes
+// the balance's extra reads in the time that 256 threads took without them)
+constexpr int kLongRow = 4096;
+template <int NT>
+__global__ void __launch_bounds__(NT) exps_kmajor(int R, int K, const double2* __restrict__ X, long ld, double c,
                                                    Balance bal, int zero, int* exps) {
     chain_begin();
     const int r = blockIdx.x;
     double ss = 0.0, mx = 0.0;
     if (r < R) {
         const double2* x = X + (long)r * ld;
-        for (int k = threadIdx.x; k < K; k += 4 * 256) {
+        for (int k = threadIdx.x; k < K; k += 4 * NT) {
             double2 v[4];
             double f[4];
 #pragma unroll
             for (int u = 0; u < 4; ++u) {
-                const bool ok = k + 256 * u < K;
-                v[u] = ok ? x[k + 256 * u] : make_double2(0.0, 0.0);
-                f[u] = pow2(ok ? bal.at(k + 256 * u) : 0);
+                const bool ok = k + NT * u < K;
+                v[u] = ok ? x[k + NT * u] : make_double2(0.0, 0.0);
+                f[u] = pow2(ok ? bal.at(k + NT * u) : 0);
             }
 #pragma unroll
             for (int u = 0; u < 4; ++u) take(f[u] * v[u], ss, mx);
         }
     }
-    __shared__ double s_ss[8], s_mx[8];
+    __shared__ double s_ss[NT / 32], s_mx[NT / 32];
     for (int o = 16; o > 0; o >>= 1) {
         ss += __shfl_xor_sync(0xffffffffu, ss, o);
         mx = fmax(mx, __shfl_xor_sync(0xffffffffu, mx, o));
@@ -218,7 +222,7 @@ __global__ void __launch_bounds__(256) exps_kmajor(int R, int K, const double2* 
     }
     __syncthreads();
     if (threadIdx.x == 0) {
-        for (int w = 1; w < 8; ++w) {
+        for (int w = 1; w < NT / 32; ++w) {
             ss += s_ss[w];
             mx = fmax(mx, s_mx[w]);
         }
@@ -766,7 +770,9 @@ void pack_operand(cudaStream_t st, int R, int K, const double2* X, long ld, cons
     const Balance bal{balance, AS == kPackA ? -1 : 1};
     const int padded = ceil_div(R, 2 * ROWS) * 2 * ROWS, nkb = ceil_div(K, BK);
     if (nkb > 65535) throw std::runtime_error("complex GEMM: operand too large to pack");
-    if (KMAJOR) launch_chained(exps_kmajor, padded, 256, 0, st, R, K, X, ld, scale_bits(), bal, 0, exps);
+    if (KMAJOR && K >= kLongRow)
+        launch_chained(exps_kmajor<1024>, padded, 1024, 0, st, R, K, X, ld, scale_bits(), bal, 0, exps);
+    else if (KMAJOR) launch_chained(exps_kmajor<256>, padded, 256, 0, st, R, K, X, ld, scale_bits(), bal, 0, exps);
     else launch_chained(exps_mmajor<8>, padded / 32, 256, 0, st, R, K, X, ld, scale_bits(), bal, 0, exps);
     Q3B_LAUNCH_CHECK();
     launch_chained(pack_rows<KMAJOR, ROWS, AS>, dim3(padded / PACK_ROWS, nkb), 256, PACK_SMEM, st, R, K, X, ld, bal, exps, nkb, tiles);
@@ -825,7 +831,7 @@ size_t balance_ints(int lines) { return (size_t)ceil_div(lines, BK) * BK; }
 
 void balance_projectors(cudaStream_t st, int npw, int nproj, const double2* beta, int* along_proj, int* along_pw) {
     if (npw <= 0 || nproj <= 0) return;
-    launch_chained(exps_kmajor, nproj, 256, 0, st, nproj, npw, beta, npw, scale_bits(), Balance{nullptr, 0}, kZeroLine,
+    launch_chained(exps_kmajor<256>, nproj, 256, 0, st, nproj, npw, beta, npw, scale_bits(), Balance{nullptr, 0}, kZeroLine,
                    along_proj);
     Q3B_LAUNCH_CHECK();
     launch_chained(balance_lines, 1, 1024, 0, st, nproj, (int)balance_ints(nproj), -1, along_proj);
