@@ -98,7 +98,9 @@ void count_launch();
 // of spreading over all of them, and where a product has one block for each SM
 // that costs more than the latency.  H|psi> launched plainly, let in by any grid of
 // up to four blocks an SM, and as it is: eight atoms 75.7, 85.5 and 68.4 us, two
-// atoms 37.4, 34.1 and 34.4.  Grids above kChainBlocks are launched plainly.
+// atoms 37.4, 34.1 and 34.4.  Grids above kChainBlocks are launched plainly.  The SM
+// count is the B200's, a literal because both sides of a launch compare with it and
+// neither should look it up; a part with fewer SMs would be served as correctly.
 constexpr int kEarlyBlocks = 148, kChainBlocks = 4 * 148;
 __device__ __forceinline__ void chain_begin() {
     asm volatile("griddepcontrol.wait;" ::: "memory");
