@@ -185,17 +185,17 @@ __global__ void __launch_bounds__(256) pack_rows(int R, int K, const float2* __r
     }
     __syncthreads();
     const int row = tid >> 3, ch = tid & 7, gr = r0 + row, e = exps[gr];
-    const float f1 = pow2f(e / 2);
     int along[8];
     bal.get8(k0 + 8 * ch, along);
     unsigned hi[2][4], lo[2][4];
 #pragma unroll
     for (int j = 0; j < 4; ++j) {
         const float2 a = s[row * PACK_PITCH + ch * 9 + 2 * j], b = s[row * PACK_PITCH + ch * 9 + 2 * j + 1];
-        const float f2 = pow2f(e - e / 2 + along[2 * j]), g2 = pow2f(e - e / 2 + along[2 * j + 1]);
+        const int ea = e + along[2 * j], eb = e + along[2 * j + 1];
+        const float a1 = pow2f(ea / 2), a2 = pow2f(ea - ea / 2), b1 = pow2f(eb / 2), b2 = pow2f(eb - eb / 2);
 #pragma unroll
         for (int p = 0; p < 2; ++p) {
-            const float x = scaled(p ? a.y : a.x, f1, f2), y = scaled(p ? b.y : b.x, f1, g2);
+            const float x = scaled(p ? a.y : a.x, a1, a2), y = scaled(p ? b.y : b.x, b1, b2);
             const __half2 h = __floats2half2_rn(x, y);
             const float2 hf = __half22float2(h);
             const __half2 l = __floats2half2_rn(x - hf.x, y - hf.y);

@@ -62,3 +62,30 @@ def test_projector_products(cuda_device, npw, nproj, nvec, kind):
         torch.cuda.synchronize()
         got = y.cpu().numpy().T
         assert np.max(np.abs(got - want) / mag) < tol, precision
+
+
+@pytest.mark.parametrize("precision,scale,tol", [(MIXED, 3e-38, 4e-6), (FP64, 1e-290, 1e-15)], ids=["mixed", "fp64"])
+def test_tiny_projectors_with_zeros_among_them(cuda_device, precision, scale, tol):
+    """Projectors near the end of the range, a projector of zeros and plane waves that no projector
+    reaches: scales and balance together stay in range, and the zeros contribute nothing."""
+    import torch
+    from q3_b200.applicator import PlanewaveHamiltonianApplicator
+    npw, nproj, nvec = 12289, 640, 130
+    beta, psi, _ = _inputs(npw, nproj, nvec, "normal")
+    beta[:, 17] = 0.0
+    beta[1000:1200] = 0.0
+    ap = PlanewaveHamiltonianApplicator()
+    ap.update_potential(np.zeros(16 ** 3), (16, 16, 16))
+    # D takes the scale out of the coefficients again, so that the result is beta's size
+    ap.prepare_kpoint(0, npw, np.full(npw, -1, np.int32), np.zeros(npw), scale * beta,
+                      np.arange(0, nproj + 1, 8, dtype=np.int32), np.tile(np.eye(8).reshape(-1) / scale, nproj // 8))
+    x = torch.from_numpy(np.ascontiguousarray(psi.T)).cuda()
+    y = torch.full_like(x, np.nan)
+    ap.apply_batch(x, y, nvec, precision)
+    torch.cuda.synchronize()
+    want = beta @ (beta.conj().T @ psi)
+    mag = np.abs(beta) @ (np.abs(beta).T @ np.abs(psi))
+    got = y.cpu().numpy().T / scale
+    assert np.all(got[1000:1200] == 0.0)
+    keep = mag > 0.0
+    assert np.max(np.abs(got - want)[keep] / mag[keep]) < tol
