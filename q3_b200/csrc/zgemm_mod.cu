@@ -843,15 +843,15 @@ void balance_projectors(cudaStream_t st, int npw, int nproj, const double2* beta
     Q3B_LAUNCH_CHECK();
 }
 
-// Estimated times of both paths, from runs of q3b_gemm on shapes of the 8- to
-// 128-atom cells (B200, 1965 MHz): here 19 ps per packed entry, 60 ns per 128 x 64
-// tile and K block, 10 ps per output, and 40 us of launches; on the FP64 units as
-// their own tiles are chosen.  Measured, here against there: 23847 x 256 x 512
-// (N,N) 0.49 ms against 1.12, 512 x 256 x 23847 (C,N) 0.53 against 0.97,
-// 1024 x 512 x 62669 3.6 against 10.2; the two meet near 23847 x 64 x 512 (0.33
-// against 0.33) and 12000 x 128 x 256 (0.15 against 0.17).  With A packed before
-// (the projectors), beta Q beta^H psi of 90 bands of the 64-atom cell takes 0.39 ms
-// against 1.14.
+// Estimated times of both paths, from runs of q3b_gemm_residue and q3b_gemm on shapes
+// of the 8- to 128-atom cells (B200, 1965 MHz): here 19 ps per packed entry, 60 ns per
+// 128 x 64 tile and K block, 10 ps per output, and 40 us of launches; on the FP64 units
+// as their own tiles are chosen.  Measured, here against there: 23847 x 256 x 512
+// (N,N) 0.48 ms against 1.00, 512 x 256 x 23847 (C,N) 0.51 against 0.96,
+// 1024 x 512 x 62669 (C,N) 3.5 against 10.2; the two meet near 23847 x 64 x 512 (N,N, 0.35
+// against 0.30), 12000 x 128 x 256 (N,N, 0.145 against 0.158) and 256 x 128 x 12000 (C,N,
+// 0.157 against 0.142).  With A packed before (the projectors), beta Q beta^H psi of 90
+// bands of the 64-atom cell takes 0.37 ms against 1.14.
 bool worth(bool conj_a, int M, int N, int K, bool packed) {
     if (M < 64 || N < 16 || K < 64 || K > kLongestK) return false;
     const double tiles = (double)ceil_div(M, 2 * BM) * (narrow(N) ? 2 : 4 * ceil_div(N, 128)) * ceil_div(K, BK);
